@@ -144,14 +144,15 @@ int scg_mesh_from_plot3d(const char * data, int64_t nbyte, scg_mesh ** out);
 /* Precision of the march. */
 #define SCG_FP64 0        /* the reference's FP64 arithmetic */
 /* The FP32 form of the EulerCore: FP32 state and flux arithmetic with
- * compensated face sums, mesh geometry kept in FP64 tables, FP64 totals and
- * CFL reduction.  The march rounds the FP64 geometry to FP32 where it uses
- * it; a mesh whose geometry (at this time increment) reaches 2^128 in
+ * compensated face sums, mesh geometry formed in FP64 (the CE volumes,
+ * centroids and sub-face moments) and every value that the march uses rounded
+ * once to FP32, FP64 totals and CFL reduction.  A mesh whose geometry (at
+ * this time increment) reaches 2^128 in
  * magnitude, or holds infinities or NaN, is refused with SCG_EINVAL when the
  * core is created or one of its CE geometry arrays is set. */
 #define SCG_FP32_GEOM64 1
 /* A faster EulerCore variant beside it: the same FP32 march with its
- * geometry (computed in FP64) stored in FP32, ~35% less traffic per cell. */
+ * gradient-element displacements formed in FP32 from fewer stored values. */
 #define SCG_FP32_GEOM32 2
 /* Euler1DCore's FP32 state (its coordinates stay FP64), and the FP32 pipe of
  * scg_fma_peak; as an EulerCore precision the same code as SCG_FP32_GEOM32. */
@@ -432,7 +433,7 @@ int scg_st_stream(const scg_st * solver, void ** out);
  * ---------------------------------------------------------------------- */
 
 /* Not in the reference: round n FP64 values to FP32 on the device exactly as
- * the FP32 march rounds its FP64 geometry tables where it uses them
+ * the FP32 form rounds its FP64 geometry when it builds its march tables
  * (round to nearest even, formed on the integer pipe; values below FP32's
  * normal range give a signed zero, and values of magnitude 2^128 and beyond,
  * which a core refuses, are not defined here), for checking that rounding.  Synchronous; allocates its own device buffers. */

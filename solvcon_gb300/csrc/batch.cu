@@ -138,7 +138,7 @@ public:
 
     // The precision code of the cores this instantiation marches.
     static constexpr int PREC = sizeof(R) == 8 ? scg::PREC_FP64
-                                               : (sizeof(G) == 8 ? scg::PREC_FP32_GEOM64 : scg::PREC_FP32);
+                                               : (scg::dev::Geo<ND, G>::MID ? scg::PREC_FP32 : scg::PREC_FP32_GEOM64);
 
     bool retarget(std::vector<scg::EulerCoreBase *> cs) override
     {
@@ -444,13 +444,13 @@ std::unique_ptr<BatchBase> make_batch(std::vector<scg::EulerCoreBase *> cores, i
         if (prec == scg::PREC_FP64)
             return make_for_block<2, double, double>(std::move(cores), block, persistent);
         if (prec == scg::PREC_FP32_GEOM64)
-            return make_for_block<2, float, double>(std::move(cores), block, persistent);
+            return make_for_block<2, float, scg::dev::Rounded>(std::move(cores), block, persistent);
         return make_for_block<2, float, float>(std::move(cores), block, persistent);
     }
     if (prec == scg::PREC_FP64)
         return make_for_block<3, double, double>(std::move(cores), block, persistent);
     if (prec == scg::PREC_FP32_GEOM64)
-        return make_for_block<3, float, double>(std::move(cores), block, persistent);
+        return make_for_block<3, float, scg::dev::Rounded>(std::move(cores), block, persistent);
     return make_for_block<3, float, float>(std::move(cores), block, persistent);
 }
 

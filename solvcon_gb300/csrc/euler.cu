@@ -1049,39 +1049,32 @@ public:
             return;
         }
         ensure_ce();
+        // The FP32 form's geometry is rounded to FP32 here: values that FP32
+        // cannot hold are counted, and the mesh refused.
+        constexpr bool ROUNDS = std::is_same<G, Rounded>::value;
+        DevBuf<unsigned long long> bad(ROUNDS ? 1 : 0);
+        if constexpr (ROUNDS)
+        {
+            cuda_check(cudaMemsetAsync(bad.ptr, 0, sizeof(unsigned long long), stream), "memset");
+        }
         k_compact<ND, G><<<grid_for(ncell), BLOCK, 0, stream>>>(mv, ce[0].ptr, ce[1].ptr, ce[2].ptr, ce[3].ptr,
                                                                 0.5 * time_increment, std::max(nslot, 1),
-                                                                d_fgeo.ptr, d_cgeo.ptr, d_nbr.ptr, d_ctype.ptr);
+                                                                d_fgeo.ptr, d_cgeo.ptr, d_nbr.ptr, d_ctype.ptr,
+                                                                bad.ptr);
         launched(stream, "compact");
-        if constexpr (sizeof(R) == 4 && sizeof(G) == 8)
+        if constexpr (ROUNDS)
         {
-            check_geometry_range();
-        }
-    }
-
-    // The FP32 march rounds its FP64 geometry without range selects
-    // (scg::dev::geo_r): refuse tables holding values it does not take.
-    void check_geometry_range()
-    {
-        DevBuf<unsigned long long> bad(1);
-        cuda_check(cudaMemsetAsync(bad.ptr, 0, sizeof(unsigned long long), stream), "memset");
-        for (auto const * t : {&d_fgeo, &d_cgeo})
-        {
-            int64_t const n = static_cast<int64_t>(t->bytes() / sizeof(G));
-            int64_t const blocks = std::min<int64_t>((n + BLOCK - 1) / BLOCK, 4096);
-            k_geo_range<<<static_cast<unsigned>(std::max<int64_t>(blocks, 1)), BLOCK, 0, stream>>>(
-                reinterpret_cast<double const *>(t->ptr), n, bad.ptr);
-            launched(stream, "geo_range");
-        }
-        unsigned long long cnt = 0;
-        cuda_check(cudaMemcpyAsync(&cnt, bad.ptr, sizeof(cnt), cudaMemcpyDeviceToHost, stream), "D2H");
-        sync();
-        if (cnt)
-        {
-            throw std::invalid_argument("EulerCore: precision fp32 keeps FP64 geometry and uses it in FP32; " +
-                                        std::to_string(cnt) +
-                                        " geometry values of this mesh lie beyond FP32's range (magnitude 2^128 "
-                                        "or more, infinite or NaN): use precision fp64, or rescale the mesh");
+            unsigned long long cnt = 0;
+            cuda_check(cudaMemcpyAsync(&cnt, bad.ptr, sizeof(cnt), cudaMemcpyDeviceToHost, stream), "D2H");
+            sync();
+            if (cnt)
+            {
+                throw std::invalid_argument("EulerCore: precision fp32 uses the mesh geometry, computed in FP64, in "
+                                            "FP32; " +
+                                            std::to_string(cnt) +
+                                            " geometry values of this mesh lie beyond FP32's range (magnitude 2^128 "
+                                            "or more, infinite or NaN): use precision fp64, or rescale the mesh");
+            }
         }
     }
 
@@ -2116,13 +2109,13 @@ std::unique_ptr<EulerCoreBase> make_euler_core(HostMesh const & mesh, double dt,
         if (prec == PREC_FP64)
             return std::make_unique<EulerCoreImpl<2, double, double>>(mesh, dt, prec);
         if (prec == PREC_FP32_GEOM64)
-            return std::make_unique<EulerCoreImpl<2, float, double>>(mesh, dt, prec);
+            return std::make_unique<EulerCoreImpl<2, float, Rounded>>(mesh, dt, prec);
         return std::make_unique<EulerCoreImpl<2, float, float>>(mesh, dt, prec);
     }
     if (prec == PREC_FP64)
         return std::make_unique<EulerCoreImpl<3, double, double>>(mesh, dt, prec);
     if (prec == PREC_FP32_GEOM64)
-        return std::make_unique<EulerCoreImpl<3, float, double>>(mesh, dt, prec);
+        return std::make_unique<EulerCoreImpl<3, float, Rounded>>(mesh, dt, prec);
     return std::make_unique<EulerCoreImpl<3, float, float>>(mesh, dt, prec);
 }
 
@@ -2137,7 +2130,7 @@ __global__ void k_geo_round(double const * in, float * out, int64_t n)
     int64_t const i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i < n)
     {
-        out[i] = scg::dev::geo_r<float>(in[i]);
+        out[i] = scg::dev::geo_r(in[i]);
     }
 }
 

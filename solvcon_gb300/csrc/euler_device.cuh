@@ -40,6 +40,7 @@
 #include "divide.cuh"
 
 #include <cstdint>
+#include <type_traits>
 
 namespace scg
 {
@@ -57,26 +58,36 @@ struct Dim
     static constexpr int KC = 2;
 };
 
+// FP64 geometry rounded once to FP32, when the tables are built: the storage
+// of the FP32 form's geometry (precision fp32).  The FP32 march uses every
+// geometry value in FP32, so the tables hold the rounding that it would
+// otherwise form from an FP64 table at every use, with the same bits and half
+// the bytes (see geo_store in euler_setup.cuh).
+struct Rounded
+{
+    float v;
+};
+
 // Per-face geometry components, stored as G: bvol, dB[ND] = x_BCE - x_nbr,
 // Nh[ND], Mh[ND][ND], then either the gradient-element displacements P[ND],
-// Q[ND], R[ND] (FP64 geometry) or mid[ND] = x_BCE - x_cell (FP32 geometry).
+// Q[ND], R[ND] (geometry computed in FP64: G double or Rounded) or
+// mid[ND] = x_BCE - x_cell (fp32-geom32: G float).
 // P, Q and R follow from dB and mid with means over the cell's faces:
 //   P = mid - mean(mid),  Q = mean(dB) - dB,  R = dB - mean(mid),
-// which the memory-bound FP32 march forms in registers for 4 (2D) or 6 (3D)
-// fewer stored values per face; the FP64 march, bound by its FP64 pipe,
-// reads them.
+// which the fp32-geom32 march forms in registers, in FP32, for 4 (2D) or 6
+// (3D) fewer stored values per face; the others read them as formed in FP64.
 template <int ND, typename G>
 struct Geo
 {
-    static constexpr bool MID = sizeof(G) == 4;
+    static constexpr bool MID = std::is_same<G, float>::value;
     static constexpr int K_BVOL = 0;
     static constexpr int K_DB = 1;
     static constexpr int K_NH = 1 + ND;
     static constexpr int K_MH = 1 + 2 * ND;
-    static constexpr int K_P = 1 + 2 * ND + ND * ND; // FP64 geometry
+    static constexpr int K_P = 1 + 2 * ND + ND * ND; // FP64-computed geometry
     static constexpr int K_Q = K_P + ND;
     static constexpr int K_R = K_Q + ND;
-    static constexpr int K_MID = K_P; // FP32 geometry
+    static constexpr int K_MID = K_P; // fp32-geom32
     static constexpr int KF = MID ? K_MID + ND : K_R + ND;
 };
 
@@ -117,12 +128,9 @@ struct Tiny<float>
     static constexpr float AZ = 1.e-37f;
 };
 
-// A geometry value (stored G) in the march's precision R.  FP64 geometry read
-// by the FP32 march is rounded with integer instructions only: a double ->
-// float conversion instruction issues on the FP64 pipe (16 cycles per warp on
-// GB300, measured), and the FP32 march converts ~60 geometry values per
-// cell-substep, which made that pipe the FP32 march's bottleneck.  In the
-// FP32 normal range the result is IEEE round-to-nearest-even: adding
+// An FP64 geometry value rounded to FP32 for the FP32 form's tables, with
+// integer instructions (a double -> float conversion issues on the FP64 pipe).
+// In the FP32 normal range the result is IEEE round-to-nearest-even: adding
 // 2^28 - 1 plus the kept part's lowest bit to the 64-bit pattern carries
 // into bit 29 exactly when the 29 bits to be dropped exceed half, or equal
 // half with an odd lowest kept bit; the funnel shift then takes bits 29..60,
@@ -130,12 +138,18 @@ struct Tiny<float>
 // (1023 - 127) << 23 modulo 2^32 rebiases the exponent (its high bits
 // shifted out cancel).  Values below the FP32 normal range (round-off
 // residue in the tables) become a signed zero, by one compare and select.
-// Larger ones are not taken here: a core of the FP32 form checks its
-// geometry tables when it builds them (k_geo_range) and refuses values at
-// 2^128 and beyond, infinities and NaNs, so the rounding needs no second
-// range select (9 integer instructions per value instead of 15, for ~47
-// values per cell-substep in 2D).  Branch-free, so nothing falls back to the
-// conversion instruction.
+// Larger ones are not taken here: a core of the FP32 form checks each value
+// as it builds its tables and refuses values at 2^128 and beyond, infinities
+// and NaNs.
+__device__ __forceinline__ float geo_r(double v)
+{
+    unsigned long long const b = static_cast<unsigned long long>(__double_as_longlong(v));
+    unsigned const hi = static_cast<unsigned>(b >> 32);
+    unsigned long long const t = b + 0x0FFFFFFFull + ((b >> 29) & 1ull);
+    unsigned const r = __funnelshift_l(static_cast<unsigned>(t), static_cast<unsigned>(t >> 32), 3) - 0xC0000000u;
+    return __uint_as_float(((hi & 0x7FF00000u) >= (897u << 20) ? r : 0u) | (hi & 0x80000000u));
+}
+
 // The geometry values geo_r takes: magnitudes below 2^128 (biased exponent
 // up to 1150).
 __device__ __forceinline__ bool geo_r_takes(double v)
@@ -144,17 +158,13 @@ __device__ __forceinline__ bool geo_r_takes(double v)
     return e <= 1150u;
 }
 
+// A stored geometry value in the march's precision R.
 template <typename R, typename G>
-__device__ __forceinline__ R geo_r(G v)
+__device__ __forceinline__ R geo_val(G v)
 {
-    if constexpr (sizeof(R) == 4 && sizeof(G) == 8)
+    if constexpr (std::is_same<G, Rounded>::value)
     {
-        unsigned long long const b = static_cast<unsigned long long>(__double_as_longlong(v));
-        unsigned const hi = static_cast<unsigned>(b >> 32);
-        unsigned long long const t = b + 0x0FFFFFFFull + ((b >> 29) & 1ull);
-        unsigned const r =
-            __funnelshift_l(static_cast<unsigned>(t), static_cast<unsigned>(t >> 32), 3) - 0xC0000000u;
-        return __uint_as_float(((hi & 0x7FF00000u) >= (897u << 20) ? r : 0u) | (hi & 0x80000000u));
+        return v.v;
     }
     else
     {

@@ -119,54 +119,24 @@ __device__ __forceinline__ void store_rec(R * base, R const * so0, R const * so0
     }
 }
 
-// A geometry table value, loaded once per cell-substep and streamed: the
-// FP32 3D march (FP64 tables, 816 B per tetrahedron) loads it evict-first,
-// which leaves the caches to the neighbour records (measured on 24.6M
-// tetrahedra: 7.08 -> 6.84 ms per launch; in 2D, and with L1 no-allocate
-// loads, it was slower, so the other marches load it plainly).
+// A geometry table value, loaded once per cell-substep and streamed.
 template <int ND, typename R, typename G>
-__device__ __forceinline__ G geo_ld(G const * p)
+__device__ __forceinline__ R geo_ld(G const * p)
 {
-    if constexpr (ND == 3 && sizeof(R) == 4 && sizeof(G) == 8)
+    if constexpr (std::is_same<G, Rounded>::value)
     {
-        return __ldcs(p);
+        return ldg(&p->v);
     }
     else
     {
-        return ldg(p);
+        return geo_val<R>(ldg(p));
     }
 }
 
 template <int ND, typename R, typename G>
 __device__ __forceinline__ R fg(MarchArgs<R, G> const & a, int f, int k, int64_t icl)
 {
-    return geo_r<R>(geo_ld<ND, R>(a.fgeo + (static_cast<int64_t>(f) * Geo<ND, G>::KF + k) * a.ncell + icl));
-}
-
-// The same rounding (IEEE round-to-nearest-even: the same bits over FP32's
-// normal range, where geometry values lie) for the
-// few values the FP32 3D march uses last (the gradient-element displacement
-// P and the two per-cell scalars): there the conversion instruction, on the
-// otherwise idle FP64 pipe, relieves the integer pipe of 14 roundings per
-// tetrahedron (6.84 -> 6.70 ms per 24.6M-cell launch; in 2D it was 1% slower,
-// so 2D rounds everything with integers).
-template <int ND, typename R, typename G>
-__device__ __forceinline__ R geo_late(G v)
-{
-    if constexpr (ND == 3 && sizeof(R) == 4 && sizeof(G) == 8)
-    {
-        return R(v);
-    }
-    else
-    {
-        return geo_r<R>(v);
-    }
-}
-
-template <int ND, typename R, typename G>
-__device__ __forceinline__ R fg_late(MarchArgs<R, G> const & a, int f, int k, int64_t icl)
-{
-    return geo_late<ND, R>(geo_ld<ND, R>(a.fgeo + (static_cast<int64_t>(f) * Geo<ND, G>::KF + k) * a.ncell + icl));
+    return geo_ld<ND, R>(a.fgeo + (static_cast<int64_t>(f) * Geo<ND, G>::KF + k) * a.ncell + icl);
 }
 
 // What calc_soln hands to calc_dsoln of the same cell when the neighbour
@@ -196,21 +166,22 @@ __host__ __device__ constexpr bool carries()
 // registers, 80 bytes spilled), 4.66 ms at 4 (128 registers).  With the
 // FP32 delta form (u0, d0 below) 7 blocks stay best in 2D (0.1628 ms; 6:
 // 0.1688, 8: 0.1683) and 4 in 3D (4.80 ms).  The budget per thread (72 /
-// 128 registers) is kept for other block sizes.  With FP64 geometry tables
-// (G = double) the budget is set apart, as the geometry loads and their
-// rounding hold more registers: 2D, 980k triangles, 0.2350 / 0.2364 /
-// 0.2296 / 0.2175 ms per 2M-cell launch at 64 / 72 / 80 / 96 registers.
+// 128 registers) is kept for other block sizes.  The FP32 form (G = Rounded,
+// 15 / 25 stored values per face instead of 11 / 19) has its own budget: 2D,
+// 2M triangles, 0.2016 ms per launch at 96 registers against 0.2573 at 80,
+// 0.2750 at 72 and 0.3126 at 64 (spills); 3D, 1.3M tetrahedra, 0.299 ms at 128
+// and at 96, 0.334 at 80, 0.345 at 168.
 #ifndef SCG_CARRY_REGS_2D
 #define SCG_CARRY_REGS_2D 72
 #endif
-#ifndef SCG_CARRY_REGS_2D_G64
-#define SCG_CARRY_REGS_2D_G64 96
+#ifndef SCG_CARRY_REGS_2D_ROUNDED
+#define SCG_CARRY_REGS_2D_ROUNDED 96
 #endif
 #ifndef SCG_CARRY_REGS_3D
 #define SCG_CARRY_REGS_3D 128
 #endif
-#ifndef SCG_CARRY_REGS_3D_G64
-#define SCG_CARRY_REGS_3D_G64 128
+#ifndef SCG_CARRY_REGS_3D_ROUNDED
+#define SCG_CARRY_REGS_3D_ROUNDED 128
 #endif
 template <int ND, typename R, int CT, int BLOCK, typename G = R>
 __host__ __device__ constexpr int min_blocks()
@@ -221,8 +192,8 @@ __host__ __device__ constexpr int min_blocks()
     }
     else
     {
-        constexpr int regs = ND == 3 ? (sizeof(G) == 8 ? SCG_CARRY_REGS_3D_G64 : SCG_CARRY_REGS_3D)
-                                     : (sizeof(G) == 8 ? SCG_CARRY_REGS_2D_G64 : SCG_CARRY_REGS_2D);
+        constexpr int regs = ND == 3 ? (Geo<ND, G>::MID ? SCG_CARRY_REGS_3D : SCG_CARRY_REGS_3D_ROUNDED)
+                                     : (Geo<ND, G>::MID ? SCG_CARRY_REGS_2D : SCG_CARRY_REGS_2D_ROUNDED);
         return 65536 / (BLOCK * regs);
     }
 }
@@ -426,7 +397,7 @@ __device__ __forceinline__ void soln_cell(MarchArgs<R, G> const & a, int64_t icl
             acc[i].add(-fl[i]);
         }
     }
-    R const ivol = geo_late<ND, R>(geo_ld<ND, R>(a.cgeo + 0 * a.ncell + icl));
+    R const ivol = geo_ld<ND, R>(a.cgeo + 0 * a.ncell + icl);
 #pragma unroll
     for (int i = 0; i < NEQ; ++i)
     {
@@ -468,7 +439,7 @@ __device__ __forceinline__ R cfl_cell(MarchArgs<R, G> const & a, int64_t icl, in
     R const pr = ga1 * (so0n[NEQ - 1] - ke);
     R const pra = (pr + fabs(pr)) / R(2);
     R const wspd = sqr_t(ga * pra * ri) + sqr_t(momsq) * ri;
-    R const cflo = wspd * geo_late<ND, R>(geo_ld<ND, R>(a.cgeo + 1 * a.ncell + icl));
+    R const cflo = wspd * geo_ld<ND, R>(a.cgeo + 1 * a.ncell + icl);
     // pra / (pra + TINY) is exactly 1 whenever TINY does not change pra (any
     // pressure above ~1e-44 in FP64), so the division is taken only below.
     R const prt = pra + Tiny<R>::CFL;
@@ -539,7 +510,7 @@ __device__ __forceinline__ void dsoln_cell(MarchArgs<R, G> const & a, int64_t ic
             }
             else
             {
-                idis[f][d] = fg_late<ND>(a, f, D::K_P + d, icl) + tau * fg<ND>(a, f, D::K_Q + d, icl);
+                idis[f][d] = fg<ND>(a, f, D::K_P + d, icl) + tau * fg<ND>(a, f, D::K_Q + d, icl);
             }
         }
     }

@@ -40,22 +40,6 @@ struct MeshView
 // cell icl, its face count and faces, each face's two cells (one of them icl)
 // and its node count and nodes.  Reads only inside the tables; the first bad
 // cell lands in *bad (atomicMin).
-// Count the values of an FP64 geometry table that the FP32 march's rounding
-// (geo_r) does not take.
-__global__ void k_geo_range(double const * g, int64_t n, unsigned long long * bad)
-{
-    unsigned long long cnt = 0;
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x)
-    {
-        cnt += geo_r_takes(g[i]) ? 0ull : 1ull;
-    }
-    if (cnt)
-    {
-        atomicAdd(bad, cnt);
-    }
-}
-
 __global__ void k_validate_mesh(MeshView m, int64_t nface, int64_t nnode, unsigned long long * bad)
 {
     int64_t const icl = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -249,13 +233,35 @@ __global__ void k_prepare_ce_3d(MeshView m, CeView ce)
     }
 }
 
+// A geometry value (computed in FP64) as the march's tables store it.  The
+// FP32 form's tables are rounded here, once (geo_r, or the conversion
+// instruction, which keeps FP32 subnormals, where the 3D march reads the
+// value with `conv`); a value that FP32 cannot hold is counted in *bad.
+template <int ND, typename G>
+__device__ __forceinline__ G geo_store(double v, bool conv, unsigned long long * bad)
+{
+    if constexpr (std::is_same<G, Rounded>::value)
+    {
+        if (!geo_r_takes(v))
+        {
+            atomicAdd(bad, 1ull);
+        }
+        return Rounded{ND == 3 && conv ? float(v) : geo_r(v)};
+    }
+    else
+    {
+        return G(v);
+    }
+}
+
 // Compact the reference-layout CE geometry into the march's per-face
 // moments and per-cell scalars (layout in euler_device.cuh), in FP64, then
-// store them as G.  Also writes the neighbour-row table and the cell types.
+// store them as G (*bad: see geo_store, used for G = Rounded).  Also writes the
+// neighbour-row table and the cell types.
 template <int ND, typename G>
 __global__ void k_compact(MeshView m, double const * cevol, double const * cecnd, double const * sfcnd,
                           double const * sfnml, double hdt, int nslot, G * fgeo, G * cgeo, int32_t * nbr,
-                          int8_t * ctype)
+                          int8_t * ctype, unsigned long long * bad)
 {
     using D = Geo<ND, G>;
     int64_t const icl = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -280,7 +286,10 @@ __global__ void k_compact(MeshView m, double const * cevol, double const * cecnd
         B[d] = 0.0;
     }
     double dist = 1.79769313486231570815e+308;
-    auto put = [&](int f, int k, double v) { fgeo[(static_cast<int64_t>(f) * D::KF + k) * nc + icl] = G(v); };
+    auto put = [&](int f, int k, double v) {
+        bool const conv = !D::MID && k >= D::K_P && k < D::K_P + ND;
+        fgeo[(static_cast<int64_t>(f) * D::KF + k) * nc + icl] = geo_store<ND, G>(v, conv, bad);
+    };
     for (int f = 0; f < clnfc; ++f)
     {
         int const ifl = f + 1;
@@ -364,8 +373,8 @@ __global__ void k_compact(MeshView m, double const * cevol, double const * cecnd
             put(f, k, 0.0);
         }
     }
-    cgeo[0 * nc + icl] = G(1.0 / cevol[row * 7]);
-    cgeo[1 * nc + icl] = G(hdt / dist);
+    cgeo[0 * nc + icl] = geo_store<ND, G>(1.0 / cevol[row * 7], true, bad);
+    cgeo[1 * nc + icl] = geo_store<ND, G>(hdt / dist, true, bad);
 }
 
 } // namespace dev

@@ -33,7 +33,7 @@ _ID = {n: i for i, n in enumerate(ARRAYS)}
 _OPS = {"prepare_ce": 0, "update": 1, "calc_solt": 2, "calc_soln": 3,
         "bc_soln": 4, "calc_cfl": 5, "calc_dsoln": 6, "bc_dsoln": 7,
         "march_substep": 8, "reset_state": 9}
-# "fp32" is the FP32 form (FP32 state and flux, FP64 geometry tables);
+# "fp32" is the FP32 form (FP32 state and flux, geometry formed in FP64);
 # "fp32-geom64" names the same; "fp32-geom32" also stores the geometry FP32.
 PRECISIONS = {"fp64": 0, "fp32": 1, "fp32-geom64": 1, "fp32-geom32": 2}
 _SWAP = (("so0c", "so0n"), ("so1c", "so1n"))
@@ -50,10 +50,11 @@ class EulerCore:
     :param time_increment: the fixed time step.
     :param precision: ``"fp64"`` (the reference's arithmetic), ``"fp32"``
         (not in the reference: FP32 state and flux arithmetic with
-        compensated face sums, the mesh geometry in FP64 tables, totals and
-        the CFL reduction in FP64; ``"fp32-geom64"`` is the same) or
-        ``"fp32-geom32"`` (the same march with the geometry, computed in FP64,
-        stored in FP32: less traffic, slightly larger error).
+        compensated face sums, the mesh geometry formed in FP64 and each
+        value the march uses rounded once to FP32, totals and the CFL
+        reduction in FP64; ``"fp32-geom64"`` is the same) or
+        ``"fp32-geom32"`` (the same march with part of the geometry formed
+        in FP32 from fewer stored values: slightly larger error).
     """
 
     SUBSTEP_RUN = 2
