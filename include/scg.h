@@ -445,6 +445,11 @@ int scg_geometry_round(const double * in, float * out, int64_t n);
  * (Newton's iteration, within one ulp of 1 / d).  Synchronous; allocates its
  * own device buffers. */
 int scg_divide_check(const double * x, const double * d, double * q, double * qdiv, double * rcp, int64_t n);
+/* Not in the reference: the FP64 march's reciprocal roots r[i] = 1 / sqrt(x[i])
+ * and roots s[i] = sqrt(x[i]) on the device, formed on the integer pipe for
+ * positive normal x (within 0.52 ulp; other x by the library functions), for
+ * checking them.  Synchronous; allocates its own device buffers. */
+int scg_root_check(const double * x, double * r, double * s, int64_t n);
 /* Device FMA throughput in TFLOP/s for SCG_FP64 or SCG_FP32 (a register-only
  * FMA chain over all SMs, iters FMAs-per-accumulator). */
 int scg_fma_peak(int precision, int iters, double * tflops);

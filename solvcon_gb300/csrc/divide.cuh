@@ -1,5 +1,6 @@
 /*
- * FP64 divisions that cost fewer FP64 instructions than the IEEE division.
+ * FP64 divisions and roots that cost fewer FP64-pipe instructions than the
+ * IEEE operations.
  *
  * div_rcp: division by a tabulated reciprocal, rounded exactly as x / d.
  *
@@ -27,8 +28,8 @@
  * divides.  The results equal CUDA's IEEE division bit for bit; the device
  * check scg_divide_check compares the two.
  *
- * recip: a reciprocal within one ulp, for the marches whose results are
- * compared to round-off (below).
+ * recip, rsq, sqr_t: reciprocals and roots within 0.52 ulp, on the integer
+ * pipe (below).
  */
 #pragma once
 
@@ -70,47 +71,160 @@ __device__ __forceinline__ double div_rcp(double x, double d, double r)
     return div_plain(x, d);
 }
 
-// Reciprocal.  FP64: Newton's iteration r <- r + r (1 - d r) from the FP32
-// hardware approximation of the reciprocal of d's significand (its top 23
-// bits), rescaled by d's exponent; each step squares the relative error, so
-// two take it from ~2^-22 below 2^-86 and r is within one ulp of 1 / d, in
-// four fused multiply-adds (a correctly rounded division takes about twice
-// as many FP64 instructions).  That holds for |d| in [2^-1022, 2^1022);
-// outside it (zero, subnormals, the largest magnitudes, infinities, NaN) the
-// division replaces the result, behind a branch inside one asm statement.
-// The compiler then sees no branch, as it sees none in a division
-// instruction: with the edges taken by branches or selects it could see,
-// kernels inlining this in different code contracted the callers'
-// multiply-adds differently, and batched and single-core marches no longer
-// rounded alike.  A predicated division instead of the branch was issued at
-// every call.  FP32: the division.
+// ---------------------------------------------------------------------------
+// Reciprocals and roots on the integer pipe.
+//
+// GB300 issues one FP64 instruction per SM every 16 cycles, and the FP64
+// marches keep that pipe ~88% busy while the integer and FP32 pipes idle (8%
+// of the issue slots used), so these functions form their results with
+// integer instructions alone: Newton's iteration in fixed point from the FP32
+// hardware approximation, the residual kept exactly or to 62 bits, the result
+// rounded once to 53 bits.  About 30 (recip), 40 (rsq) and 48 (sqr) integer
+// instructions in place of 4, 5 and 8 of the FP64 pipe (a triangle's substep
+// takes 6, 12 and 2 of them, a hexahedron's 15, 40 and 2).
+// Results are within 0.52 ulp (scg_divide_check and scg_root_check compare
+// them on the device).
+//
+// Operands outside the stated ranges take the division or the library
+// function behind a branch that such values alone take.
+
+// |d|'s top 24 significand bits as a float in [1, 2).
+__device__ __forceinline__ float sig_top(unsigned hi, unsigned lo)
+{
+    return __uint_as_float((127u << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29));
+}
+
+// A seed y in (0.5, 1] as a 24-bit integer y 2^24, kept inside [2^23, 2^24).
+__device__ __forceinline__ unsigned seed24(float y)
+{
+    unsigned const b = min(max(__float_as_uint(y), 0x3f000000u), 0x3f7fffffu);
+    return (b & 0x7fffffu) | 0x800000u;
+}
+
+// t * y for a signed 64-bit t and y below 2^24, modulo 2^64.
+__device__ __forceinline__ long long mul_s64_u24(long long t, unsigned y)
+{
+    unsigned long long const u = static_cast<unsigned long long>(t);
+    unsigned long long const lo = static_cast<unsigned long long>(static_cast<unsigned>(u)) * y;
+    return static_cast<long long>(lo + (static_cast<unsigned long long>(static_cast<unsigned>(u >> 32) * y) << 32));
+}
+
+// a * b / 2^64 up to two units of the result.
+__device__ __forceinline__ unsigned long long mul_hi64(unsigned long long a, unsigned long long b)
+{
+    unsigned const ah = static_cast<unsigned>(a >> 32), al = static_cast<unsigned>(a);
+    unsigned const bh = static_cast<unsigned>(b >> 32), bl = static_cast<unsigned>(b);
+    return static_cast<unsigned long long>(ah) * bh + __umulhi(ah, bl) + __umulhi(al, bh);
+}
+
+// Reciprocal.  FP64, |d| in [2^-1022, 2^1022): with m = |d|'s significand
+// (m 2^52 an integer) and the seed y = Y 2^-24, the residual e = 1 - m y is
+// exact in the low 64 bits of the product (|e| < 2^-21), and
+// 1 / m = y (1 + e + e^2) up to 2^-65.  Outside that range (zero, subnormals,
+// the largest magnitudes, infinities, NaN) the division.  FP32: the division.
 __device__ __forceinline__ double recip(double d)
 {
     unsigned const hi = static_cast<unsigned>(__double2hiint(d));
+    unsigned const lo = static_cast<unsigned>(__double2loint(d));
     unsigned const e = (hi >> 20) & 0x7ffu;
-    float const m =
-        __uint_as_float((127u << 23) | ((hi & 0xfffffu) << 3) | (static_cast<unsigned>(__double2loint(d)) >> 29));
+    if (e - 1u > 2043u)
+    {
+        return 1.0 / d;
+    }
     float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(m));
-    unsigned const yb = __float_as_uint(y);
-    double r = __hiloint2double(static_cast<int>(((yb >> 3) + (896u << 20) - ((e - 1023u) << 20)) | (hi & 0x80000000u)),
-                                static_cast<int>(yb << 29));
-    double t = __fma_rn(-d, r, 1.0);
-    r = __fma_rn(r, t, r);
-    t = __fma_rn(-d, r, 1.0);
-    r = __fma_rn(r, t, r);
-    asm("{\n\t"
-        ".reg .pred p;\n\t"
-        "setp.le.u32 p, %2, 2043;\n\t"
-        "@p bra RCP_DONE;\n\t"
-        "div.rn.f64 %0, 0d3FF0000000000000, %1;\n\t"
-        "RCP_DONE:\n\t"
-        "}"
-        : "+d"(r)
-        : "d"(d), "r"(e - 1u));
-    return r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(sig_top(hi, lo)));
+    unsigned const Y = seed24(y);
+    unsigned long long const m =
+        (static_cast<unsigned long long>((hi & 0xfffffu) | 0x100000u) << 32) | lo;
+    long long const E = -mul_s64_u24(static_cast<long long>(m), Y); // e 2^76
+    int const Es = static_cast<int>(E >> 24);                       // e 2^52
+    long long const T = (E >> 14) + (static_cast<long long>(Es) * Es >> 42); // (e + e^2) 2^62
+    unsigned long long const r = (static_cast<unsigned long long>(Y) << 38) +
+                                 static_cast<unsigned long long>(mul_s64_u24((T + 4) >> 3, Y) >> 21); // 2^62 / m
+    unsigned long long const bits = ((r + 256u) >> 9) + (static_cast<unsigned long long>(2044u - e) << 52);
+    return __longlong_as_double(static_cast<long long>(bits | (static_cast<unsigned long long>(hi & 0x80000000u) << 32)));
 }
 __device__ __forceinline__ float recip(float d) { return 1.0f / d; }
+
+// Whether x is a positive normal number.
+__device__ __forceinline__ bool pos_normal(unsigned hi) { return hi - 0x00100000u < 0x7fe00000u; }
+
+// Reciprocal root of m in [1, 4), the significand of a positive normal x
+// taken with its exponent's parity: x = m 4^h.  X = m 2^62; returns
+// 2^62 / sqrt(m).  With the seed y, e = 1 - m y^2 to 2^-61 (|e| < 2^-20) and
+// 1 / sqrt(m) = y (1 + e / 2 + 3 e^2 / 8) up to 2^-61.
+__device__ __forceinline__ unsigned long long rsq_fixed(unsigned hi, unsigned lo, unsigned long long & X, int & h)
+{
+    int const k = static_cast<int>(hi >> 20) - 1023;
+    h = k >> 1;
+    unsigned const odd = static_cast<unsigned>(k) & 1u;
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint_as_float(__float_as_uint(sig_top(hi, lo)) + (odd << 23))));
+    unsigned const Y = seed24(y);
+    X = ((static_cast<unsigned long long>((hi & 0xfffffu) | 0x100000u) << 32) | lo) << (10u + odd);
+    unsigned long long const Z = static_cast<unsigned long long>(Y) * Y << 16; // y^2 2^64
+    long long const E = static_cast<long long>((1ull << 62) - mul_hi64(X, Z)); // e 2^62
+    int const Es = static_cast<int>(E >> 12);                                   // e 2^50
+    unsigned const sq = static_cast<unsigned>(static_cast<unsigned long long>(static_cast<long long>(Es) * Es) >> 32);
+    long long const T = E + static_cast<long long>(sq * 3u >> 8); // (e + 3 e^2 / 4) 2^62
+    return (static_cast<unsigned long long>(Y) << 38) +
+           static_cast<unsigned long long>(mul_s64_u24((T + 4) >> 3, Y) >> 22);
+}
+
+// 1 / sqrt(x): FP64 positive normal x as above, else the library's; FP32 the
+// library's.
+__device__ __forceinline__ double rsq(double x)
+{
+    unsigned const hi = static_cast<unsigned>(__double2hiint(x));
+    if (!pos_normal(hi))
+    {
+        return rsqrt(x);
+    }
+    unsigned long long X;
+    int h;
+    unsigned long long const r = rsq_fixed(hi, static_cast<unsigned>(__double2loint(x)), X, h);
+    return __longlong_as_double(
+        static_cast<long long>(((r + 256u) >> 9) + (static_cast<unsigned long long>(1021 - h) << 52)));
+}
+__device__ __forceinline__ float rsq(float x) { return rsqrtf(x); }
+
+// sqrt(x) = x / sqrt(x): FP64 positive normal x and zero, else the library's;
+// FP32 the library's.
+__device__ __forceinline__ double sqr_t(double x)
+{
+    unsigned const hi = static_cast<unsigned>(__double2hiint(x));
+    unsigned const lo = static_cast<unsigned>(__double2loint(x));
+    if (!pos_normal(hi))
+    {
+        return ((hi << 1) | lo) == 0u ? x : sqrt(x);
+    }
+    unsigned long long X;
+    int h;
+    unsigned long long const r = rsq_fixed(hi, lo, X, h);
+    unsigned long long const q = mul_hi64(X, r); // sqrt(m) 2^60
+    return __longlong_as_double(
+        static_cast<long long>(((q + 128u) >> 8) + (static_cast<unsigned long long>(1022 + h) << 52)));
+}
+__device__ __forceinline__ float sqr_t(float x) { return sqrtf(x); }
+
+// Comparisons of FP64 values on the integer pipe (a DSETP issues on the FP64
+// pipe): the bit patterns of non-negative values order as signed integers,
+// and every negative value's is below them.
+__device__ __forceinline__ bool lt_nonneg(double a, double b) // a < b for a >= 0
+{
+    return __double_as_longlong(a) < __double_as_longlong(b);
+}
+__device__ __forceinline__ double max_pos(double m, double u) // the larger of u and m >= +0
+{
+    return lt_nonneg(m, u) ? u : m;
+}
+__device__ __forceinline__ double min_neg(double m, double u) // the smaller of u and m <= -0
+{
+    return static_cast<unsigned long long>(__double_as_longlong(m)) <
+                   static_cast<unsigned long long>(__double_as_longlong(u))
+               ? u
+               : m;
+}
 
 } // namespace dev
 } // namespace scg

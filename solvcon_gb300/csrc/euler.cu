@@ -40,29 +40,53 @@ inline unsigned grid_for(int64_t n)
 // --------------------------------------------------------------------------
 // Per-operation kernels (one thread per row or body cell).
 
+// calc_solt of a row whose so0 and so1 are v's: so0t and (FP64) the flux terms
+// into its record.
 template <int ND, typename R>
-__global__ void k_solt_rows(R * rec, R const * gamma, int64_t nrow)
+__device__ __forceinline__ void solt_record(R * row, R const * v, R ga, R qdt)
 {
     constexpr int NEQ = ND + 2;
+    using RC = Rec<ND, R>;
+    R t[NEQ];
+    if constexpr (RC::TERMS)
+    {
+        R c[FluxTerms<ND>::N];
+        solt_terms<ND>(v, v + 2 * NEQ, ga, qdt, t, c);
+#pragma unroll
+        for (int i = 0; i < FluxTerms<ND>::N; ++i)
+        {
+            row[RC::OP + i] = c[i];
+        }
+    }
+    else
+    {
+        (void)qdt;
+        solt_prim<ND, R>(Prim<ND, R>(v, ga), v, v + 2 * NEQ, t);
+    }
+#pragma unroll
+    for (int i = 0; i < NEQ; ++i)
+    {
+        row[NEQ + i] = t[i];
+    }
+}
+
+template <int ND, typename R>
+__global__ void k_solt_rows(R * rec, R const * gamma, int64_t nrow, R qdt)
+{
     int64_t const r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (r >= nrow)
     {
         return;
     }
     using RC = Rec<ND, R>;
+    R * const row = rec + r * RC::RS;
     R v[RC::NUSED];
-    load_rec<ND, R>(rec + r * RC::RS, v);
-    R t[NEQ];
-    Prim<ND, R> const q(v, gamma[r]);
-    solt_prim<ND, R>(q, v, v + 2 * NEQ, t);
-    for (int i = 0; i < NEQ; ++i)
+#pragma unroll
+    for (int i = 0; i < RC::NUSED; ++i)
     {
-        rec[r * RC::RS + NEQ + i] = t[i];
+        v[i] = row[i];
     }
-    if constexpr (RC::PRIM)
-    {
-        q.cache(rec + r * RC::RS + RC::OP);
-    }
+    solt_record<ND, R>(row, v, gamma[r], qdt);
 }
 
 template <int ND, typename R>
@@ -79,6 +103,24 @@ __global__ void k_copy_field(R const * src, R * dst, int64_t nrow, int off, int 
     }
 }
 
+// One cell's calc_soln, calc_cfl or calc_dsoln in either precision.
+template <int CT, typename R, typename G>
+__device__ __forceinline__ void soln_any(MarchArgs<R, G> const & a, int64_t icl, R * so0n)
+{
+    if constexpr (sizeof(R) == 8)
+        soln64<CT, false>(a, icl, so0n);
+    else
+        soln_cell<CT, R, G>(a, icl, so0n);
+}
+template <int CT, typename R, typename G>
+__device__ __forceinline__ void dsoln_any(MarchArgs<R, G> const & a, int64_t icl, R const * so0n, R cflc, R * so1n)
+{
+    if constexpr (sizeof(R) == 8)
+        dsoln64<CT>(a, icl, so0n, cflc, so1n);
+    else
+        dsoln_cell<CT, R, G>(a, icl, so0n, cflc, so1n);
+}
+
 template <int ND, typename R, typename G>
 __global__ void k_soln(MarchArgs<R, G> a)
 {
@@ -93,18 +135,18 @@ __global__ void k_soln(MarchArgs<R, G> a)
     if constexpr (ND == 2)
     {
         if (ct == 4)
-            soln_cell<4, R, G>(a, icl, so0n);
+            soln_any<4>(a, icl, so0n);
         else
-            soln_cell<3, R, G>(a, icl, so0n);
+            soln_any<3>(a, icl, so0n);
     }
     else
     {
         switch (ct)
         {
-        case 6: soln_cell<6, R, G>(a, icl, so0n); break;
-        case 5: soln_cell<5, R, G>(a, icl, so0n); break;
-        case 7: soln_cell<7, R, G>(a, icl, so0n); break;
-        default: soln_cell<8, R, G>(a, icl, so0n); break;
+        case 6: soln_any<6>(a, icl, so0n); break;
+        case 5: soln_any<5>(a, icl, so0n); break;
+        case 7: soln_any<7>(a, icl, so0n); break;
+        default: soln_any<8>(a, icl, so0n); break;
         }
     }
     R * out = a.nxt + (icl + a.ngst) * Rec<ND, R>::RS;
@@ -131,7 +173,10 @@ __global__ void k_cfl(MarchArgs<R, G> a)
         s[i] = out[i];
     }
     R rinv;
-    cfl_cell<ND, R, G>(a, icl, row, s, rinv);
+    if constexpr (sizeof(R) == 8)
+        cfl64<ND>(a, icl, row, s, rinv);
+    else
+        cfl_cell<ND, R, G>(a, icl, row, s, rinv);
     out[NEQ - 1] = s[NEQ - 1];
 }
 
@@ -157,18 +202,18 @@ __global__ void k_dsoln(MarchArgs<R, G> a)
     if constexpr (ND == 2)
     {
         if (ct == 4)
-            dsoln_cell<4, R, G>(a, icl, s, cflc, g);
+            dsoln_any<4>(a, icl, s, cflc, g);
         else
-            dsoln_cell<3, R, G>(a, icl, s, cflc, g);
+            dsoln_any<3>(a, icl, s, cflc, g);
     }
     else
     {
         switch (ct)
         {
-        case 6: dsoln_cell<6, R, G>(a, icl, s, cflc, g); break;
-        case 5: dsoln_cell<5, R, G>(a, icl, s, cflc, g); break;
-        case 7: dsoln_cell<7, R, G>(a, icl, s, cflc, g); break;
-        default: dsoln_cell<8, R, G>(a, icl, s, cflc, g); break;
+        case 6: dsoln_any<6>(a, icl, s, cflc, g); break;
+        case 5: dsoln_any<5>(a, icl, s, cflc, g); break;
+        case 7: dsoln_any<7>(a, icl, s, cflc, g); break;
+        default: dsoln_any<8>(a, icl, s, cflc, g); break;
         }
     }
     for (int i = 0; i < NEQ * ND; ++i)
@@ -430,7 +475,7 @@ __global__ void k_chunk_top_row(int32_t const * nbr, int8_t const * ctype, int64
 
 // so1n written from a mapped host table and then calc_solt of each row as
 // it now stands (its so0 already in the record): the next march finds so0t
-// and the FP64 primitive cache of the new state made, and the Jacobian
+// and the FP64 flux terms of the new state made, and the Jacobian
 // products run while other blocks wait on the host link.  A block copies its
 // rows' contiguous stretch of the host table to shared memory in 16-byte
 // pieces (vec: the table is 16-byte aligned; a block's stretch starts at a
@@ -439,7 +484,7 @@ __global__ void k_chunk_top_row(int32_t const * nbr, int8_t const * ctype, int64
 // k_set_field_host followed by k_solt_rows.
 template <int ND, typename R>
 __global__ void __launch_bounds__(BLOCK) k_set_so1_host_solt(R * rec, double const * in, R const * gamma,
-                                                             int64_t nrow, bool vec)
+                                                             int64_t nrow, bool vec, R qdt)
 {
     constexpr int NEQ = ND + 2;
     constexpr int W = NEQ * ND;
@@ -487,23 +532,12 @@ __global__ void __launch_bounds__(BLOCK) k_set_so1_host_solt(R * rec, double con
             {
                 v[2 * NEQ + k] = R(buf[threadIdx.x * W + k]);
             }
-            Prim<ND, R> const q(v, gamma[r]);
-            R t[NEQ];
-            solt_prim<ND, R>(q, v, v + 2 * NEQ, t);
-#pragma unroll
-            for (int i = 0; i < NEQ; ++i)
-            {
-                row[NEQ + i] = t[i];
-            }
 #pragma unroll
             for (int k = 0; k < W; ++k)
             {
                 row[2 * NEQ + k] = v[2 * NEQ + k];
             }
-            if constexpr (RC::PRIM)
-            {
-                q.cache(row + RC::OP);
-            }
+            solt_record<ND, R>(row, v, gamma[r], qdt);
         }
     }
 }
@@ -1271,7 +1305,8 @@ public:
                     // The new state's so0t can go into its record (the
                     // logical so0t lives in the other buffer): make it now.
                     k_set_so1_host_solt<ND, R><<<grid_for(nrow), BLOCK, 0, stream>>>(
-                        base, dev, d_gamma.ptr, nrow, reinterpret_cast<uintptr_t>(dev) % 16 == 0);
+                        base, dev, d_gamma.ptr, nrow, reinterpret_cast<uintptr_t>(dev) % 16 == 0,
+                        R(time_increment * 0.25));
                     launched(stream, "set_so1_host_solt");
                     next_valid = true;
                     next_buf = cur ^ 1;
@@ -1364,7 +1399,8 @@ public:
 
     void run_solt()
     {
-        k_solt_rows<ND, R><<<grid_for(nrow), BLOCK, 0, stream>>>(rec[cur].ptr, d_gamma.ptr, nrow);
+        k_solt_rows<ND, R><<<grid_for(nrow), BLOCK, 0, stream>>>(rec[cur].ptr, d_gamma.ptr, nrow,
+                                                                 R(time_increment * 0.25));
         launched(stream, "calc_solt");
         tbuf = cur;
     }
@@ -1638,7 +1674,8 @@ public:
             if (solt)
             {
                 k_set_so1_host_solt<ND, R><<<grid_for(nr), BLOCK, 0, m_xfer>>>(
-                    base + r0 * RS, in1, d_gamma.ptr + r0, nr, reinterpret_cast<uintptr_t>(in1) % 16 == 0);
+                    base + r0 * RS, in1, d_gamma.ptr + r0, nr, reinterpret_cast<uintptr_t>(in1) % 16 == 0,
+                    R(time_increment * 0.25));
                 launched(m_xfer, "set_so1_host_solt");
             }
             else
@@ -1855,7 +1892,8 @@ public:
         // kernel, minus the buffer swap: so0t of the state in rec[cur ^ 1].
         if (!(next_valid && next_buf == (cur ^ 1)) && nrow > 0)
         {
-            k_solt_rows<ND, R><<<grid_for(nrow), BLOCK, 0, stream>>>(rec[cur ^ 1].ptr, d_gamma.ptr, nrow);
+            k_solt_rows<ND, R><<<grid_for(nrow), BLOCK, 0, stream>>>(rec[cur ^ 1].ptr, d_gamma.ptr, nrow,
+                                                                     R(time_increment * 0.25));
             launched(stream, "calc_solt");
             next_valid = true;
             next_buf = cur ^ 1;
@@ -2087,7 +2125,7 @@ private:
 
     int cur = 0;           // index of the current (so0c/so1c) record buffer
     int tbuf = 0;          // buffer holding the logical so0t
-    bool next_valid = false; // rec[next_buf].so0t (and its primitive cache) == calc_solt of rec[next_buf]
+    bool next_valid = false; // rec[next_buf].so0t (and its flux terms) == calc_solt of rec[next_buf]
     bool async_pending = false; // march() returned with its kernels possibly still running
     int next_buf = 1;
 };

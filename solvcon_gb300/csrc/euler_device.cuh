@@ -28,13 +28,15 @@
  *
  * Results equal the reference's up to floating-point round-off.
  *
+ * This file holds what both precisions share and the FP32 march's building
+ * blocks; euler_fp64.cuh has the FP64 march's.
+ *
  * Storage (one record per mesh row, ghost rows first, row = icl + ngstcell):
- *   record[row] = { so0[NEQ], so0t[NEQ], so1[NEQ][ND], prim } padded to RS
- * reals, where prim (FP64 records only) caches the primitive variables of so0
- * (1/rho, v, p, E + p, |v|^2).  It is written with so0t, by the same thread
- * and from the same state, so it is valid exactly when so0t is; the fused
- * march then reads a neighbour's primitives instead of re-deriving them for
- * every face (a division and about twenty FP64 operations each).
+ *   record[row] = { so0[NEQ], so0t[NEQ], so1[NEQ][ND], terms } padded to RS
+ * reals, where terms (FP64 records only) are the row's flux terms: functions
+ * of its so0, so1 and so0t that calc_soln reads for each of the row's faces
+ * (euler_fp64.cuh).  They are written with so0t, by the same thread and from
+ * the same state, so they are valid exactly when so0t is.
  */
 
 #include "divide.cuh"
@@ -68,8 +70,8 @@ struct Rounded
     float v;
 };
 
-// Per-face geometry components, stored as G: bvol, dB[ND] = x_BCE - x_nbr,
-// Nh[ND], Mh[ND][ND], then either the gradient-element displacements P[ND],
+// Per-face geometry components, stored as G: bvol, dB[ND] = x_BCE - x_nbr
+// (G double: bvol dB), Nh[ND], Mh[ND][ND], then either the gradient-element displacements P[ND],
 // Q[ND], R[ND] (geometry computed in FP64: G double or Rounded) or
 // mid[ND] = x_BCE - x_cell (fp32-geom32: G float).
 // P, Q and R follow from dB and mid with means over the cell's faces:
@@ -97,13 +99,15 @@ struct Rec
 {
     static constexpr int NEQ = ND + 2;
     static constexpr int NUSED = 2 * NEQ + NEQ * ND; // so0, so0t, so1: 16 / 25
-    // Primitive cache (FP64 only: the FP64 march is bound by the FP64 pipe,
-    // the FP32 march by memory, where the extra bytes would cost more).
-    static constexpr bool PRIM = sizeof(R) == 8;
-    static constexpr int OP = NUSED;    // cache offset: r, v[ND], p, h, vsq
-    static constexpr int NPRIM = ND + 4;
-    static constexpr int NLOAD = PRIM ? NUSED + NPRIM : NUSED;
-    static constexpr int RS = (ND == 2) ? (PRIM ? 24 : 16) : 32;
+    // Flux terms (FP64 only: the FP64 march is bound by the FP64 pipe, the
+    // FP32 march by memory, where the extra bytes would cost more); see
+    // euler_fp64.cuh.
+    static constexpr bool TERMS = sizeof(R) == 8;
+    static constexpr int OP = NUSED; // their offset
+    static constexpr int NTERM = ND == 2 ? 17 : 39;
+    static constexpr int NLOAD = TERMS ? NUSED + NTERM : NUSED;
+    // 2D FP64: 33 values in 36 reals (nine whole 32-byte sectors).
+    static constexpr int RS = TERMS ? (ND == 2 ? 36 : 64) : (ND == 2 ? 16 : 32);
     static_assert(NLOAD <= RS, "record overflow");
 };
 
@@ -172,30 +176,16 @@ __device__ __forceinline__ R geo_val(G v)
     }
 }
 
-// Reciprocal square root: the library routine for each precision.
-__device__ __forceinline__ double rsq(double x) { return rsqrt(x); }
-__device__ __forceinline__ float rsq(float x) { return rsqrtf(x); }
-
-__device__ __forceinline__ double sqr_t(double x) { return sqrt(x); }
-__device__ __forceinline__ float sqr_t(float x) { return sqrtf(x); }
-
-
-// The march's reciprocals and quotients.  FP64: recip (Newton) and the
-// division.  FP32 in 2D: the approximate quotient (div.approx.f32, one
-// instruction and within 2 ulp for divisors of magnitude in [2^-126, 2^126];
-// a zero divisor gives a signed infinity, or NaN over zero, as the division
-// does), where a correctly rounded FP32 division is a multi-instruction
-// sequence with a branch and the 2D march divides about a dozen times per
-// cell-substep by densities, determinants, weight sums and CFL numbers, all
-// far inside that range (2M triangles: 0.2352 -> 0.2155 ms per launch).
-// FP32 in 3D: the division (with the approximate quotient the tetrahedron
-// kernel ran 6.45 -> 8.59 ms per launch at the same registers, scheduled
-// differently).
-template <int ND>
-__device__ __forceinline__ double mrecip(double d)
-{
-    return recip(d);
-}
+// The FP32 march's reciprocals and quotients.  2D: the approximate quotient
+// (div.approx.f32, one instruction and within 2 ulp for divisors of magnitude
+// in [2^-126, 2^126]; a zero divisor gives a signed infinity, or NaN over
+// zero, as the division does), where a correctly rounded FP32 division is a
+// multi-instruction sequence with a branch and the 2D march divides about a
+// dozen times per cell-substep by densities, determinants, weight sums and
+// CFL numbers, all far inside that range (2M triangles: 0.2352 -> 0.2155 ms
+// per launch).  3D: the division (with the approximate quotient the
+// tetrahedron kernel ran 6.45 -> 8.59 ms per launch at the same registers,
+// scheduled differently).
 template <int ND>
 __device__ __forceinline__ float mrecip(float d)
 {
@@ -203,11 +193,6 @@ __device__ __forceinline__ float mrecip(float d)
         return __fdividef(1.0f, d);
     else
         return 1.0f / d;
-}
-template <int ND>
-__device__ __forceinline__ double mquot(double x, double y)
-{
-    return x / y;
 }
 template <int ND>
 __device__ __forceinline__ float mquot(float x, float y)
@@ -218,16 +203,8 @@ __device__ __forceinline__ float mquot(float x, float y)
         return x / y;
 }
 
-// Compensated (Kahan) accumulator for the FP32 flux sums; plain sum in FP64.
-template <typename R>
+// Compensated (Kahan) accumulator for the FP32 flux sums.
 struct Acc
-{
-    R s = R(0);
-    __device__ __forceinline__ void add(R x) { s += x; }
-    __device__ __forceinline__ R value() const { return s; }
-};
-template <>
-struct Acc<float>
 {
     float s = 0.f;
     float c = 0.f;
@@ -271,38 +248,6 @@ struct Prim
         ga1 = ga - R(1);
         p = ga1 * (u[NEQ - 1] - R(0.5) * ke2);
         h = u[NEQ - 1] + p;
-    }
-
-    Prim() = default;
-
-    // From a record's primitive cache (see Rec).
-    __device__ __forceinline__ static Prim cached(R const * c, R ga)
-    {
-        Prim q;
-        q.r = c[0];
-#pragma unroll
-        for (int d = 0; d < ND; ++d)
-        {
-            q.v[d] = c[1 + d];
-        }
-        q.p = c[1 + ND];
-        q.h = c[2 + ND];
-        q.vsq = c[3 + ND];
-        q.ga1 = ga - R(1);
-        return q;
-    }
-
-    __device__ __forceinline__ void cache(R * c) const
-    {
-        c[0] = r;
-#pragma unroll
-        for (int d = 0; d < ND; ++d)
-        {
-            c[1 + d] = v[d];
-        }
-        c[1 + ND] = p;
-        c[2 + ND] = h;
-        c[3 + ND] = vsq;
     }
 };
 
@@ -503,6 +448,32 @@ struct MarchArgs
     R dt, hdt, qdt;
     R sigma0, taumin, tauscale;
 };
+
+template <typename T>
+__device__ __forceinline__ T ldg(T const * p)
+{
+    return __ldg(p);
+}
+
+// A geometry table value, loaded once per cell-substep and streamed.
+template <int ND, typename R, typename G>
+__device__ __forceinline__ R geo_ld(G const * p)
+{
+    if constexpr (std::is_same<G, Rounded>::value)
+    {
+        return ldg(&p->v);
+    }
+    else
+    {
+        return geo_val<R>(ldg(p));
+    }
+}
+
+template <int ND, typename R, typename G>
+__device__ __forceinline__ R fg(MarchArgs<R, G> const & a, int f, int k, int64_t icl)
+{
+    return geo_ld<ND, R>(a.fgeo + (static_cast<int64_t>(f) * Geo<ND, G>::KF + k) * a.ncell + icl);
+}
 
 } // namespace dev
 } // namespace scg

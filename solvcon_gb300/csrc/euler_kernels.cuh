@@ -5,10 +5,12 @@
  * routines for calc_soln, bc_soln, calc_cfl, calc_dsoln, bc_dsoln and calc_solt,
  * the fused one-kernel substep built from them, and the set-up kernels
  * (prepare_ce and the geometry compaction).  See euler_device.cuh for the data
- * layout and for how the arithmetic relates to the reference's.
+ * layout and for how the arithmetic relates to the reference's, and
+ * euler_fp64.cuh for the FP64 march's own routines.
  */
 
 #include "euler_device.cuh"
+#include "euler_fp64.cuh"
 
 #include <type_traits>
 
@@ -17,60 +19,34 @@ namespace scg
 namespace dev
 {
 
-template <typename T>
-__device__ __forceinline__ T ldg(T const * p)
+// Load the first N reals of an FP32 record (default: so0, so0t, so1).
+template <int ND, int N = Rec<ND, float>::NUSED>
+__device__ __forceinline__ void load_rec(float const * base, float * out)
 {
-    return __ldg(p);
-}
-
-// Load the first N reals of a record (default: so0, so0t, so1).
-template <int ND, typename R, int N = Rec<ND, R>::NUSED>
-__device__ __forceinline__ void load_rec(R const * base, R * out)
-{
-    if constexpr (sizeof(R) == 8)
-    {
-        double2 const * p = reinterpret_cast<double2 const *>(base);
+    float4 const * p = reinterpret_cast<float4 const *>(base);
 #pragma unroll
-        for (int k = 0; k < N / 2; ++k)
-        {
-            double2 const v = __ldg(p + k);
-            out[2 * k] = v.x;
-            out[2 * k + 1] = v.y;
-        }
-        if constexpr (N % 2)
-        {
-            out[N - 1] = __ldg(base + N - 1);
-        }
+    for (int k = 0; k < N / 4; ++k)
+    {
+        float4 const v = __ldg(p + k);
+        out[4 * k] = v.x;
+        out[4 * k + 1] = v.y;
+        out[4 * k + 2] = v.z;
+        out[4 * k + 3] = v.w;
     }
-    else
+#pragma unroll
+    for (int k = (N / 4) * 4; k < N; ++k)
     {
-        float4 const * p = reinterpret_cast<float4 const *>(base);
-#pragma unroll
-        for (int k = 0; k < N / 4; ++k)
-        {
-            float4 const v = __ldg(p + k);
-            out[4 * k] = v.x;
-            out[4 * k + 1] = v.y;
-            out[4 * k + 2] = v.z;
-            out[4 * k + 3] = v.w;
-        }
-#pragma unroll
-        for (int k = (N / 4) * 4; k < N; ++k)
-        {
-            out[k] = __ldg(base + k);
-        }
+        out[k] = __ldg(base + k);
     }
 }
 
-// Store a record: so0, so0t, so1 and (FP64) the primitive cache of so0.
-template <int ND, typename R>
-__device__ __forceinline__ void store_rec(R * base, R const * so0, R const * so0t, R const * so1,
-                                          Prim<ND, R> const & q)
+// Store an FP32 record: so0, so0t, so1.
+template <int ND>
+__device__ __forceinline__ void store_rec(float * base, float const * so0, float const * so0t, float const * so1)
 {
     constexpr int NEQ = ND + 2;
-    using RC = Rec<ND, R>;
-    constexpr int N = RC::NLOAD;
-    R v[N];
+    constexpr int N = Rec<ND, float>::NUSED;
+    float v[N];
 #pragma unroll
     for (int i = 0; i < NEQ; ++i)
     {
@@ -82,61 +58,17 @@ __device__ __forceinline__ void store_rec(R * base, R const * so0, R const * so0
     {
         v[2 * NEQ + i] = so1[i];
     }
-    if constexpr (RC::PRIM)
-    {
-        q.cache(v + RC::OP);
-    }
-    else
-    {
-        (void)q;
-    }
-    if constexpr (sizeof(R) == 8)
-    {
-        double2 * p = reinterpret_cast<double2 *>(base);
+    float4 * p = reinterpret_cast<float4 *>(base);
 #pragma unroll
-        for (int k = 0; k < N / 2; ++k)
-        {
-            p[k] = make_double2(v[2 * k], v[2 * k + 1]);
-        }
-        if constexpr (N % 2)
-        {
-            base[N - 1] = v[N - 1];
-        }
-    }
-    else
+    for (int k = 0; k < N / 4; ++k)
     {
-        float4 * p = reinterpret_cast<float4 *>(base);
+        p[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+    }
 #pragma unroll
-        for (int k = 0; k < N / 4; ++k)
-        {
-            p[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
-        }
-#pragma unroll
-        for (int k = (N / 4) * 4; k < N; ++k)
-        {
-            base[k] = v[k];
-        }
-    }
-}
-
-// A geometry table value, loaded once per cell-substep and streamed.
-template <int ND, typename R, typename G>
-__device__ __forceinline__ R geo_ld(G const * p)
-{
-    if constexpr (std::is_same<G, Rounded>::value)
+    for (int k = (N / 4) * 4; k < N; ++k)
     {
-        return ldg(&p->v);
+        base[k] = v[k];
     }
-    else
-    {
-        return geo_val<R>(ldg(p));
-    }
-}
-
-template <int ND, typename R, typename G>
-__device__ __forceinline__ R fg(MarchArgs<R, G> const & a, int f, int k, int64_t icl)
-{
-    return geo_ld<ND, R>(a.fgeo + (static_cast<int64_t>(f) * Geo<ND, G>::KF + k) * a.ncell + icl);
 }
 
 // What calc_soln hands to calc_dsoln of the same cell when the neighbour
@@ -150,10 +82,10 @@ __device__ __forceinline__ R fg(MarchArgs<R, G> const & a, int f, int k, int64_t
 // geometry (R_f and Q_f with FP64 geometry); delta is zero for simplices.
 // Whether the fused substep of cell type CT carries calc_soln's neighbour
 // terms to calc_dsoln (FP32 simplices) instead of gathering again.
-template <typename R, int CT>
+template <int CT>
 __host__ __device__ constexpr bool carries()
 {
-    return sizeof(R) == 4 && CellT<CT>::SIMPLEX;
+    return CellT<CT>::SIMPLEX;
 }
 
 // Resident blocks of `block` threads to ask of the compiler for a fused
@@ -186,7 +118,7 @@ __host__ __device__ constexpr bool carries()
 template <int ND, typename R, int CT, int BLOCK, typename G = R>
 __host__ __device__ constexpr int min_blocks()
 {
-    if constexpr (!carries<R, CT>())
+    if constexpr (sizeof(R) == 8 || !carries<CT>())
     {
         return 0;
     }
@@ -280,14 +212,11 @@ __device__ __forceinline__ void face_means(MarchArgs<R, G> const & a, int64_t ic
 // calc_soln for one body cell (euler_march.cpp:197-303): the CESE flux
 // integral over the cell's BCEs, divided by the CCE volume.
 //
-// With CACHE set (the fused march, where every record's primitive cache is
-// valid) a neighbour's primitives come from its record.  With u0 (the cell's
-// own current state; the FP32 march) the neighbour values enter as
-// differences from u0 and d0 receives so0n - u0: in FP32 the absolute
+// FP32.  With u0 (the cell's own current state; the march) the neighbour
+// values enter as differences from u0 and d0 receives so0n - u0: the absolute
 // rounding then scales with the change, not with the state (the gradients
 // calc_dsoln forms from these differences are O(h) of the state).
-template <int CT, typename R, typename G, bool CACHE = false,
-          typename CA = Carry<CellT<CT>::ND, CellT<CT>::NFC, R>>
+template <int CT, typename R, typename G, typename CA = Carry<CellT<CT>::ND, CellT<CT>::NFC, R>>
 __device__ __forceinline__ void soln_cell(MarchArgs<R, G> const & a, int64_t icl, R * so0n, CA * carry = nullptr,
                                           R const * u0 = nullptr, R * d0 = nullptr)
 {
@@ -296,14 +225,13 @@ __device__ __forceinline__ void soln_cell(MarchArgs<R, G> const & a, int64_t icl
     constexpr int NFC = CellT<CT>::NFC;
     using D = Geo<ND, G>;
     using RC = Rec<ND, R>;
-    constexpr bool USE = CACHE && RC::PRIM;
-    Acc<R> acc[NEQ];
+    Acc acc[NEQ];
 #pragma unroll
     for (int f = 0; f < NFC; ++f)
     {
         int64_t const jr = ldg(a.nbr + f * a.ncell + icl);
-        R rec[USE ? RC::NLOAD : RC::NUSED];
-        load_rec<ND, R, USE ? RC::NLOAD : RC::NUSED>(a.cur + jr * RC::RS, rec);
+        R rec[RC::NUSED];
+        load_rec<ND>(a.cur + jr * RC::RS, rec);
         R const * u = rec;
         R const * t = rec + NEQ;
         R const * g = rec + 2 * NEQ;
@@ -379,15 +307,7 @@ __device__ __forceinline__ void soln_cell(MarchArgs<R, G> const & a, int64_t icl
                 w[i * ND + d] = s;
             }
         }
-        Prim<ND, R> q;
-        if constexpr (USE)
-        {
-            q = Prim<ND, R>::cached(rec + RC::OP, ga);
-        }
-        else
-        {
-            q = Prim<ND, R>(u, ga);
-        }
+        Prim<ND, R> const q(u, ga);
         R fl[NEQ];
         flux_dot<ND, R>(q, u, nh, fl);
         jvp_sum<ND, R>(q, u, w, fl);
@@ -415,11 +335,10 @@ __device__ __forceinline__ void soln_cell(MarchArgs<R, G> const & a, int64_t icl
     }
 }
 
-// calc_cfl for one body cell (euler_solution.cpp:106-160): original and
+// calc_cfl for one body cell in FP32 (euler_solution.cpp:106-160): original and
 // clamped CFL, and the energy rewritten from the non-negative pressure.  The
 // reference's three divisions by rho use one reciprocal 1/(rho + TINY) (the
-// floor changes nothing unless rho is below 1e-44 in FP64, 1e-23 in FP32,
-// where the reference itself produces inf); it is returned in rinv for the
+// floor changes nothing unless rho is below 1e-23); it is returned in rinv for the
 // primitives of the same state.
 template <int ND, typename R, typename G>
 __device__ __forceinline__ R cfl_cell(MarchArgs<R, G> const & a, int64_t icl, int64_t row, R * so0n, R & rinv)
@@ -474,7 +393,7 @@ __device__ __forceinline__ void dsoln_cell(MarchArgs<R, G> const & a, int64_t ic
     using D = Geo<ND, G>;
 
     R const acfl = fabs(cflc);
-    R const sgm0 = sizeof(R) == 8 ? R(0) : mquot<ND>(a.sigma0, acfl); // FP32 cap only
+    R const sgm0 = mquot<ND>(a.sigma0, acfl);
     R const tau = a.taumin + acfl * a.tauscale;
     R const ofg1 = R(1) / R(NFGE);
 
@@ -584,7 +503,7 @@ __device__ __forceinline__ void dsoln_cell(MarchArgs<R, G> const & a, int64_t ic
         {
             int64_t const jr = ldg(a.nbr + f * a.ncell + icl);
             R rec[Rec<ND, R>::NUSED];
-            load_rec<ND, R>(a.cur + jr * Rec<ND, R>::RS, rec);
+            load_rec<ND>(a.cur + jr * Rec<ND, R>::RS, rec);
             R jd[ND];
 #pragma unroll
             for (int d = 0; d < ND; ++d)
@@ -614,10 +533,8 @@ __device__ __forceinline__ void dsoln_cell(MarchArgs<R, G> const & a, int64_t ic
     }
 
     // Rows of each element's inverse displacement matrix (prescaled by
-    // 1/det): grad = sum_v uf[v] * C[k][v].  In FP64 the NFGE reciprocals
-    // come from one division by the product of the determinants (prefix
-    // products, then peeled off backwards); in FP32 that product could
-    // underflow, so each element divides.
+    // 1/det): grad = sum_v uf[v] * C[k][v].  Each element divides by its own
+    // determinant (a product of all of them could underflow in FP32).
     R dets[NFGE];
     R bcx[NFGE][ND == 3 ? 3 : 1]; // 3D: rb x rc, the first row of the adjugate
 #pragma unroll
@@ -639,31 +556,10 @@ __device__ __forceinline__ void dsoln_cell(MarchArgs<R, G> const & a, int64_t ic
         }
     }
     R invs[NFGE];
-    if constexpr (sizeof(R) == 8)
+#pragma unroll
+    for (int k = 0; k < NFGE; ++k)
     {
-        R pre[NFGE];
-        pre[0] = dets[0];
-#pragma unroll
-        for (int k = 1; k < NFGE; ++k)
-        {
-            pre[k] = pre[k - 1] * dets[k];
-        }
-        R inv = recip(pre[NFGE - 1]);
-#pragma unroll
-        for (int k = NFGE - 1; k > 0; --k)
-        {
-            invs[k] = inv * pre[k - 1];
-            inv *= dets[k];
-        }
-        invs[0] = inv;
-    }
-    else
-    {
-#pragma unroll
-        for (int k = 0; k < NFGE; ++k)
-        {
-            invs[k] = mrecip<ND>(dets[k]);
-        }
+        invs[k] = mrecip<ND>(dets[k]);
     }
     R C[NFGE][ND][ND];
 #pragma unroll
@@ -721,54 +617,6 @@ __device__ __forceinline__ void dsoln_cell(MarchArgs<R, G> const & a, int64_t ic
             wgt[k] = rsq(sq + Tiny<R>::AZ);
             wacc += wgt[k];
         }
-        if constexpr (sizeof(R) == 8)
-        {
-            // FP64: one division per equation.  With u = w - wacc/n (the
-            // deviations scaled by wacc > 0) the reference's weight
-            // 1/n + sm (w/wacc - 1/n) is 1/n + (sm/wacc) u, and each of its
-            // three caps divided by wacc is a quotient of known sign:
-            //   T1 = (1 - 1/n) / (umax + TINY wacc),  T2 = (1/n) / (TINY wacc - umin),
-            //   T0 = sigma0 / (|cfl| wacc).
-            // The smaller of T1, T2 is chosen by cross-multiplying as in
-            // FP32 below; it fires (the W-3/4 cap binds) when it is below
-            // T0, again by cross-multiplying, and only the chosen quotient
-            // is divided out.
-            R const wq = ofg1 * wacc;
-            R umax = R(0);
-            R umin = R(0);
-#pragma unroll
-            for (int k = 0; k < NFGE; ++k)
-            {
-                wgt[k] -= wq;
-                umax = fmax(umax, wgt[k]);
-                umin = fmin(umin, wgt[k]);
-            }
-            R const za = Tiny<R>::AZ * wacc;
-            R const d1 = umax + za;
-            R const d2 = za - umin;
-            bool const first = (R(1) - ofg1) * d2 <= ofg1 * d1;
-            R const nn = first ? R(1) - ofg1 : ofg1;
-            R const dd = first ? d1 : d2;
-            R const cw = acfl * wacc;
-            bool const fire = nn * cw < a.sigma0 * dd;
-            R const c = (fire ? nn : a.sigma0) * recip(fire ? dd : cw);
-            if (fire)
-            {
-                fired |= static_cast<uint8_t>(1u << i);
-            }
-#pragma unroll
-            for (int d = 0; d < ND; ++d)
-            {
-                R s = R(0);
-#pragma unroll
-                for (int k = 0; k < NFGE; ++k)
-                {
-                    s += (ofg1 + c * wgt[k]) * grad[k][d];
-                }
-                so1n[i * ND + d] = s;
-            }
-        }
-        else
         {
             R const rw = mrecip<ND>(wacc);
             R wmax = R(0);
@@ -1010,7 +858,7 @@ __device__ __forceinline__ void fused_cell(MarchArgs<R, G> const & a, int64_t ic
     // The choice depends on the cell type and precision only, never on the
     // kernel, so a core's cells give the same bits in every kernel that
     // marches them (single-type or mixed, alone or batched).
-    constexpr bool CARRY = carries<R, CT>();
+    constexpr bool CARRY = carries<CT>();
     // SB > 0: the carried sums in shared memory, SB threads per block.
     using CA = std::conditional_t<(SB > 0 && CARRY), CarrySh<ND, NFC, R, SB>, Carry<ND, NFC, R>>;
     CA carry;
@@ -1024,15 +872,11 @@ __device__ __forceinline__ void fused_cell(MarchArgs<R, G> const & a, int64_t ic
     {
         face_means<CT, R, G>(a, icl, carry.mm, carry.mb);
     }
-    // FP32: work relative to the cell's own current state (delta form).
-    constexpr bool DELTA = sizeof(R) == 4;
+    // Work relative to the cell's own current state (delta form).
     R u0[NEQ], d0[NEQ];
-    if constexpr (DELTA)
-    {
-        load_rec<ND, R, NEQ>(a.cur + row * Rec<ND, R>::RS, u0);
-    }
+    load_rec<ND, NEQ>(a.cur + row * Rec<ND, R>::RS, u0);
     R so0n[NEQ];
-    soln_cell<CT, R, G, true>(a, icl, so0n, CARRY ? &carry : nullptr, DELTA ? u0 : nullptr, d0);
+    soln_cell<CT, R, G>(a, icl, so0n, CARRY ? &carry : nullptr, u0, d0);
     // FP32 error feedback: what rounding the new so0 to FP32 drops is kept per
     // cell and equation (comp) and added back to the cell's next new value,
     // the rounding taken by an exact two-sum (Knuth) so the kept residual is
@@ -1047,20 +891,17 @@ __device__ __forceinline__ void fused_cell(MarchArgs<R, G> const & a, int64_t ic
     // the rounded so0; the API's so0n and the totals are so0 + comp; d0 becomes
     // the change including the residual.
     R cnew[NEQ];
-    if constexpr (DELTA)
+    if (a.comp)
     {
-        if (a.comp)
-        {
 #pragma unroll
-            for (int i = 0; i < NEQ; ++i)
-            {
-                R const y = d0[i] + a.comp[i * a.ncell + icl];
-                R const t = u0[i] + y;
-                R const yb = t - u0[i];
-                cnew[i] = (u0[i] - (t - yb)) + (y - yb);
-                so0n[i] = t;
-                d0[i] = y;
-            }
+        for (int i = 0; i < NEQ; ++i)
+        {
+            R const y = d0[i] + a.comp[i * a.ncell + icl];
+            R const t = u0[i] + y;
+            R const yb = t - u0[i];
+            cnew[i] = (u0[i] - (t - yb)) + (y - yb);
+            so0n[i] = t;
+            d0[i] = y;
         }
     }
 
@@ -1075,14 +916,13 @@ __device__ __forceinline__ void fused_cell(MarchArgs<R, G> const & a, int64_t ic
             if (kind >= 0)
             {
                 R own[Rec<ND, R>::NUSED];
-                load_rec<ND, R>(a.cur + row * Rec<ND, R>::RS, own);
+                load_rec<ND>(a.cur + row * Rec<ND, R>::RS, own);
                 R g0[NEQ], g1[NEQ * ND], gt[NEQ];
                 bc0_ghost<ND, R>(kind, a.gnml + jr * ND, a.gval + jr * NEQ, so0n, g0);
                 bc1_ghost<ND, R>(kind, a.gnml + jr * ND, own + 2 * NEQ, g1);
                 Prim<ND, R> const qg(g0, ldg(a.gamma + jr));
                 solt_prim<ND, R>(qg, g0, g1, gt);
-                store_rec<ND, R>(a.nxt + jr * Rec<ND, R>::RS, g0, gt, g1, qg);
-                deliver_row<ND>(a, jr, g0, g1);
+                store_rec<ND>(a.nxt + jr * Rec<ND, R>::RS, g0, gt, g1);
             }
         }
     }
@@ -1090,43 +930,94 @@ __device__ __forceinline__ void fused_cell(MarchArgs<R, G> const & a, int64_t ic
     R rinv;
     R const e_soln = so0n[NEQ - 1];
     R const cflc = cfl_cell<ND, R, G>(a, icl, row, so0n, rinv);
-    if (DELTA && so0n[NEQ - 1] != e_soln)
+    if (so0n[NEQ - 1] != e_soln)
     {
         d0[NEQ - 1] = so0n[NEQ - 1] - u0[NEQ - 1]; // calc_cfl rewrote the energy
         cnew[NEQ - 1] = R(0);                      // ... and nothing was dropped
     }
-    if constexpr (DELTA)
+    if (a.comp)
     {
-        if (a.comp)
-        {
 #pragma unroll
-            for (int i = 0; i < NEQ; ++i)
-            {
-                a.comp[i * a.ncell + icl] = cnew[i];
-            }
+        for (int i = 0; i < NEQ; ++i)
+        {
+            a.comp[i * a.ncell + icl] = cnew[i];
         }
     }
     if constexpr (CARRY)
     {
-        // Take the cell's own change (FP32, delta form) or new state out of
-        // the carried sums now, so it need not stay live through calc_dsoln.
+        // Take the cell's own change (delta form) out of the carried sums
+        // now, so it need not stay live through calc_dsoln.
 #pragma unroll
         for (int f = 0; f < NFC; ++f)
         {
 #pragma unroll
             for (int i = 0; i < NEQ; ++i)
             {
-                carry.p[f][i] -= DELTA ? d0[i] : so0n[i];
+                carry.p[f][i] -= d0[i];
             }
         }
     }
     R so1n[NEQ * ND];
-    dsoln_cell<CT, R, G>(a, icl, so0n, cflc, so1n, CARRY ? &carry : nullptr, DELTA ? u0 : nullptr, d0);
+    dsoln_cell<CT, R, G>(a, icl, so0n, cflc, so1n, CARRY ? &carry : nullptr, u0, d0);
     R so0t[NEQ];
     Prim<ND, R> const q(so0n, ldg(a.gamma + row), rinv);
     solt_prim<ND, R>(q, so0n, so1n, so0t);
-    store_rec<ND, R>(a.nxt + row * Rec<ND, R>::RS, so0n, so0t, so1n, q);
+    store_rec<ND>(a.nxt + row * Rec<ND, R>::RS, so0n, so0t, so1n);
+}
+
+// The same in FP64 (euler_fp64.cuh).
+template <int CT>
+__device__ __forceinline__ void fused_cell64(MarchArgs<double, double> const & a, int64_t icl)
+{
+    constexpr int ND = CellT<CT>::ND;
+    constexpr int NEQ = ND + 2;
+    constexpr int NFC = CellT<CT>::NFC;
+    using RC = Rec<ND, double>;
+    using F = FluxTerms<ND>;
+    int64_t const row = icl + a.ngst;
+    double so0n[NEQ];
+    soln64<CT, true>(a, icl, so0n);
+#pragma unroll 1
+    for (int f = 0; f < NFC; ++f)
+    {
+        int64_t const jr = ldg(a.nbr + f * a.ncell + icl);
+        if (jr < a.ngst)
+        {
+            int const kind = a.gkind[jr];
+            if (kind >= 0)
+            {
+                double own[RC::NUSED + 1], g0[NEQ], g1[NEQ * ND], gt[NEQ], gc[F::N];
+                load_part<2 * NEQ, RC::NUSED>(a.cur + row * RC::RS, own);
+                bc0_ghost<ND, double>(kind, a.gnml + jr * ND, a.gval + jr * NEQ, so0n, g0);
+                bc1_ghost<ND, double>(kind, a.gnml + jr * ND, own + 2 * NEQ, g1);
+                solt_terms<ND>(g0, g1, ldg(a.gamma + jr), a.qdt, gt, gc);
+                store_row<ND>(a.nxt + jr * RC::RS, g0, gt, g1, gc);
+                deliver_row<ND>(a, jr, g0, g1);
+            }
+        }
+    }
+    double rinv;
+    double const cflc = cfl64<ND>(a, icl, row, so0n, rinv);
+    double so1n[NEQ * ND];
+    dsoln64<CT>(a, icl, so0n, cflc, so1n);
+    double so0t[NEQ], c[F::N];
+    solt_terms<ND>(so0n, so1n, ldg(a.gamma + row), rinv, a.qdt, so0t, c);
+    store_row<ND>(a.nxt + row * RC::RS, so0n, so0t, so1n, c);
     deliver_row<ND>(a, row, so0n, so1n);
+}
+
+// A cell's fused substep in either precision.
+template <int CT, typename R, typename G, int SB = 0>
+__device__ __forceinline__ void substep_cell(MarchArgs<R, G> const & a, int64_t icl)
+{
+    if constexpr (sizeof(R) == 8)
+    {
+        fused_cell64<CT>(a, icl);
+    }
+    else
+    {
+        fused_cell<CT, R, G, SB>(a, icl);
+    }
 }
 
 // The work of thread t of one substep: body cell t for t < ncell, ghost row
@@ -1142,23 +1033,23 @@ __device__ __forceinline__ void fused_thread(MarchArgs<R, G> const & a, int64_t 
         if constexpr (CT1 != 0)
         {
             (void)ct;
-            fused_cell<CT1, R, G, SB>(a, t);
+            substep_cell<CT1, R, G, SB>(a, t);
         }
         else if constexpr (ND == 2)
         {
             if (ct == 4)
-                fused_cell<4, R, G>(a, t);
+                substep_cell<4, R, G>(a, t);
             else
-                fused_cell<3, R, G>(a, t);
+                substep_cell<3, R, G>(a, t);
         }
         else
         {
             switch (ct)
             {
-            case 6: fused_cell<6, R, G>(a, t); break;
-            case 5: fused_cell<5, R, G>(a, t); break;
-            case 7: fused_cell<7, R, G>(a, t); break;
-            default: fused_cell<8, R, G>(a, t); break;
+            case 6: substep_cell<6, R, G>(a, t); break;
+            case 5: substep_cell<5, R, G>(a, t); break;
+            case 7: substep_cell<7, R, G>(a, t); break;
+            default: substep_cell<8, R, G>(a, t); break;
             }
         }
     }
@@ -1170,13 +1061,26 @@ __device__ __forceinline__ void fused_thread(MarchArgs<R, G> const & a, int64_t 
         if (a.gkind[g] < 0)
         {
             constexpr int NEQ = ND + 2;
-            R rec[Rec<ND, R>::NUSED];
-            load_rec<ND, R>(a.nxt + g * Rec<ND, R>::RS, rec);
-            R tt[NEQ];
-            Prim<ND, R> const q(rec, ldg(a.gamma + g));
-            solt_prim<ND, R>(q, rec, rec + 2 * NEQ, tt);
-            store_rec<ND, R>(a.nxt + g * Rec<ND, R>::RS, rec, tt, rec + 2 * NEQ, q);
-            deliver_row<ND>(a, g, rec, rec + 2 * NEQ);
+            R * const base = a.nxt + g * Rec<ND, R>::RS;
+            R rec[Rec<ND, R>::NUSED], tt[NEQ];
+#pragma unroll
+            for (int i = 0; i < Rec<ND, R>::NUSED; ++i)
+            {
+                rec[i] = base[i];
+            }
+            if constexpr (sizeof(R) == 8)
+            {
+                double c[FluxTerms<ND>::N];
+                solt_terms<ND>(rec, rec + 2 * NEQ, ldg(a.gamma + g), a.qdt, tt, c);
+                store_row<ND>(base, rec, tt, rec + 2 * NEQ, c);
+                deliver_row<ND>(a, g, rec, rec + 2 * NEQ);
+            }
+            else
+            {
+                Prim<ND, R> const q(rec, ldg(a.gamma + g));
+                solt_prim<ND, R>(q, rec, rec + 2 * NEQ, tt);
+                store_rec<ND>(base, rec, tt, rec + 2 * NEQ);
+            }
         }
     }
 }

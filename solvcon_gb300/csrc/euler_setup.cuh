@@ -332,7 +332,9 @@ __global__ void k_compact(MeshView m, double const * cevol, double const * cecnd
         }
         for (int d = 0; d < ND; ++d)
         {
-            put(f, D::K_DB + d, bc[d] - jce[d]);
+            double const db = bc[d] - jce[d];
+            // The FP64 march uses dB only times the element's volume.
+            put(f, D::K_DB + d, std::is_same<G, double>::value ? cevol[row * 7 + ifl] * db : db);
             put(f, D::K_NH + d, hdt * nsum[d]);
             for (int e = 0; e < ND; ++e)
             {

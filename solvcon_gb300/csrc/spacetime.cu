@@ -540,6 +540,17 @@ __global__ void k_divide_check(double const * x, double const * d, double * q, d
     }
 }
 
+// The FP64 march's reciprocal root and root of x.
+__global__ void k_root_check(double const * x, double * r, double * s, int64_t n)
+{
+    int64_t const i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i < n)
+    {
+        r[i] = scg::dev::rsq(x[i]);
+        s[i] = scg::dev::sqr_t(x[i]);
+    }
+}
+
 } // namespace
 
 struct scg_st
@@ -631,6 +642,27 @@ int scg_divide_check(const double * x, const double * d, double * q, double * qd
         scg::cuda_check(cudaMemcpy(q, dq.ptr, dq.bytes(), cudaMemcpyDeviceToHost), "D2H");
         scg::cuda_check(cudaMemcpy(qdiv, dqd.ptr, dqd.bytes(), cudaMemcpyDeviceToHost), "D2H");
         scg::cuda_check(cudaMemcpy(rcp, dr.ptr, dr.bytes(), cudaMemcpyDeviceToHost), "D2H");
+    });
+}
+
+int scg_root_check(const double * x, double * r, double * s, int64_t n)
+{
+    return scg::guarded([&] {
+        if (n < 0 || (n > 0 && (!x || !r || !s)))
+        {
+            throw std::invalid_argument("scg_root_check: null buffer or negative count");
+        }
+        if (n == 0)
+        {
+            return;
+        }
+        size_t const sz = static_cast<size_t>(n);
+        scg::DevBuf<double> dx(sz), dr(sz), ds(sz);
+        scg::cuda_check(cudaMemcpy(dx.ptr, x, dx.bytes(), cudaMemcpyHostToDevice), "H2D");
+        k_root_check<<<static_cast<unsigned>((n + 255) / 256), 256>>>(dx.ptr, dr.ptr, ds.ptr, n);
+        scg::launched(nullptr, "root_check");
+        scg::cuda_check(cudaMemcpy(r, dr.ptr, dr.bytes(), cudaMemcpyDeviceToHost), "D2H");
+        scg::cuda_check(cudaMemcpy(s, ds.ptr, ds.bytes(), cudaMemcpyDeviceToHost), "D2H");
     });
 }
 
