@@ -6,14 +6,13 @@
  * A half step updates the points of one parity from the solution elements
  * ("kernels") at the points of the other parity.  The reference sweeps the
  * points serially with a two-kernel sliding window so that each kernel is
- * derived once; here each thread derives the kernel at one point and shares
- * the quantities its left neighbour needs (flux_lr, up, x - xneg) through
- * shared memory, so each kernel is still derived once per half step.  The
- * first half step also performs the copy-out boundary treatment (it touches
- * only points the half step neither reads nor writes), and update_cfl (which
- * reads only the kernel points) is folded into the same kernel, so a full
- * march_alpha step is two launches.  The fine-grained methods run as separate
- * kernels built from the same device routines.  The FP32 core (Euler1D32,
+ * derived once; here each lane derives the kernel at one point and shares
+ * the quantities its left neighbour needs (flux_lr, up, x - xneg) by warp
+ * shuffles.  The first half step also performs the copy-out boundary treatment
+ * (it touches only points the half step neither reads nor writes), and
+ * update_cfl (which reads only the kernel points) is folded into the same
+ * kernel, so a full march_alpha step is two launches.  The fine-grained methods
+ * run the same kernel with less asked of it.  The FP32 core (Euler1D32,
  * not in the reference) keeps its state split by parity in a layout of its
  * own and updates four outputs per thread; see the comment above it.
  */
@@ -22,6 +21,7 @@
 #include "common.hpp"
 #include "divide.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <memory>
@@ -30,8 +30,6 @@
 
 namespace
 {
-
-constexpr int B1D = 256;
 
 // Euler1DKernel::tiny (Euler1DCore.hpp:182) in FP64; it underflows in FP32,
 // where the same expressions use the smallest floor that keeps them finite.
@@ -48,34 +46,28 @@ struct Tiny1D<float>
     static constexpr float V = 1.e-30f;
 };
 
-// The FP64 core's device state: the reference's [n][3] tables.
-template <typename R>
+// The FP64 core's device state: the reference's [n][3] tables, and what depends
+// on the grid (and the time increment) alone, formed once per coordinate write.
 struct E1DArgs
 {
-    double const * coord;
-    R const * gamma;
-    R * so0; // [n][3]
-    R * so1; // [n][3]
-    R * cfl;
+    double const * gamma;
+    double * so0; // [n][3]
+    double * so1; // [n][3]
+    double * cfl;
     int64_t n;
     double hdt, qdt;
-    // 1 / (x[i + 1] - x[i]) and 1 / (x[i + 2] - x[i]): the divisions of a
-    // half step that depend on the grid alone, formed once per coordinate
-    // write by the same expressions (so the same bits) instead of every
-    // half step.
-    double const * invdx;
-    double const * invd2;
-    // The solution element's offsets from the grid alone, [5][n]: x - xctr,
-    // xpos - x, (x + xpos) / 2 - xctr, x - xneg, (x + xneg) / 2 - xctr with
-    // xctr = (xpos + xneg) / 2 (Euler1DCore.hpp:210-244), formed once per
-    // coordinate write.
+    double const * invdx; // 1 / (x[i + 1] - x[i])
+    double const * invd2; // 1 / (x[i + 2] - x[i])
+    double const * cflr;  // dt / 2 / min(x[i] - x[i - 1], x[i + 1] - x[i])
+    // The solution element's offsets, [5][n]: x - xctr, xpos - x,
+    // (x + xpos) / 2 - xctr, x - xneg, (x + xneg) / 2 - xctr with
+    // xctr = (xpos + xneg) / 2 (Euler1DCore.hpp:210-244).
     double const * seo;
 };
 
-// The grid's tables of E1DArgs.  The offsets round every operation on its
-// own (no contraction), so their bits do not depend on the kernel that
-// forms them.
-__global__ void k_inv_spacing(double const * coord, int64_t n, double * invdx, double * invd2, double * seo)
+// The grid's tables of E1DArgs.
+__global__ void k_inv_spacing(double const * coord, int64_t n, double hdt, double * invdx, double * invd2,
+                              double * cflr, double * seo)
 {
     int64_t const i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i < n)
@@ -83,6 +75,7 @@ __global__ void k_inv_spacing(double const * coord, int64_t n, double * invdx, d
         invdx[i] = i + 1 < n ? 1.0 / (coord[i + 1] - coord[i]) : 0.0;
         invd2[i] = i + 2 < n ? 1.0 / (coord[i + 2] - coord[i]) : 0.0;
         double o[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+        double q = 0.0;
         if (i > 0 && i + 1 < n)
         {
             double const x = coord[i];
@@ -94,7 +87,9 @@ __global__ void k_inv_spacing(double const * coord, int64_t n, double * invdx, d
             o[2] = __dsub_rn(__dmul_rn(0.5, __dadd_rn(x, xpos)), xctr);
             o[3] = __dsub_rn(x, xneg);
             o[4] = __dsub_rn(__dmul_rn(0.5, __dadd_rn(x, xneg)), xctr);
+            q = hdt / (o[1] < o[3] ? o[1] : o[3]);
         }
+        cflr[i] = q;
         for (int k = 0; k < 5; ++k)
         {
             seo[k * n + i] = o[k];
@@ -102,242 +97,227 @@ __global__ void k_inv_spacing(double const * coord, int64_t n, double * invdx, d
     }
 }
 
-// The solution-element kernel at point ic (Euler1DKernel::set_value and
-// derive, Euler1DCore.hpp:193-244): flux f, temporal derivatives ut, ft and
-// the value up at the point, plus the two half fluxes of calc_flux_ll/lr
-// (Euler1DCore.hpp:246-266).  Reciprocals of rho are formed once: for any
-// density above ~1e-50 the reference's denominators rho^k + tiny equal rho^k.
-// Its divisions (this one, update_cfl's and the W-alpha weights') multiply
-// by scg::dev::recip, a Newton reciprocal within one ulp that takes about
-// half the FP64 instructions of a division.
-template <typename R>
-struct K1D
+// The FP64 half step is bound by the FP64 pipe (one instruction per SM every 16
+// cycles), so its routines take the fewest FP64 instructions: the Jacobian
+// products are directional derivatives of the flux from the primitive
+// variables, the divisions and the root are integer arithmetic (divide.cuh),
+// and what the grid fixes is read from tables: 98 FP64 instructions per output
+// point (196 with the Jacobian formed, FP64 Newton reciprocals and a library
+// root).  Every operation is written as the instruction it is, so the
+// fine-grained methods and the fused march round alike, as the reference
+// requires.
+__device__ __forceinline__ double fm(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ double mu(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ double ad(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ double sb(double a, double b) { return __dsub_rn(a, b); }
+
+// The primitive variables of one point, r = 1 / (rho + tiny); for any density
+// above ~1e-50 the reference's denominators rho^k + tiny equal rho^k.
+struct P1D
 {
-    R r; // 1 / (rho + tiny), shared with update_cfl at the same point
-    R up[3];
-    R ll[3]; // flux through the lower-left of the CE to the right
-    R lr[3]; // flux through the lower-right of the CE to the left
+    double u[3], r, v, p, ga;
+
+    __device__ __forceinline__ P1D(E1DArgs const & a, int64_t ic)
+    {
+        for (int i = 0; i < 3; ++i)
+        {
+            u[i] = a.so0[ic * 3 + i];
+        }
+        ga = a.gamma[ic];
+        r = scg::dev::recip(ad(u[0], Tiny1D<double>::V));
+        v = mu(u[1], r);
+        p = mu(sb(ga, 1.0), fm(-0.5, mu(u[1], v), u[2]));
+    }
+
+    // update_cfl at the point (Euler1DCore.cpp:70-94), times the table's
+    // dt / 2 / dx.  The reference's sqrt(m * m) / rho is |v|.
+    __device__ __forceinline__ double cfl(double cflr) const
+    {
+        // (p + |p|) / 2: zero for a negative p, NaN for -infinity and NaN.
+        unsigned const hp = static_cast<unsigned>(__double2hiint(p));
+        double const pr =
+            hp >= 0x80000000u ? (hp >= 0xfff00000u ? __longlong_as_double(0x7ff8000000000000ll) : 0.0) : p;
+        return mu(ad(scg::dev::sqr_t(mu(mu(ga, pr), r)), fabs(v)), cflr);
+    }
 };
 
-template <typename R>
-__device__ __forceinline__ void derive(E1DArgs<R> const & a, int64_t ic, K1D<R> & k)
+// The solution-element kernel at point ic (Euler1DKernel::set_value and
+// derive, Euler1DCore.hpp:193-244): the value up at the next half level and the
+// two half fluxes of calc_flux_ll/lr (Euler1DCore.hpp:246-266).
+struct K1D
 {
-    R const ga = a.gamma[ic];
-    R u[3], ux[3];
-    for (int i = 0; i < 3; ++i)
-    {
-        u[i] = a.so0[ic * 3 + i];
-        ux[i] = a.so1[ic * 3 + i];
-    }
-    R const r = scg::dev::recip(u[0] + Tiny1D<R>::V);
-    k.r = r;
-    R const r2 = r * r;
-    R const m2r2 = u[1] * u[1] * r2; // u1^2 / u0^2
-    R jac[3][3];
-    jac[0][0] = R(0);
-    jac[0][1] = R(1);
-    jac[0][2] = R(0);
-    jac[1][0] = (ga - R(3)) / R(2) * m2r2;
-    jac[1][1] = -(ga - R(3)) * u[1] * r;
-    jac[1][2] = ga - R(1);
-    jac[2][0] = (ga - R(1)) * m2r2 * u[1] * r - ga * u[1] * u[2] * r2;
-    jac[2][1] = ga * u[2] * r - R(1.5) * (ga - R(1)) * m2r2;
-    jac[2][2] = ga * u[1] * r;
-    R f[3], ut[3], ft[3];
-    f[0] = u[1];
-    f[1] = (ga - R(1)) * u[2] + (R(3) - ga) / R(2) * u[1] * u[1] * r;
-    f[2] = ga * u[1] * u[2] * r - (ga - R(1)) / R(2) * u[1] * m2r2;
-    for (int i = 0; i < 3; ++i)
-    {
-        ut[i] = -jac[i][0] * ux[0] - jac[i][1] * ux[1] - jac[i][2] * ux[2];
-    }
-    for (int i = 0; i < 3; ++i)
-    {
-        ft[i] = jac[i][0] * ut[0] + jac[i][1] * ut[1] + jac[i][2] * ut[2];
-    }
-    R const hdt = R(a.hdt), qdt = R(a.qdt);
-    R const dxctr = R(a.seo[0 * a.n + ic]);
-    R const dxl = R(a.seo[1 * a.n + ic]);
-    R const dml = R(a.seo[2 * a.n + ic]);
-    R const dxr = R(a.seo[3 * a.n + ic]);
-    R const dmr = R(a.seo[4 * a.n + ic]);
-    for (int i = 0; i < 3; ++i)
-    {
-        k.up[i] = u[i] + dxctr * ux[i] + hdt * ut[i];
-    }
-    for (int i = 0; i < 3; ++i)
-    {
-        R const tf = f[i] - dxctr * ut[i] + qdt * ft[i];
-        k.ll[i] = dxl * (u[i] + dml * ux[i]) + hdt * tf;
-        k.lr[i] = dxr * (u[i] + dmr * ux[i]) - hdt * tf;
-    }
-}
+    double up[3];
+    double ll[3]; // flux through the lower-left of the CE to the right
+    double lr[3]; // flux through the lower-right of the CE to the left
 
-// update_cfl at one point (Euler1DCore.cpp:70-94).  The reference's three
-// divisions by rho use r = 1 / (rho + tiny), the reciprocal the kernel
-// derivation at the same point forms (equal unless rho < ~1e-84, where the
-// reference itself overflows).
-template <typename R>
-__device__ __forceinline__ R rho_recip(E1DArgs<R> const & a, int64_t it)
+    __device__ __forceinline__ void derive(E1DArgs const & a, int64_t ic, P1D const & q)
+    {
+        double const * const u = q.u;
+        double ux[3], ut[3], ft[3];
+        for (int i = 0; i < 3; ++i)
+        {
+            ux[i] = a.so1[ic * 3 + i];
+        }
+        double const ga1 = sb(q.ga, 1.0);
+        double const hv = mu(mu(0.5, q.v), q.v);
+        double const h = ad(u[2], q.p);
+        // The flux's change along a change w of the state.
+        auto along = [&](double const * w, double * o) {
+            double const dp = mu(ga1, fm(-q.v, w[1], fm(hv, w[0], w[2])));
+            double const dv = mu(fm(-q.v, w[0], w[1]), q.r);
+            o[0] = w[1];
+            o[1] = fm(u[1], dv, fm(w[1], q.v, dp));
+            o[2] = fm(h, dv, mu(ad(w[2], dp), q.v));
+        };
+        along(ux, ut);
+        for (int i = 0; i < 3; ++i)
+        {
+            ut[i] = -ut[i];
+        }
+        along(ut, ft);
+        double const f[3] = {u[1], fm(u[1], q.v, q.p), mu(h, q.v)};
+        double const dxctr = a.seo[0 * a.n + ic];
+        double const dxl = a.seo[1 * a.n + ic];
+        double const dml = a.seo[2 * a.n + ic];
+        double const dxr = a.seo[3 * a.n + ic];
+        double const dmr = a.seo[4 * a.n + ic];
+        for (int i = 0; i < 3; ++i)
+        {
+            up[i] = fm(a.hdt, ut[i], fm(dxctr, ux[i], u[i]));
+            double const tf = mu(a.hdt, fm(a.qdt, ft[i], fm(-dxctr, ut[i], f[i])));
+            ll[i] = fm(dxl, fm(dml, ux[i], u[i]), tf);
+            lr[i] = fm(dxr, fm(dmr, ux[i], u[i]), -tf);
+        }
+    }
+};
+
+// The W-alpha gradient (march_half_so1_alpha, Euler1DCore.hpp:284-320); for
+// alpha = 2 its numerator duxp^2 duxn + duxn^2 duxp is duxn duxp (duxn + duxp).
+__device__ __forceinline__ double wgrad(int alpha, double duxn, double duxp)
 {
-    return scg::dev::recip(a.so0[it * 3 + 0] + Tiny1D<R>::V);
-}
-
-__device__ __forceinline__ double sqrt_r(double x) { return sqrt(x); }
-
-template <typename R>
-__device__ __forceinline__ void cfl_at(E1DArgs<R> const & a, int64_t it, double hdt, R r)
-{
-    R const ga = a.gamma[it];
-    R const m = a.so0[it * 3 + 1];
-    R const m2 = m * m;
-    R const ke = R(0.5) * m2 * r;
-    R pr = (ga - R(1)) * (a.so0[it * 3 + 2] - ke);
-    pr = (pr + fabs(pr)) / R(2);
-    // The reference's sqrt(m * m) is |m| exactly: in binary IEEE arithmetic
-    // the square root of a correctly rounded square returns the operand's
-    // magnitude (barring overflow or underflow of the square).
-    R const wspd = sqrt_r(ga * pr * r) + fabs(m) * r;
-    double const dxpos = a.coord[it + 1] - a.coord[it];
-    double const dxneg = a.coord[it] - a.coord[it - 1];
-    a.cfl[it] = R(hdt) * wspd * scg::dev::recip(R(dxpos < dxneg ? dxpos : dxneg));
-}
-
-// The W-alpha gradient (march_half_so1_alpha, Euler1DCore.hpp:284-320).
-template <typename R>
-__device__ __forceinline__ R wgrad(int alpha, R duxn, R duxp)
-{
-    R fan = fabs(duxn);
-    R fap = fabs(duxp);
+    double num, den;
     if (alpha == 2)
     {
-        fan *= fan;
-        fap *= fap;
+        num = mu(mu(duxn, duxp), ad(duxn, duxp));
+        den = fm(duxn, duxn, fm(duxp, duxp, Tiny1D<double>::V));
     }
-    return (fap * duxn + fan * duxp) * scg::dev::recip(fap + fan + Tiny1D<R>::V);
+    else
+    {
+        num = fm(fabs(duxp), duxn, mu(fabs(duxn), duxp));
+        den = ad(ad(fabs(duxp), fabs(duxn)), Tiny1D<double>::V);
+    }
+    return mu(num, scg::dev::recip(den));
 }
 
-// What a half step does (k_half's mask): so0, cfl, the copy-out boundary
+// What a half step does (its mask): so0, cfl, the copy-out boundary
 // treatment, and so1 with the W-alpha weights for alpha = (mask >> 8) > 0.
 constexpr unsigned H_SO0 = 1u, H_CFL = 2u, H_BND = 4u;
 constexpr unsigned h_alpha(int alpha) { return static_cast<unsigned>(alpha) << 8; }
 
-// Fused half step: so0, cfl and (alpha > 0) so1 at one parity, with the
-// copy-out boundary treatment (Euler1DCore.cpp:132-172), each as the mask
-// asks.  Output j is point start + 2j + 1 for j < nout; kernels are at
-// start + 2j for j <= nout.  The mask is a launch argument, not a template
-// parameter: the fine-grained operations (march_half_so0, then
-// march_half_so1_alpha on the so0 it stored) and the fused march then run
-// the same compiled code and round alike, which the reference requires of
-// its two marches; compiled apart, the kernels contracted their
-// multiply-adds differently once the divisions became Newton reciprocals.
-template <typename R>
-__global__ void __launch_bounds__(B1D) k_half(E1DArgs<R> a, int64_t start, int64_t nout, unsigned mask)
-{
-    {
-        int const alpha = static_cast<int>(mask >> 8);
-        __shared__ R s_lr[B1D + 1][3];
-        __shared__ R s_up[B1D + 1][3];
-        __shared__ R s_idxr[B1D + 1]; // 1 / (x - xneg) of each kernel
-        int64_t const j0 = static_cast<int64_t>(blockIdx.x) * B1D;
-        int64_t const j = j0 + threadIdx.x;
-        K1D<R> k;
-        bool const have = j <= nout;
-        if (have)
-        {
-            derive(a, start + 2 * j, k);
-            for (int i = 0; i < 3; ++i)
-            {
-                s_lr[threadIdx.x][i] = k.lr[i];
-                s_up[threadIdx.x][i] = k.up[i];
-            }
-            s_idxr[threadIdx.x] = R(a.invdx[start + 2 * j - 1]);
-        }
-        if (threadIdx.x == 0)
-        {
-            int64_t const jh = j0 + B1D; // halo kernel on the right
-            if (jh <= nout)
-            {
-                K1D<R> h;
-                derive(a, start + 2 * jh, h);
-                for (int i = 0; i < 3; ++i)
-                {
-                    s_lr[B1D][i] = h.lr[i];
-                    s_up[B1D][i] = h.up[i];
-                }
-                s_idxr[B1D] = R(a.invdx[start + 2 * jh - 1]);
-            }
-        }
-        __syncthreads();
-        if (have && j < nout)
-        {
-            int64_t const ic = start + 2 * j;
-            R v[3];
-            if (mask & H_SO0)
-            {
-                R const idx = R(a.invd2[ic]);
-                for (int i = 0; i < 3; ++i)
-                {
-                    v[i] = (k.ll[i] + s_lr[threadIdx.x + 1][i]) * idx;
-                    a.so0[(ic + 1) * 3 + i] = v[i];
-                }
-            }
-            else
-            {
-                for (int i = 0; i < 3; ++i)
-                {
-                    v[i] = a.so0[(ic + 1) * 3 + i];
-                }
-            }
-            if (mask & H_CFL)
-            {
-                cfl_at(a, ic, a.hdt, k.r);
-            }
-            if (alpha > 0)
-            {
-                R const idn = R(a.invdx[ic]);
-                R const idp = s_idxr[threadIdx.x + 1];
-                for (int i = 0; i < 3; ++i)
-                {
-                    R const duxn = (v[i] - k.up[i]) * idn;
-                    R const duxp = (s_up[threadIdx.x + 1][i] - v[i]) * idp;
-                    a.so1[(ic + 1) * 3 + i] = wgrad(alpha, duxn, duxp);
-                }
-            }
-        }
-        if ((mask & H_BND) && blockIdx.x == 0 && threadIdx.x == 0)
-        {
-            int64_t const l = 1, r = a.n - 2;
-            for (int i = 0; i < 3; ++i)
-            {
-                a.so0[l * 3 + i] = a.so0[(l + 1) * 3 + i];
-                a.so0[r * 3 + i] = a.so0[(r - 1) * 3 + i];
-                a.so1[l * 3 + i] = a.so1[(l + 1) * 3 + i];
-                a.so1[r * 3 + i] = a.so1[(r - 1) * 3 + i];
-            }
-        }
+// One warp's part of a half step.  Output j is point start + 2j + 1 for
+// j < nout; kernels are at start + 2j for j <= nout.  Lane l of warp w derives
+// kernel 31 w + l, and lanes 0 .. 30 update the output to its right, with the
+// next lane's kernel by shuffles: warps share nothing, so a small tube spreads
+// over the SMs in blocks of one warp, and a kernel is derived once but for the
+// one in 32 at the seams.
+constexpr int WOUT = 31; // outputs per warp
 
+__device__ __forceinline__ void half_warp(E1DArgs const & a, int64_t start, int64_t nout, unsigned mask, int64_t w)
+{
+    int const alpha = static_cast<int>(mask >> 8);
+    int const lane = static_cast<int>(threadIdx.x) & 31;
+    int64_t const j = w * WOUT + lane;
+    int64_t const ic = start + 2 * (j < nout ? j : nout); // lanes past the end repeat the last kernel
+    P1D const q(a, ic);
+    K1D k;
+    k.derive(a, ic, q);
+    double const idxr = a.invdx[ic - 1]; // 1 / (x - xneg)
+    double lr[3], up[3];
+    for (int i = 0; i < 3; ++i)
+    {
+        lr[i] = __shfl_down_sync(0xffffffffu, k.lr[i], 1);
+        up[i] = __shfl_down_sync(0xffffffffu, k.up[i], 1);
+    }
+    double const idp = __shfl_down_sync(0xffffffffu, idxr, 1);
+    if (lane < WOUT && j < nout)
+    {
+        double v[3];
+        if (mask & H_SO0)
+        {
+            double const idx = a.invd2[ic];
+            for (int i = 0; i < 3; ++i)
+            {
+                v[i] = mu(ad(k.ll[i], lr[i]), idx);
+                a.so0[(ic + 1) * 3 + i] = v[i];
+            }
+        }
+        else
+        {
+            for (int i = 0; i < 3; ++i)
+            {
+                v[i] = a.so0[(ic + 1) * 3 + i];
+            }
+        }
+        if (mask & H_CFL)
+        {
+            a.cfl[ic] = q.cfl(a.cflr[ic]);
+        }
+        if (alpha > 0)
+        {
+            double const idn = a.invdx[ic];
+            for (int i = 0; i < 3; ++i)
+            {
+                a.so1[(ic + 1) * 3 + i] = wgrad(alpha, mu(sb(v[i], k.up[i]), idn), mu(sb(up[i], v[i]), idp));
+            }
+        }
+    }
+}
+
+// The copy-out boundary treatment (Euler1DCore.cpp:132-172) of points 1 and
+// n - 2, which the first half step neither reads nor writes.
+__device__ __forceinline__ void copy_out(E1DArgs const & a)
+{
+    int64_t const l = 1, r = a.n - 2;
+    for (int i = 0; i < 3; ++i)
+    {
+        a.so0[l * 3 + i] = a.so0[(l + 1) * 3 + i];
+        a.so0[r * 3 + i] = a.so0[(r - 1) * 3 + i];
+        a.so1[l * 3 + i] = a.so1[(l + 1) * 3 + i];
+        a.so1[r * 3 + i] = a.so1[(r - 1) * 3 + i];
+    }
+}
+
+// One half step: so0, cfl and so1 at one parity and the boundary treatment, as
+// the mask asks.
+__global__ void __launch_bounds__(128) k_half(E1DArgs a, int64_t start, int64_t nout, unsigned mask)
+{
+    int64_t const w = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / 32;
+    if (w * WOUT < nout)
+    {
+        half_warp(a, start, nout, mask, w);
+    }
+    if ((mask & H_BND) && blockIdx.x == 0 && threadIdx.x == 0)
+    {
+        copy_out(a);
     }
 }
 
 // update_cfl alone.
-template <typename R>
-__global__ void k_cfl1d(E1DArgs<R> a, int64_t start, int64_t nout)
+__global__ void k_cfl1d(E1DArgs a, int64_t start, int64_t nout)
 {
     int64_t const j = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (j < nout)
     {
         int64_t const it = start + 2 * j;
-        cfl_at(a, it, a.hdt, rho_recip(a, it));
+        a.cfl[it] = P1D(a, it).cfl(a.cflr[it]);
     }
 }
 
 // treat_boundary_so0 / treat_boundary_so1.
-template <typename R>
-__global__ void k_bnd1d(E1DArgs<R> a, int which)
+__global__ void k_bnd1d(E1DArgs a, int which)
 {
     int64_t const l = 1, r = a.n - 2;
-    R * s = which == 0 ? a.so0 : a.so1;
+    double * s = which == 0 ? a.so0 : a.so1;
     for (int i = 0; i < 3; ++i)
     {
         s[l * 3 + i] = s[(l + 1) * 3 + i];
@@ -362,9 +342,8 @@ struct Euler1DBase
     cudaStream_t stream = nullptr;
 };
 
-// The FP64 core (R = double): the reference's arithmetic on the reference's
-// [n][3] device tables.  The FP32 core is Euler1D32 below.
-template <typename R>
+// The FP64 core: the reference's arithmetic on the reference's [n][3] device
+// tables.  The FP32 core is Euler1D32 below.
 class Euler1D : public Euler1DBase
 {
 public:
@@ -385,6 +364,7 @@ public:
         coord.alloc(static_cast<size_t>(n));
         invdx.alloc(static_cast<size_t>(n));
         invd2.alloc(static_cast<size_t>(n));
+        cflr.alloc(static_cast<size_t>(n));
         seo.alloc(static_cast<size_t>(5 * n));
         for (auto * b : {&cfl, &gamma})
             b->alloc(static_cast<size_t>(n));
@@ -412,7 +392,7 @@ public:
 
     std::unique_ptr<Euler1DBase> clone() override
     {
-        auto c = std::make_unique<Euler1D<R>>(n, time_increment);
+        auto c = std::make_unique<Euler1D>(n, time_increment);
         scg::cuda_check(cudaMemcpyAsync(c->coord.ptr, coord.ptr, sizeof(double) * static_cast<size_t>(n),
                                         cudaMemcpyDeviceToDevice, stream),
                         "copy");
@@ -421,15 +401,15 @@ public:
         for (int k = 1; k < 5; ++k)
         {
             size_t const cnt = static_cast<size_t>(count(k));
-            scg::cuda_check(cudaMemcpyAsync(c->state(k), state(k), cnt * sizeof(R), cudaMemcpyDeviceToDevice, stream),
+            scg::cuda_check(cudaMemcpyAsync(c->state(k), state(k), cnt * sizeof(double), cudaMemcpyDeviceToDevice, stream),
                             "copy");
         }
         sync();
         return c;
     }
 
-    // 0 coord (FP64), 1 cfl, 2 so0, 3 so1, 4 gamma (R)
-    R * state(int which)
+    // 0 coord (FP64), 1 cfl, 2 so0, 3 so1, 4 gamma
+    double * state(int which)
     {
         switch (which)
         {
@@ -471,16 +451,17 @@ public:
     // The grid's tables (E1DArgs) from the coordinates.
     void spacing()
     {
-        k_inv_spacing<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(coord.ptr, n, invdx.ptr, invd2.ptr,
+        k_inv_spacing<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(coord.ptr, n, time_increment / 2.0,
+                                                                                   invdx.ptr, invd2.ptr, cflr.ptr,
                                                                                    seo.ptr);
         scg::launched(stream, "e1d_inv_spacing");
         sync();
     }
 
-    E1DArgs<R> args()
+    E1DArgs args()
     {
-        return E1DArgs<R>{coord.ptr, gamma.ptr, so0.ptr, so1.ptr, cfl.ptr, n, time_increment / 2.0,
-                          time_increment / 4.0, invdx.ptr, invd2.ptr, seo.ptr};
+        return E1DArgs{gamma.ptr, so0.ptr, so1.ptr, cfl.ptr, n, time_increment / 2.0, time_increment / 4.0,
+                       invdx.ptr, invd2.ptr, cflr.ptr, seo.ptr};
     }
 
     // Loop bounds of a half step (Euler1DCore.cpp:73-74, 99-100).
@@ -495,8 +476,12 @@ public:
     {
         int64_t start, nout;
         range(odd, start, nout);
-        unsigned const grid = static_cast<unsigned>((nout + B1D) / B1D);
-        k_half<R><<<grid, B1D, 0, stream>>>(args(), start, nout, mask);
+        // Blocks of one warp while they all are resident at once (32 blocks
+        // on each of 152 SMs), so that a tube takes the FP64 pipes of as many
+        // SMs as it has warps; beyond that blocks of four.
+        int64_t const warps = std::max<int64_t>((nout + WOUT - 1) / WOUT, 1);
+        int const wpb = warps <= 152 * 32 ? 1 : 4;
+        k_half<<<static_cast<unsigned>((warps + wpb - 1) / wpb), 32 * wpb, 0, stream>>>(args(), start, nout, mask);
         scg::launched(stream, "e1d_half");
     }
 
@@ -510,7 +495,7 @@ public:
             range(odd != 0, start, nout);
             if (nout > 0)
             {
-                k_cfl1d<R><<<static_cast<unsigned>((nout + 255) / 256), 256, 0, stream>>>(args(), start, nout);
+                k_cfl1d<<<static_cast<unsigned>((nout + 255) / 256), 256, 0, stream>>>(args(), start, nout);
                 scg::launched(stream, "e1d_cfl");
             }
             break;
@@ -523,7 +508,7 @@ public:
             break;
         case 3: // treat_boundary_so0
         case 4: // treat_boundary_so1
-            k_bnd1d<R><<<1, 1, 0, stream>>>(args(), which - 3);
+            k_bnd1d<<<1, 1, 0, stream>>>(args(), which - 3);
             scg::launched(stream, "e1d_bnd");
             break;
         case 5: // setup_march
@@ -532,7 +517,7 @@ public:
             range(false, start, nout);
             if (nout > 0)
             {
-                k_cfl1d<R><<<static_cast<unsigned>((nout + 255) / 256), 256, 0, stream>>>(args(), start, nout);
+                k_cfl1d<<<static_cast<unsigned>((nout + 255) / 256), 256, 0, stream>>>(args(), start, nout);
                 scg::launched(stream, "e1d_cfl");
             }
             break;
@@ -619,8 +604,8 @@ private:
     }
 
     scg::DevBuf<double> coord;
-    scg::DevBuf<double> invdx, invd2, seo; // see E1DArgs
-    scg::DevBuf<R> cfl, so0, so1, gamma;
+    scg::DevBuf<double> invdx, invd2, cflr, seo; // see E1DArgs
+    scg::DevBuf<double> cfl, so0, so1, gamma;
     cudaGraphExec_t graph_exec = nullptr;
     int graph_alpha = 0;
 };
@@ -1329,7 +1314,7 @@ int scg_e1d_create_precision(int64_t ncoord, double time_increment, int precisio
     return scg::guarded([&] {
         auto h = std::make_unique<scg_e1d>();
         if (precision == SCG_FP64)
-            h->c = std::make_unique<Euler1D<double>>(ncoord, time_increment);
+            h->c = std::make_unique<Euler1D>(ncoord, time_increment);
         else if (precision == SCG_FP32)
             h->c = std::make_unique<Euler1D32>(ncoord, time_increment);
         else
