@@ -117,13 +117,13 @@ struct P1D
 {
     double u[3], r, v, p, ga;
 
-    __device__ __forceinline__ P1D(E1DArgs const & a, int64_t ic)
+    __device__ __forceinline__ P1D(double const * so0, double gamma)
     {
         for (int i = 0; i < 3; ++i)
         {
-            u[i] = a.so0[ic * 3 + i];
+            u[i] = so0[i];
         }
-        ga = a.gamma[ic];
+        ga = gamma;
         r = scg::dev::recip(ad(u[0], Tiny1D<double>::V));
         v = mu(u[1], r);
         p = mu(sb(ga, 1.0), fm(-0.5, mu(u[1], v), u[2]));
@@ -141,7 +141,22 @@ struct P1D
     }
 };
 
-// The solution-element kernel at point ic (Euler1DKernel::set_value and
+// The offsets of the solution element at point ic (E1DArgs::seo).
+struct Offsets1D
+{
+    double dxctr, dxl, dml, dxr, dmr;
+
+    __device__ __forceinline__ Offsets1D(E1DArgs const & a, int64_t ic)
+        : dxctr(a.seo[0 * a.n + ic])
+        , dxl(a.seo[1 * a.n + ic])
+        , dml(a.seo[2 * a.n + ic])
+        , dxr(a.seo[3 * a.n + ic])
+        , dmr(a.seo[4 * a.n + ic])
+    {
+    }
+};
+
+// The solution-element kernel at one point (Euler1DKernel::set_value and
 // derive, Euler1DCore.hpp:193-244): the value up at the next half level and the
 // two half fluxes of calc_flux_ll/lr (Euler1DCore.hpp:246-266).
 struct K1D
@@ -150,14 +165,10 @@ struct K1D
     double ll[3]; // flux through the lower-left of the CE to the right
     double lr[3]; // flux through the lower-right of the CE to the left
 
-    __device__ __forceinline__ void derive(E1DArgs const & a, int64_t ic, P1D const & q)
+    __device__ __forceinline__ K1D(E1DArgs const & a, P1D const & q, double const * ux, Offsets1D const & x)
     {
         double const * const u = q.u;
-        double ux[3], ut[3], ft[3];
-        for (int i = 0; i < 3; ++i)
-        {
-            ux[i] = a.so1[ic * 3 + i];
-        }
+        double jx[3], jj[3]; // J u_x = -u_t and J J u_x = -f_t, J the flux's Jacobian
         double const ga1 = sb(q.ga, 1.0);
         double const hv = mu(mu(0.5, q.v), q.v);
         double const h = ad(u[2], q.p);
@@ -169,24 +180,15 @@ struct K1D
             o[1] = fm(u[1], dv, fm(w[1], q.v, dp));
             o[2] = fm(h, dv, mu(ad(w[2], dp), q.v));
         };
-        along(ux, ut);
-        for (int i = 0; i < 3; ++i)
-        {
-            ut[i] = -ut[i];
-        }
-        along(ut, ft);
+        along(ux, jx);
+        along(jx, jj);
         double const f[3] = {u[1], fm(u[1], q.v, q.p), mu(h, q.v)};
-        double const dxctr = a.seo[0 * a.n + ic];
-        double const dxl = a.seo[1 * a.n + ic];
-        double const dml = a.seo[2 * a.n + ic];
-        double const dxr = a.seo[3 * a.n + ic];
-        double const dmr = a.seo[4 * a.n + ic];
         for (int i = 0; i < 3; ++i)
         {
-            up[i] = fm(a.hdt, ut[i], fm(dxctr, ux[i], u[i]));
-            double const tf = mu(a.hdt, fm(a.qdt, ft[i], fm(-dxctr, ut[i], f[i])));
-            ll[i] = fm(dxl, fm(dml, ux[i], u[i]), tf);
-            lr[i] = fm(dxr, fm(dmr, ux[i], u[i]), -tf);
+            up[i] = fm(-a.hdt, jx[i], fm(x.dxctr, ux[i], u[i]));
+            double const tf = mu(a.hdt, fm(-a.qdt, jj[i], fm(x.dxctr, jx[i], f[i])));
+            ll[i] = fm(x.dxl, fm(x.dml, ux[i], u[i]), tf);
+            lr[i] = fm(x.dxr, fm(x.dmr, ux[i], u[i]), -tf);
         }
     }
 };
@@ -228,9 +230,8 @@ __device__ __forceinline__ void half_warp(E1DArgs const & a, int64_t start, int6
     int const lane = static_cast<int>(threadIdx.x) & 31;
     int64_t const j = w * WOUT + lane;
     int64_t const ic = start + 2 * (j < nout ? j : nout); // lanes past the end repeat the last kernel
-    P1D const q(a, ic);
-    K1D k;
-    k.derive(a, ic, q);
+    P1D const q(a.so0 + ic * 3, a.gamma[ic]);
+    K1D const k(a, q, a.so1 + ic * 3, Offsets1D(a, ic));
     double const idxr = a.invdx[ic - 1]; // 1 / (x - xneg)
     double lr[3], up[3];
     for (int i = 0; i < 3; ++i)
@@ -302,6 +303,243 @@ __global__ void __launch_bounds__(128) k_half(E1DArgs a, int64_t start, int64_t 
     }
 }
 
+// Small tubes: a whole march in one launch of one cluster of at most 16 blocks,
+// the tube in the threads' registers.  A half step of a small tube is latency
+// and nothing else, most of it outside the arithmetic: the launch, the loads
+// from the L2 and the stores on their way back (201 points FP64: 6.4 us per
+// half step in a graph of launches, 8.4 launched singly, 5.7 with one cluster
+// marching the state in the L2).  Thread k keeps the even point 2k and the odd
+// point 2k + 1; a half step hands what one neighbour needs of each kernel along
+// by shuffles within a warp, and from warp to warp through a slot of shared
+// memory (of the neighbouring block's, where it lies there), ordered by the
+// cluster's hardware barrier once per half step.
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// A slot of shared memory of another block of the cluster, and a store to it.
+__device__ __forceinline__ unsigned slot_of(void const * p, unsigned rank)
+{
+    unsigned out;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;"
+        : "=r"(out)
+        : "r"(static_cast<unsigned>(__cvta_generic_to_shared(p))), "r"(rank));
+    return out;
+}
+__device__ __forceinline__ void slot_put(unsigned at, double v)
+{
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(at), "d"(v) : "memory");
+}
+__device__ __forceinline__ void slot_put(unsigned at, float v)
+{
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(v) : "memory");
+}
+
+// Hands N values of each thread's v to the thread before it (Q = 1, into w) or
+// after it (Q = 0), over the whole cluster; slots: this half step's, one row of N
+// per warp of the block.  Every thread of the cluster calls it.  The threads
+// at the cluster's ends receive their own values or an unwritten slot's, which
+// they do not use.
+template <int N, int Q, typename R>
+__device__ __forceinline__ void hand_over(R const * v, R * w, R (*slots)[N])
+{
+    int const ln = static_cast<int>(threadIdx.x) & 31;
+    int const warp = static_cast<int>(threadIdx.x) >> 5;
+    int const last = static_cast<int>(blockDim.x >> 5) - 1;
+    int const from = Q == 1 ? 0 : 31; // the lane whose values leave the warp
+    if (ln == from)
+    {
+        int const to = Q == 1 ? warp - 1 : warp + 1;
+        unsigned const me = blockIdx.x;
+        if (to >= 0 && to <= last)
+        {
+            for (int i = 0; i < N; ++i)
+            {
+                slots[to][i] = v[i];
+            }
+        }
+        else if (Q == 1 ? me > 0 : me + 1 < gridDim.x)
+        {
+            unsigned const at = slot_of(slots[Q == 1 ? last : 0], Q == 1 ? me - 1 : me + 1);
+            for (int i = 0; i < N; ++i)
+            {
+                slot_put(at + static_cast<unsigned>(i * sizeof(R)), v[i]);
+            }
+        }
+    }
+    cluster_sync();
+    for (int i = 0; i < N; ++i)
+    {
+        R const x = Q == 1 ? __shfl_down_sync(0xffffffffu, v[i], 1) : __shfl_up_sync(0xffffffffu, v[i], 1);
+        w[i] = ln == 31 - from ? slots[warp][i] : x;
+    }
+}
+
+// A block's warps at most: one for each of the SM's four FP64 pipes (measured,
+// per half step: 3.9 us up to 2,001 points, 4.35 us at 4,001, against 6.0 to
+// 6.4 us in graph launches; a second warp per pipe: 7.6 against 6.2).
+constexpr int TUBE_WARPS64 = 4;
+
+__global__ void __launch_bounds__(32 * TUBE_WARPS64) k_tube(E1DArgs a, int alpha, int64_t steps, int64_t nout1,
+                                                            int64_t nout2)
+{
+    __shared__ double slots[2][TUBE_WARPS64][6];
+    int64_t const nk = (a.n - 1) / 2; // threads with a point pair
+    int64_t const t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    int64_t const k = t < nk ? t : nk - 1; // the others repeat the last pair, and write nothing
+    int64_t const e = 2 * k, o = 2 * k + 1;
+    int64_t const l = k > 0 ? e - 1 : 0;
+    double ue[3], xe[3], uo[3], xo[3];
+    for (int i = 0; i < 3; ++i)
+    {
+        ue[i] = a.so0[e * 3 + i];
+        xe[i] = a.so1[e * 3 + i];
+        uo[i] = a.so0[o * 3 + i];
+        xo[i] = a.so1[o * 3 + i];
+    }
+    double const ge = a.gamma[e], go = a.gamma[o];
+    Offsets1D const oe(a, e), oo(a, o);
+    double const il = a.invdx[l], ie = a.invdx[e], io = a.invdx[o];
+    double const dl = a.invd2[l], de = a.invd2[e];
+    bool const out1 = t >= 1 && t <= nout1, out2 = t >= 1 && t <= nout2;
+    cluster_sync(); // every block runs before any stores to another's slots
+    for (int64_t s = 0; s < steps; ++s)
+    {
+        bool const end = s + 1 == steps; // a CFL number is overwritten by the next step's
+        // First half step: odd points from the even kernels k and k + 1.
+        {
+            P1D const q(ue, ge);
+            K1D const c(a, q, xe, oe);
+            double const v[6] = {c.lr[0], c.lr[1], c.lr[2], c.up[0], c.up[1], c.up[2]};
+            double w[6];
+            hand_over<6, 1>(v, w, slots[0]);
+            // The copy-out boundary: point 1 takes point 2's, n - 2 takes n - 3's.
+            for (int i = 0; i < 3; ++i)
+            {
+                double const un = __shfl_down_sync(0xffffffffu, ue[i], 1);
+                double const xn = __shfl_down_sync(0xffffffffu, xe[i], 1);
+                if (t == 0)
+                {
+                    uo[i] = un;
+                    xo[i] = xn;
+                }
+                else if (t == nk - 1)
+                {
+                    uo[i] = ue[i];
+                    xo[i] = xe[i];
+                }
+            }
+            if (out1)
+            {
+                for (int i = 0; i < 3; ++i)
+                {
+                    uo[i] = mu(ad(c.ll[i], w[i]), de);
+                    xo[i] = wgrad(alpha, mu(sb(uo[i], c.up[i]), ie), mu(sb(w[3 + i], uo[i]), io));
+                }
+                if (end)
+                {
+                    a.cfl[e] = q.cfl(a.cflr[e]);
+                }
+            }
+        }
+        // Second half step: even points from the odd kernels k - 1 and k.
+        {
+            P1D const q(uo, go);
+            K1D const c(a, q, xo, oo);
+            double const v[6] = {c.ll[0], c.ll[1], c.ll[2], c.up[0], c.up[1], c.up[2]};
+            double w[6];
+            hand_over<6, 0>(v, w, slots[1]);
+            if (out2)
+            {
+                for (int i = 0; i < 3; ++i)
+                {
+                    ue[i] = mu(ad(w[i], c.lr[i]), dl);
+                    xe[i] = wgrad(alpha, mu(sb(ue[i], w[3 + i]), il), mu(sb(c.up[i], ue[i]), ie));
+                }
+            }
+            if (end && t < nout2)
+            {
+                a.cfl[o] = q.cfl(a.cflr[o]);
+            }
+        }
+    }
+    if (t < nk)
+    {
+        for (int i = 0; i < 3; ++i)
+        {
+            a.so0[e * 3 + i] = ue[i];
+            a.so1[e * 3 + i] = xe[i];
+            a.so0[o * 3 + i] = uo[i];
+            a.so1[o * 3 + i] = xo[i];
+        }
+    }
+}
+
+// The largest cluster this GPU schedules for a kernel at `threads` threads a
+// block: 16 where it can (a non-portable size), else 8.  Asked once per kernel.
+template <auto KERNEL, int THREADS>
+int cluster_limit()
+{
+    static int const limit = [] {
+        cudaLaunchAttribute attr{};
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim = {16, 1, 1};
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(16);
+        cfg.blockDim = dim3(THREADS);
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaFuncSetAttribute(KERNEL, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+            cudaOccupancyMaxActiveClusters(&n, KERNEL, &cfg) == cudaSuccess && n > 0)
+        {
+            return 16;
+        }
+        (void)cudaGetLastError();
+        return 8;
+    }();
+    return limit;
+}
+
+// Launch a kernel as one cluster of `blocks` blocks.
+template <typename K, typename... A>
+void launch_cluster(K * kernel, int blocks, int threads, cudaStream_t stream, A... args)
+{
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim = {static_cast<unsigned>(blocks), 1, 1};
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(blocks));
+    cfg.blockDim = dim3(static_cast<unsigned>(threads));
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    scg::cuda_check(cudaLaunchKernelEx(&cfg, kernel, args...), "cluster launch");
+}
+
+// Steps per launch of the cluster kernels (a launch of a few milliseconds).
+constexpr int64_t CLUSTER_STEPS = 1024;
+
+// Blocks and warps per block of a cluster that holds a tube of n points, one
+// point pair per thread: as many blocks as the limit allows before a second
+// warp per block, so that the warps have an SM each as long as there are SMs.
+// False where the tube does not fit.
+template <auto KERNEL, int MAX_WARPS>
+bool tube_shape(int64_t n, int & blocks, int & warps)
+{
+    int const limit = cluster_limit<KERNEL, 32 * MAX_WARPS>();
+    int64_t const w = ((n - 1) / 2 + 31) / 32;
+    blocks = 1;
+    while (blocks < limit && blocks < w)
+    {
+        blocks *= 2;
+    }
+    warps = static_cast<int>(std::min<int64_t>((w + blocks - 1) / blocks, MAX_WARPS + 1));
+    return warps <= MAX_WARPS;
+}
+
 // update_cfl alone.
 __global__ void k_cfl1d(E1DArgs a, int64_t start, int64_t nout)
 {
@@ -309,7 +547,7 @@ __global__ void k_cfl1d(E1DArgs a, int64_t start, int64_t nout)
     if (j < nout)
     {
         int64_t const it = start + 2 * j;
-        a.cfl[it] = P1D(a, it).cfl(a.cflr[it]);
+        a.cfl[it] = P1D(a.so0 + it * 3, a.gamma[it]).cfl(a.cflr[it]);
     }
 }
 
@@ -542,13 +780,18 @@ public:
         half(H_SO0 | H_CFL | h_alpha(alpha), true);
     }
 
-    // march_alpha(steps): chunks of GRAPH_STEPS steps replay one captured
-    // CUDA graph; the remainder launches directly.
+    // march_alpha(steps): a small tube in launches of one cluster, a larger one
+    // in chunks of GRAPH_STEPS steps that replay one captured CUDA graph, the
+    // remainder launched directly.
     void march(int alpha, int64_t steps) override
     {
         if (alpha != 1 && alpha != 2)
         {
             throw std::invalid_argument("Euler1DCore: alpha must be 1 or 2");
+        }
+        if (cluster_march(alpha, steps))
+        {
+            return;
         }
         int64_t const chunks = steps / GRAPH_STEPS;
         if (chunks > 0)
@@ -567,6 +810,25 @@ public:
         {
             step(alpha);
         }
+    }
+
+    bool cluster_march(int alpha, int64_t steps)
+    {
+        int blocks, warps;
+        if (!tube_shape<k_tube, TUBE_WARPS64>(n, blocks, warps))
+        {
+            return false;
+        }
+        int64_t start, nout1, nout2;
+        range(false, start, nout1);
+        range(true, start, nout2);
+        for (int64_t s = 0; s < steps; s += CLUSTER_STEPS)
+        {
+            launch_cluster(k_tube, blocks, 32 * warps, stream, args(), alpha, std::min(CLUSTER_STEPS, steps - s), nout1,
+                           nout2);
+            scg::launched(stream, "e1d_tube");
+        }
+        return true;
     }
 
     void capture(int alpha)
@@ -644,6 +906,17 @@ struct Planes
         return base + (static_cast<int64_t>(parity) * PL_COUNT + q) * P;
     }
 };
+
+// Warps at most of a block that holds part of a tube in registers (1,024
+// threads: 32,769 points over 16 blocks).  Per half step 0.53 us up to 2,001
+// points, 0.69 us at 8,001, 1.12 us at 20,001 and 1.56 us at 32,001, against 2.1
+// to 2.8 us in graph launches.
+constexpr int TUBE_WARPS32 = 32;
+// The largest FP32 tubes whose half steps take one output per lane instead of
+// four per thread (per half step 2.6 against 3.1 us at 80,001 points, 3.5
+// against 4.3 us at 320,001, 4.9 against 4.8 us at 640,001, 8.1 against 7.3 us at
+// 1,280,001, where the four outputs' wider loads pay).
+constexpr int64_t WARP_POINTS32 = 400000;
 
 // Division in the FP32 core: the approximate quotient (within 2 ulp over the
 // normal range; every divisor here is a spacing, a density or a positive sum
@@ -744,6 +1017,41 @@ __device__ __forceinline__ float lane(float4 v, int i)
     return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w;
 }
 
+// One output between its left and right kernels: the new so0 in delta form
+// (DO_SO0: the old value u0 plus a change formed from the kernels' states
+// relative to it, so FP32 rounding scales with the change; without it u0 is the
+// new value already) and, for ALPHA > 0, so1 by the W-alpha gradient.
+template <int ALPHA, bool DO_SO0>
+__device__ __forceinline__ void output32(K32 const & L, K32 const & R, float const * u0, float * nso0, float * nso1)
+{
+    float const dxl = L.dp;
+    float const dxr = R.dm;
+    float const idx = div32(1.f, dxl + dxr);
+#pragma unroll
+    for (int v = 0; v < 3; ++v)
+    {
+        float d;
+        if constexpr (DO_SO0)
+        {
+            d = (dxl * (L.u[v] - u0[v]) + dxr * (R.u[v] - u0[v]) + L.llp[v] + R.lrp[v]) * idx;
+            nso0[v] = u0[v] + d;
+        }
+        else
+        {
+            d = 0.f;
+            nso0[v] = u0[v];
+        }
+        if constexpr (ALPHA > 0)
+        {
+            // The gradient's differences v - up_l and up_r - v from small
+            // terms: (u0 - u_l) + d - (up_l - u_l), (u_r - u0) + (up_r - u_r) - d.
+            float const duxn = div32((u0[v] - L.u[v]) + d - L.upd[v], dxl);
+            float const duxp = div32((R.u[v] - u0[v]) + R.upd[v] - d, dxr);
+            nso1[v] = wgrad32<ALPHA>(duxn, duxp);
+        }
+    }
+}
+
 // One half step of the FP32 core, outputs of parity Q from the kernels of the
 // other parity.  Output o (1 <= o <= nout) sits between its left and right
 // kernels: kernel indices o and o + 1 when the outputs are odd points (the
@@ -754,28 +1062,12 @@ __device__ __forceinline__ float lane(float4 v, int i)
 // change formed from the kernels' states relative to it, so FP32 rounding
 // scales with the change); without it so0 is already new and only so1 is
 // formed.  ALPHA > 0: so1 by the W-alpha gradient.  DO_CFL: update_cfl at
-// each output's left kernel.  BND: the copy-out boundary treatment of points
-// 1 and n - 2, which the half step neither reads nor writes.
-template <int ALPHA, bool DO_SO0, bool DO_CFL, bool BND, int Q>
-__global__ void __launch_bounds__(B32) k_half32(Planes a, int64_t nout)
+// each output's left kernel.  k_half32's BND: the copy-out boundary treatment
+// of points 1 and n - 2, which the half step neither reads nor writes.
+template <int ALPHA, bool DO_SO0, bool DO_CFL, int Q>
+__device__ __forceinline__ void half32_four(Planes const & a, int64_t nout, int64_t c)
 {
     constexpr int P = 1 - Q; // parity of the kernels
-    if (BND && blockIdx.x == 0 && threadIdx.x == 0)
-    {
-        int64_t const hi = (a.n - 3) / 2;
-        for (int v = 0; v < 3; ++v)
-        {
-            a.at(1, PL_SO0 + v)[0] = a.at(0, PL_SO0 + v)[1];
-            a.at(1, PL_SO0 + v)[hi] = a.at(0, PL_SO0 + v)[hi];
-            a.at(1, PL_SO1 + v)[0] = a.at(0, PL_SO1 + v)[1];
-            a.at(1, PL_SO1 + v)[hi] = a.at(0, PL_SO1 + v)[hi];
-        }
-    }
-    int64_t const c = 4 * (static_cast<int64_t>(blockIdx.x) * B32 + threadIdx.x);
-    if (c > nout)
-    {
-        return;
-    }
     // The five kernels in index order: Q = 1 uses c .. c + 4, Q = 0 uses
     // c - 1 .. c + 3; the one outside the aligned four is the halo.
     int64_t const h = Q == 1 ? c + 4 : c - 1;
@@ -841,31 +1133,16 @@ __global__ void __launch_bounds__(B32) k_half32(Planes a, int64_t nout)
     {
         K32 R;
         kernel(k + 1, R);
-        float const dxl = L.dp;
-        float const dxr = R.dm;
-        float const idx = div32(1.f, dxl + dxr);
+        float const u0[3] = {lane(o4[0], k), lane(o4[1], k), lane(o4[2], k)};
+        float n0[3], n1[3];
+        output32<ALPHA, DO_SO0>(L, R, u0, n0, n1);
 #pragma unroll
         for (int v = 0; v < 3; ++v)
         {
-            float const u0 = lane(o4[v], k);
-            float d;
-            if constexpr (DO_SO0)
-            {
-                d = (dxl * (L.u[v] - u0) + dxr * (R.u[v] - u0) + L.llp[v] + R.lrp[v]) * idx;
-                nso0[v][k] = u0 + d;
-            }
-            else
-            {
-                d = 0.f; // u0 is the new value already
-                nso0[v][k] = u0;
-            }
+            nso0[v][k] = n0[v];
             if constexpr (ALPHA > 0)
             {
-                // The gradient's differences v - up_l and up_r - v from small
-                // terms: (u0 - u_l) + d - (up_l - u_l), (u_r - u0) + (up_r - u_r) - d.
-                float const duxn = div32((u0 - L.u[v]) + d - L.upd[v], dxl);
-                float const duxp = div32((R.u[v] - u0) + R.upd[v] - d, dxr);
-                nso1[v][k] = wgrad32<ALPHA>(duxn, duxp);
+                nso1[v][k] = n1[v];
             }
         }
         if constexpr (DO_CFL)
@@ -922,6 +1199,206 @@ __global__ void __launch_bounds__(B32) k_half32(Planes a, int64_t nout)
                 cf[k] = ncfl[k];
             }
         }
+    }
+}
+
+// One warp's part of a half step with one output per lane, for tubes that
+// leave the GPU's warps idle, where the latency of a thread's four outputs in
+// turn would set the time: lane l derives kernel 31 w + l of those the half
+// step reads, and lanes 0 .. 30 update the output to its right, with the next
+// lane's kernel by shuffles.
+template <int ALPHA, int Q>
+__device__ __forceinline__ void half32_warp(Planes const & a, int64_t nout, int64_t w)
+{
+    constexpr int P = 1 - Q;
+    int const ln = static_cast<int>(threadIdx.x) & 31;
+    int64_t const j = w * WOUT + ln;           // kernel j, output j + 1
+    int64_t const i = (j < nout ? j : nout) + Q; // its index in its plane
+    int64_t const o = (j < nout ? j : nout - 1) + 1;
+    float u[3], x[3], u0[3];
+#pragma unroll
+    for (int v = 0; v < 3; ++v)
+    {
+        u[v] = a.at(P, PL_SO0 + v)[i];
+        x[v] = a.at(P, PL_SO1 + v)[i];
+        u0[v] = a.at(Q, PL_SO0 + v)[o];
+    }
+    K32 L, R;
+    derive32(u, x, a.at(P, PL_GAMMA)[i], a.at(P, PL_DXM)[i], a.at(P, PL_DXP)[i], a.hdt, a.qdt, L);
+#pragma unroll
+    for (int v = 0; v < 3; ++v)
+    {
+        R.u[v] = __shfl_down_sync(0xffffffffu, L.u[v], 1);
+        R.upd[v] = __shfl_down_sync(0xffffffffu, L.upd[v], 1);
+        R.lrp[v] = __shfl_down_sync(0xffffffffu, L.lrp[v], 1);
+    }
+    R.dm = __shfl_down_sync(0xffffffffu, L.dm, 1);
+    if (ln < WOUT && j < nout)
+    {
+        float n0[3], n1[3];
+        output32<ALPHA, true>(L, R, u0, n0, n1);
+#pragma unroll
+        for (int v = 0; v < 3; ++v)
+        {
+            a.at(Q, PL_SO0 + v)[o] = n0[v];
+            a.at(Q, PL_SO1 + v)[o] = n1[v];
+        }
+        a.at(P, PL_CFL)[i] = cfl32(L, a.hdt);
+    }
+}
+
+// The copy-out boundary treatment of points 1 and n - 2.
+__device__ __forceinline__ void copy_out32(Planes const & a)
+{
+    int64_t const hi = (a.n - 3) / 2;
+    for (int v = 0; v < 3; ++v)
+    {
+        a.at(1, PL_SO0 + v)[0] = a.at(0, PL_SO0 + v)[1];
+        a.at(1, PL_SO0 + v)[hi] = a.at(0, PL_SO0 + v)[hi];
+        a.at(1, PL_SO1 + v)[0] = a.at(0, PL_SO1 + v)[1];
+        a.at(1, PL_SO1 + v)[hi] = a.at(0, PL_SO1 + v)[hi];
+    }
+}
+
+template <int ALPHA, bool DO_SO0, bool DO_CFL, bool BND, int Q>
+__global__ void __launch_bounds__(B32) k_half32(Planes a, int64_t nout)
+{
+    if (BND && blockIdx.x == 0 && threadIdx.x == 0)
+    {
+        copy_out32(a);
+    }
+    int64_t const c = 4 * (static_cast<int64_t>(blockIdx.x) * B32 + threadIdx.x);
+    if (c <= nout)
+    {
+        half32_four<ALPHA, DO_SO0, DO_CFL, Q>(a, nout, c);
+    }
+}
+
+// A small tube's whole march in one cluster, in registers (see k_tube).
+template <int ALPHA>
+__global__ void __launch_bounds__(32 * TUBE_WARPS32) k_tube32(Planes a, int64_t steps, int64_t nout1, int64_t nout2)
+{
+    __shared__ float slots[2][TUBE_WARPS32][10];
+    int64_t const nk = (a.n - 1) / 2;
+    int64_t const t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    int64_t const k = t < nk ? t : nk - 1;
+    float ue[3], xe[3], uo[3], xo[3];
+#pragma unroll
+    for (int v = 0; v < 3; ++v)
+    {
+        ue[v] = a.at(0, PL_SO0 + v)[k];
+        xe[v] = a.at(0, PL_SO1 + v)[k];
+        uo[v] = a.at(1, PL_SO0 + v)[k];
+        xo[v] = a.at(1, PL_SO1 + v)[k];
+    }
+    float const ge = a.at(0, PL_GAMMA)[k], go = a.at(1, PL_GAMMA)[k];
+    float const me = a.at(0, PL_DXM)[k], mo = a.at(1, PL_DXM)[k];
+    float const pe = a.at(0, PL_DXP)[k], po = a.at(1, PL_DXP)[k];
+    bool const out1 = t >= 1 && t <= nout1, out2 = t >= 1 && t <= nout2;
+    cluster_sync(); // every block runs before any stores to another's slots
+    for (int64_t s = 0; s < steps; ++s)
+    {
+        bool const end = s + 1 == steps;
+        {
+            K32 L, R;
+            derive32(ue, xe, ge, me, pe, a.hdt, a.qdt, L);
+            float const v[10] = {L.u[0],   L.u[1],   L.u[2],   L.upd[0], L.upd[1],
+                                 L.upd[2], L.lrp[0], L.lrp[1], L.lrp[2], L.dm};
+            float w[10];
+            hand_over<10, 1>(v, w, slots[0]);
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+            {
+                R.u[i] = w[i];
+                R.upd[i] = w[3 + i];
+                R.lrp[i] = w[6 + i];
+                float const un = __shfl_down_sync(0xffffffffu, ue[i], 1);
+                float const xn = __shfl_down_sync(0xffffffffu, xe[i], 1);
+                if (t == 0)
+                {
+                    uo[i] = un;
+                    xo[i] = xn;
+                }
+                else if (t == nk - 1)
+                {
+                    uo[i] = ue[i];
+                    xo[i] = xe[i];
+                }
+            }
+            R.dm = w[9];
+            if (out1)
+            {
+                float n0[3], n1[3];
+                output32<ALPHA, true>(L, R, uo, n0, n1);
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+                {
+                    uo[i] = n0[i];
+                    xo[i] = n1[i];
+                }
+                if (end)
+                {
+                    a.at(0, PL_CFL)[k] = cfl32(L, a.hdt);
+                }
+            }
+        }
+        {
+            K32 L, R;
+            derive32(uo, xo, go, mo, po, a.hdt, a.qdt, R);
+            float const v[10] = {R.u[0],   R.u[1],   R.u[2],   R.upd[0], R.upd[1],
+                                 R.upd[2], R.llp[0], R.llp[1], R.llp[2], R.dp};
+            float w[10];
+            hand_over<10, 0>(v, w, slots[1]);
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+            {
+                L.u[i] = w[i];
+                L.upd[i] = w[3 + i];
+                L.llp[i] = w[6 + i];
+            }
+            L.dp = w[9];
+            if (out2)
+            {
+                float n0[3], n1[3];
+                output32<ALPHA, true>(L, R, ue, n0, n1);
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+                {
+                    ue[i] = n0[i];
+                    xe[i] = n1[i];
+                }
+            }
+            if (end && t < nout2)
+            {
+                a.at(1, PL_CFL)[k] = cfl32(R, a.hdt);
+            }
+        }
+    }
+    if (t < nk)
+    {
+#pragma unroll
+        for (int v = 0; v < 3; ++v)
+        {
+            a.at(0, PL_SO0 + v)[k] = ue[v];
+            a.at(0, PL_SO1 + v)[k] = xe[v];
+            a.at(1, PL_SO0 + v)[k] = uo[v];
+            a.at(1, PL_SO1 + v)[k] = xo[v];
+        }
+    }
+}
+
+// The march's half step with one output per lane.
+template <int ALPHA, bool BND, int Q>
+__global__ void __launch_bounds__(B32) k_half32_warp(Planes a, int64_t nout)
+{
+    if (BND && blockIdx.x == 0 && threadIdx.x == 0)
+    {
+        copy_out32(a);
+    }
+    int64_t const w = (static_cast<int64_t>(blockIdx.x) * B32 + threadIdx.x) / 32;
+    if (w * WOUT < nout)
+    {
+        half32_warp<ALPHA, Q>(a, nout, w);
     }
 }
 
@@ -1151,6 +1628,24 @@ public:
         {
             return;
         }
+        if constexpr (SO0 && CFL)
+        {
+            if (n <= WARP_POINTS32)
+            {
+                int64_t const warps = (nout + WOUT - 1) / WOUT;
+                unsigned const g = static_cast<unsigned>((warps * 32 + B32 - 1) / B32);
+                if (odd)
+                {
+                    k_half32_warp<ALPHA, BND, 0><<<g, B32, 0, stream>>>(args(), nout);
+                }
+                else
+                {
+                    k_half32_warp<ALPHA, BND, 1><<<g, B32, 0, stream>>>(args(), nout);
+                }
+                scg::launched(stream, "e1d_half32_warp");
+                return;
+            }
+        }
         int64_t const threads = nout / 4 + 1;
         unsigned const grid = static_cast<unsigned>((threads + B32 - 1) / B32);
         if (odd)
@@ -1241,6 +1736,10 @@ public:
         {
             throw std::invalid_argument("Euler1DCore: alpha must be 1 or 2");
         }
+        if (cluster_march(alpha, steps))
+        {
+            return;
+        }
         int64_t const chunks = steps / GRAPH_STEPS;
         if (chunks > 0)
         {
@@ -1258,6 +1757,29 @@ public:
         {
             step(alpha);
         }
+    }
+
+    template <int ALPHA>
+    bool tube_march(int64_t steps)
+    {
+        int64_t const nout1 = nout_of(false), nout2 = nout_of(true);
+        int blocks, warps;
+        if (nout1 <= 0 || !tube_shape<k_tube32<ALPHA>, TUBE_WARPS32>(n, blocks, warps))
+        {
+            return false;
+        }
+        for (int64_t s = 0; s < steps; s += CLUSTER_STEPS)
+        {
+            launch_cluster(k_tube32<ALPHA>, blocks, 32 * warps, stream, args(), std::min(CLUSTER_STEPS, steps - s),
+                           nout1, nout2);
+            scg::launched(stream, "e1d_tube32");
+        }
+        return true;
+    }
+
+    bool cluster_march(int alpha, int64_t steps)
+    {
+        return alpha == 1 ? tube_march<1>(steps) : tube_march<2>(steps);
     }
 
     void capture(int alpha)
