@@ -439,10 +439,10 @@ int scg_st_stream(const scg_st * solver, void ** out);
  * which a core refuses, are not defined here), for checking that rounding.  Synchronous; allocates its own device buffers. */
 int scg_geometry_round(const double * in, float * out, int64_t n);
 /* Not in the reference: n FP64 quotients x[i] / d[i] on the device, q by
- * the spacetime march's division from a tabulated reciprocal (Markstein's
- * method) and qdiv by the IEEE division, for checking that the two agree bit
- * for bit; rcp[i] is the multi-dimensional FP64 march's reciprocal of d[i]
- * (Newton's iteration, within one ulp of 1 / d).  Synchronous; allocates its
+ * the spacetime march's division from a tabulated reciprocal (integer
+ * arithmetic) and qdiv by the IEEE division, for checking that the two agree
+ * bit for bit; rcp[i] is the FP64 marches' reciprocal of d[i] (Newton's
+ * iteration in integers, within one ulp of 1 / d).  Synchronous; allocates its
  * own device buffers. */
 int scg_divide_check(const double * x, const double * d, double * q, double * qdiv, double * rcp, int64_t n);
 /* Not in the reference: the FP64 march's reciprocal roots r[i] = 1 / sqrt(x[i])

@@ -1,35 +1,21 @@
 /*
- * FP64 divisions and roots that cost fewer FP64-pipe instructions than the
- * IEEE operations.
+ * FP64 reciprocals, quotients, roots and comparisons on the integer pipe.
  *
- * div_rcp: division by a tabulated reciprocal, rounded exactly as x / d.
+ * GB300 issues one FP64 instruction per SM every 19 cycles (measured; 64 on one
+ * SM sub-partition alone), and the FP64 marches keep that pipe full while the
+ * integer and FP32 pipes idle (8% of the issue slots used), so these
+ * functions form their results with integer instructions alone, half a cycle
+ * each: Newton's iteration in fixed point from the FP32 hardware
+ * approximation, the residual kept exactly or to 62 bits, the result rounded
+ * once to 53 bits.  recip, rsq and sqr_t are within 0.52 ulp, in about 30, 40
+ * and 48 instructions (4, 5 and 8 on the FP64 pipe before; a triangle's
+ * substep takes 6, 12 and 2 of them, a hexahedron's 15, 40 and 2).  div_fix is
+ * the IEEE quotient bit for bit, in about 50 (5 on the FP64 pipe from a
+ * tabulated reciprocal by Markstein's method before, more without).
+ * scg_divide_check and scg_root_check compare them on the device.
  *
- * A march that divides many times by grid-only quantities (widths,
- * spacings) can store r = 1 / d once, rounded to nearest, and recover the
- * correctly rounded quotient from it with Markstein's method (P. Markstein,
- * "Computation of elementary functions on the IBM RISC System/6000
- * processor", IBM J. Res. Dev. 34(1), 1990; the theorem is also stated in
- * Muller et al., "Handbook of Floating-Point Arithmetic"):
- *
- *   q0 = x r                  within 1.5 ulp of x / d (r within half an ulp)
- *   q1 = q0 + (x - q0 d) r    within one ulp (the correction's own error is
- *                             about 2^-53 of q0's)
- *   q2 = q1 + (x - q1 d) r    = x / d rounded to nearest (Markstein's
- *                             theorem: r within half an ulp of 1 / d, q1
- *                             within one ulp, the remainder x - q1 d exact
- *                             in a fused multiply-add)
- *
- * one multiplication and four fused multiply-adds, all on values of the
- * march.  The theorem needs the operands away from the ends of the exponent
- * range (no overflow or underflow in q, the remainder or the correction), so
- * both |x| and |d| must lie in [2^-400, 2^400); a zero x is exact too (q0
- * carries its sign, which the corrections would lose).  Anything else
- * (denormals, infinities, NaN, a d whose reciprocal was not tabulated)
- * divides.  The results equal CUDA's IEEE division bit for bit; the device
- * check scg_divide_check compares the two.
- *
- * recip, rsq, sqr_t: reciprocals and roots within 0.52 ulp, on the integer
- * pipe (below).
+ * Operands outside the stated ranges take the division or the library
+ * function behind a branch that such values alone take.
  */
 #pragma once
 
@@ -39,54 +25,6 @@ namespace scg
 {
 namespace dev
 {
-
-// High word of |v| against [2^-400, 2^400): biased exponents 623 to 1422.
-constexpr unsigned RCP_EXP_LO = (1023u - 400u) << 20;
-constexpr unsigned RCP_EXP_SPAN = 800u << 20;
-
-__device__ __forceinline__ bool rcp_window(double v)
-{
-    unsigned const h = static_cast<unsigned>(__double2hiint(v)) & 0x7fffffffu;
-    return h - RCP_EXP_LO < RCP_EXP_SPAN;
-}
-
-// The tabulated reciprocal of d: 1 / d rounded to nearest when d is in the
-// window, else 0 (div_rcp then divides).
-__device__ __forceinline__ double rcp_tab(double d) { return rcp_window(d) ? 1.0 / d : 0.0; }
-
-static __device__ __noinline__ double div_plain(double x, double d) { return x / d; }
-
-// x / d, rounded to nearest, from r = rcp_tab(d).
-__device__ __forceinline__ double div_rcp(double x, double d, double r)
-{
-    double const q0 = x * r;
-    unsigned const hx = static_cast<unsigned>(__double2hiint(x)) & 0x7fffffffu;
-    bool const xok = hx - RCP_EXP_LO < RCP_EXP_SPAN || (hx | static_cast<unsigned>(__double2loint(x))) == 0u;
-    if (__double2hiint(r) != 0 && xok)
-    {
-        double const q1 = __fma_rn(__fma_rn(-q0, d, x), r, q0);
-        double const q2 = __fma_rn(__fma_rn(-q1, d, x), r, q1);
-        return copysign(q2, q0);
-    }
-    return div_plain(x, d);
-}
-
-// ---------------------------------------------------------------------------
-// Reciprocals and roots on the integer pipe.
-//
-// GB300 issues one FP64 instruction per SM every 16 cycles, and the FP64
-// marches keep that pipe ~88% busy while the integer and FP32 pipes idle (8%
-// of the issue slots used), so these functions form their results with
-// integer instructions alone: Newton's iteration in fixed point from the FP32
-// hardware approximation, the residual kept exactly or to 62 bits, the result
-// rounded once to 53 bits.  About 30 (recip), 40 (rsq) and 48 (sqr) integer
-// instructions in place of 4, 5 and 8 of the FP64 pipe (a triangle's substep
-// takes 6, 12 and 2 of them, a hexahedron's 15, 40 and 2).
-// Results are within 0.52 ulp (scg_divide_check and scg_root_check compare
-// them on the device).
-//
-// Operands outside the stated ranges take the division or the library
-// function behind a branch that such values alone take.
 
 // |d|'s top 24 significand bits as a float in [1, 2).
 __device__ __forceinline__ float sig_top(unsigned hi, unsigned lo)
@@ -117,11 +55,31 @@ __device__ __forceinline__ unsigned long long mul_hi64(unsigned long long a, uns
     return static_cast<unsigned long long>(ah) * bh + __umulhi(ah, bl) + __umulhi(al, bh);
 }
 
-// Reciprocal.  FP64, |d| in [2^-1022, 2^1022): with m = |d|'s significand
-// (m 2^52 an integer) and the seed y = Y 2^-24, the residual e = 1 - m y is
-// exact in the low 64 bits of the product (|e| < 2^-21), and
-// 1 / m = y (1 + e + e^2) up to 2^-65.  Outside that range (zero, subnormals,
-// the largest magnitudes, infinities, NaN) the division.  FP32: the division.
+// d's significand as an integer in [2^52, 2^53).
+__device__ __forceinline__ unsigned long long sig53(unsigned hi, unsigned lo)
+{
+    return (static_cast<unsigned long long>((hi & 0xfffffu) | 0x100000u) << 32) | lo;
+}
+
+// 2^62 / m for the significand m in [1, 2) of d's words: with the seed
+// y = Y 2^-24 the residual e = 1 - m y is exact in the low 64 bits of the
+// product (|e| < 2^-21), and 1 / m = y (1 + e + e^2) up to 2^-65.  Within 2^-58
+// of itself.
+__device__ __forceinline__ unsigned long long rcp_sig(unsigned hi, unsigned lo)
+{
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(sig_top(hi, lo)));
+    unsigned const Y = seed24(y);
+    long long const E = -mul_s64_u24(static_cast<long long>(sig53(hi, lo)), Y); // e 2^76
+    int const Es = static_cast<int>(E >> 24);                                   // e 2^52
+    long long const T = (E >> 14) + (static_cast<long long>(Es) * Es >> 42);    // (e + e^2) 2^62
+    return (static_cast<unsigned long long>(Y) << 38) +
+           static_cast<unsigned long long>(mul_s64_u24((T + 4) >> 3, Y) >> 21);
+}
+
+// Reciprocal.  FP64: |d| in [2^-1022, 2^1022) as above; outside it (zero,
+// subnormals, the largest magnitudes, infinities, NaN) the division.  FP32: the
+// division.
 __device__ __forceinline__ double recip(double d)
 {
     unsigned const hi = static_cast<unsigned>(__double2hiint(d));
@@ -131,20 +89,50 @@ __device__ __forceinline__ double recip(double d)
     {
         return 1.0 / d;
     }
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(sig_top(hi, lo)));
-    unsigned const Y = seed24(y);
-    unsigned long long const m =
-        (static_cast<unsigned long long>((hi & 0xfffffu) | 0x100000u) << 32) | lo;
-    long long const E = -mul_s64_u24(static_cast<long long>(m), Y); // e 2^76
-    int const Es = static_cast<int>(E >> 24);                       // e 2^52
-    long long const T = (E >> 14) + (static_cast<long long>(Es) * Es >> 42); // (e + e^2) 2^62
-    unsigned long long const r = (static_cast<unsigned long long>(Y) << 38) +
-                                 static_cast<unsigned long long>(mul_s64_u24((T + 4) >> 3, Y) >> 21); // 2^62 / m
-    unsigned long long const bits = ((r + 256u) >> 9) + (static_cast<unsigned long long>(2044u - e) << 52);
+    unsigned long long const bits =
+        ((rcp_sig(hi, lo) + 256u) >> 9) + (static_cast<unsigned long long>(2044u - e) << 52);
     return __longlong_as_double(static_cast<long long>(bits | (static_cast<unsigned long long>(hi & 0x80000000u) << 32)));
 }
 __device__ __forceinline__ float recip(float d) { return 1.0f / d; }
+
+// The significand's reciprocal of a divisor, for div_fix: 2^62 / m of a normal
+// d, else 0 (div_fix then divides).
+__device__ __forceinline__ unsigned long long rcp_fix(double d)
+{
+    unsigned const hi = static_cast<unsigned>(__double2hiint(d));
+    unsigned const e = (hi >> 20) & 0x7ffu;
+    return e - 1u < 2046u ? rcp_sig(hi, static_cast<unsigned>(__double2loint(d))) : 0ull;
+}
+
+static __device__ __noinline__ double div_plain(double x, double d) { return x / d; }
+
+// x / d rounded to nearest, from r = rcp_fix(d): bit for bit the IEEE quotient.
+// For a normal x whose quotient is normal, Z is the significands' quotient
+// within 0.53 units (of its 53 bits) and its exact remainder, modulo 2^64, says
+// whether it is one off; a quotient is never half-way between two.  A zero x
+// gives a zero; anything else divides.
+__device__ __forceinline__ double div_fix(double x, double d, unsigned long long r)
+{
+    unsigned const hx = static_cast<unsigned>(__double2hiint(x)), lx = static_cast<unsigned>(__double2loint(x));
+    unsigned const hd = static_cast<unsigned>(__double2hiint(d)), ld = static_cast<unsigned>(__double2loint(d));
+    unsigned const ex = (hx >> 20) & 0x7ffu;
+    unsigned const e = ex - ((hd >> 20) & 0x7ffu) + 1023u; // of a quotient of significands >= 1
+    unsigned long long const sign = static_cast<unsigned long long>((hx ^ hd) & 0x80000000u) << 32;
+    if (r == 0ull || ex - 1u > 2045u || e - 2u > 2043u)
+    {
+        bool const zero = r != 0ull && ((hx << 1) | lx) == 0u;
+        return zero ? __longlong_as_double(static_cast<long long>(sign)) : div_plain(x, d);
+    }
+    unsigned long long const ma = sig53(hx, lx), mb = sig53(hd, ld);
+    unsigned const low = ma >= mb ? 0u : 1u;
+    unsigned const sh = 9u - low;
+    unsigned long long Z = (mul_hi64(ma << 11, r) + (256ull >> low)) >> sh; // (ma / mb) 2^(52 + low)
+    long long const rem2 = 2 * static_cast<long long>((ma << (52u + low)) - Z * mb);
+    long long const b = static_cast<long long>(mb);
+    Z += static_cast<unsigned long long>((rem2 > b ? 1 : 0) - (rem2 < -b ? 1 : 0));
+    return __longlong_as_double(
+        static_cast<long long>((Z + (static_cast<unsigned long long>(e - 1u - low) << 52)) | sign));
+}
 
 // Whether x is a positive normal number.
 __device__ __forceinline__ bool pos_normal(unsigned hi) { return hi - 0x00100000u < 0x7fe00000u; }
@@ -161,7 +149,7 @@ __device__ __forceinline__ unsigned long long rsq_fixed(unsigned hi, unsigned lo
     float y;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint_as_float(__float_as_uint(sig_top(hi, lo)) + (odd << 23))));
     unsigned const Y = seed24(y);
-    X = ((static_cast<unsigned long long>((hi & 0xfffffu) | 0x100000u) << 32) | lo) << (10u + odd);
+    X = sig53(hi, lo) << (10u + odd);
     unsigned long long const Z = static_cast<unsigned long long>(Y) * Y << 16; // y^2 2^64
     long long const E = static_cast<long long>((1ull << 62) - mul_hi64(X, Z)); // e 2^62
     int const Es = static_cast<int>(E >> 12);                                   // e 2^50

@@ -18,6 +18,7 @@
  */
 
 #include "../../include/scg.h"
+#include "cluster.cuh"
 #include "common.hpp"
 #include "divide.cuh"
 
@@ -30,6 +31,8 @@
 
 namespace
 {
+
+using namespace scg::cluster;
 
 // Euler1DKernel::tiny (Euler1DCore.hpp:182) in FP64; it underflows in FP32,
 // where the same expressions use the smallest floor that keeps them finite.
@@ -304,79 +307,13 @@ __global__ void __launch_bounds__(128) k_half(E1DArgs a, int64_t start, int64_t 
 }
 
 // Small tubes: a whole march in one launch of one cluster of at most 16 blocks,
-// the tube in the threads' registers.  A half step of a small tube is latency
+// the tube in the threads' registers (cluster.cuh): thread k keeps the even
+// point 2k and the odd point 2k + 1.  A half step of a small tube is latency
 // and nothing else, most of it outside the arithmetic: the launch, the loads
 // from the L2 and the stores on their way back (201 points FP64: 6.4 us per
 // half step in a graph of launches, 8.4 launched singly, 5.7 with one cluster
-// marching the state in the L2).  Thread k keeps the even point 2k and the odd
-// point 2k + 1; a half step hands what one neighbour needs of each kernel along
-// by shuffles within a warp, and from warp to warp through a slot of shared
-// memory (of the neighbouring block's, where it lies there), ordered by the
-// cluster's hardware barrier once per half step.
-__device__ __forceinline__ void cluster_sync()
-{
-    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
-}
-
-// A slot of shared memory of another block of the cluster, and a store to it.
-__device__ __forceinline__ unsigned slot_of(void const * p, unsigned rank)
-{
-    unsigned out;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;"
-        : "=r"(out)
-        : "r"(static_cast<unsigned>(__cvta_generic_to_shared(p))), "r"(rank));
-    return out;
-}
-__device__ __forceinline__ void slot_put(unsigned at, double v)
-{
-    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(at), "d"(v) : "memory");
-}
-__device__ __forceinline__ void slot_put(unsigned at, float v)
-{
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(v) : "memory");
-}
-
-// Hands N values of each thread's v to the thread before it (Q = 1, into w) or
-// after it (Q = 0), over the whole cluster; slots: this half step's, one row of N
-// per warp of the block.  Every thread of the cluster calls it.  The threads
-// at the cluster's ends receive their own values or an unwritten slot's, which
-// they do not use.
-template <int N, int Q, typename R>
-__device__ __forceinline__ void hand_over(R const * v, R * w, R (*slots)[N])
-{
-    int const ln = static_cast<int>(threadIdx.x) & 31;
-    int const warp = static_cast<int>(threadIdx.x) >> 5;
-    int const last = static_cast<int>(blockDim.x >> 5) - 1;
-    int const from = Q == 1 ? 0 : 31; // the lane whose values leave the warp
-    if (ln == from)
-    {
-        int const to = Q == 1 ? warp - 1 : warp + 1;
-        unsigned const me = blockIdx.x;
-        if (to >= 0 && to <= last)
-        {
-            for (int i = 0; i < N; ++i)
-            {
-                slots[to][i] = v[i];
-            }
-        }
-        else if (Q == 1 ? me > 0 : me + 1 < gridDim.x)
-        {
-            unsigned const at = slot_of(slots[Q == 1 ? last : 0], Q == 1 ? me - 1 : me + 1);
-            for (int i = 0; i < N; ++i)
-            {
-                slot_put(at + static_cast<unsigned>(i * sizeof(R)), v[i]);
-            }
-        }
-    }
-    cluster_sync();
-    for (int i = 0; i < N; ++i)
-    {
-        R const x = Q == 1 ? __shfl_down_sync(0xffffffffu, v[i], 1) : __shfl_up_sync(0xffffffffu, v[i], 1);
-        w[i] = ln == 31 - from ? slots[warp][i] : x;
-    }
-}
-
+// marching the state in the L2, 3.9 here).
+//
 // A block's warps at most: one for each of the SM's four FP64 pipes (measured,
 // per half step: 3.9 us up to 2,001 points, 4.35 us at 4,001, against 6.0 to
 // 6.4 us in graph launches; a second warp per pipe: 7.6 against 6.2).
@@ -475,69 +412,6 @@ __global__ void __launch_bounds__(32 * TUBE_WARPS64) k_tube(E1DArgs a, int alpha
             a.so1[o * 3 + i] = xo[i];
         }
     }
-}
-
-// The largest cluster this GPU schedules for a kernel at `threads` threads a
-// block: 16 where it can (a non-portable size), else 8.  Asked once per kernel.
-template <auto KERNEL, int THREADS>
-int cluster_limit()
-{
-    static int const limit = [] {
-        cudaLaunchAttribute attr{};
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim = {16, 1, 1};
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(16);
-        cfg.blockDim = dim3(THREADS);
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        int n = 0;
-        if (cudaFuncSetAttribute(KERNEL, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-            cudaOccupancyMaxActiveClusters(&n, KERNEL, &cfg) == cudaSuccess && n > 0)
-        {
-            return 16;
-        }
-        (void)cudaGetLastError();
-        return 8;
-    }();
-    return limit;
-}
-
-// Launch a kernel as one cluster of `blocks` blocks.
-template <typename K, typename... A>
-void launch_cluster(K * kernel, int blocks, int threads, cudaStream_t stream, A... args)
-{
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim = {static_cast<unsigned>(blocks), 1, 1};
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(static_cast<unsigned>(blocks));
-    cfg.blockDim = dim3(static_cast<unsigned>(threads));
-    cfg.stream = stream;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    scg::cuda_check(cudaLaunchKernelEx(&cfg, kernel, args...), "cluster launch");
-}
-
-// Steps per launch of the cluster kernels (a launch of a few milliseconds).
-constexpr int64_t CLUSTER_STEPS = 1024;
-
-// Blocks and warps per block of a cluster that holds a tube of n points, one
-// point pair per thread: as many blocks as the limit allows before a second
-// warp per block, so that the warps have an SM each as long as there are SMs.
-// False where the tube does not fit.
-template <auto KERNEL, int MAX_WARPS>
-bool tube_shape(int64_t n, int & blocks, int & warps)
-{
-    int const limit = cluster_limit<KERNEL, 32 * MAX_WARPS>();
-    int64_t const w = ((n - 1) / 2 + 31) / 32;
-    blocks = 1;
-    while (blocks < limit && blocks < w)
-    {
-        blocks *= 2;
-    }
-    warps = static_cast<int>(std::min<int64_t>((w + blocks - 1) / blocks, MAX_WARPS + 1));
-    return warps <= MAX_WARPS;
 }
 
 // update_cfl alone.
@@ -815,7 +689,7 @@ public:
     bool cluster_march(int alpha, int64_t steps)
     {
         int blocks, warps;
-        if (!tube_shape<k_tube, TUBE_WARPS64>(n, blocks, warps))
+        if (!cluster_shape<k_tube, TUBE_WARPS64>((n - 1) / 2, blocks, warps))
         {
             return false;
         }
@@ -1764,7 +1638,7 @@ public:
     {
         int64_t const nout1 = nout_of(false), nout2 = nout_of(true);
         int blocks, warps;
-        if (nout1 <= 0 || !tube_shape<k_tube32<ALPHA>, TUBE_WARPS32>(n, blocks, warps))
+        if (nout1 <= 0 || !cluster_shape<k_tube32<ALPHA>, TUBE_WARPS32>((n - 1) / 2, blocks, warps))
         {
             return false;
         }

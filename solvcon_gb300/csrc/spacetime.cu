@@ -10,13 +10,15 @@
  * ic, so0 then so1 at its top solution element (index 3 + 2ic + p) from its
  * two bottom solution elements (2 + 2ic + p and 4 + 2ic + p), which are all on
  * the other parity: the half step has no dependency between elements.  One
- * thread per conservation element runs so0, the periodic ghost copy, the CFL
+ * lane per conservation element runs so0, the periodic ghost copy, the CFL
  * of the top element and so1 (the order of march_half1_alpha and
  * march_half2_alpha, core.hpp:1006-1025), so a full step is two launches;
- * march_alpha replays a captured CUDA graph of 32 steps.
+ * march_alpha replays a captured CUDA graph of 32 steps, or marches a small
+ * grid in one launch of one cluster.
  */
 
 #include "../../include/scg.h"
+#include "cluster.cuh"
 #include "common.hpp"
 #include "divide.cuh"
 
@@ -45,8 +47,10 @@ struct STArgs
 // half-width and the conservation-element width of
 // update_cfl/march_half_so0, core.hpp:962-980), so the march reads them
 // instead of recomputing them and its results stay bit-identical.  The four
-// divisors of a half step also get their reciprocals (rcp_tab), from which
-// div_rcp forms each quotient exactly as the division would.
+// divisors of a half step also get their reciprocals (rcp_fix, the bits kept in
+// a double), from which div_fix forms each quotient exactly as the division
+// would, on the integer pipe: the half step is bound by the FP64 pipe (53
+// instructions per element with its quotients there, 28 without).
 enum
 {
     G_DXNEG = 0, // x - xneg
@@ -63,6 +67,15 @@ enum
     G_CFLLIN,    // the linear solver's CFL number hdt / hdx (set with dt)
     G_COUNT
 };
+
+__device__ __forceinline__ double rcp_bits(double d)
+{
+    return __longlong_as_double(static_cast<long long>(scg::dev::rcp_fix(d)));
+}
+__device__ __forceinline__ double div_bits(double x, double d, double r)
+{
+    return scg::dev::div_fix(x, d, static_cast<unsigned long long>(__double_as_longlong(r)));
+}
 
 __global__ void k_st_geo(double const * x, int64_t xsize, double * geo)
 {
@@ -84,35 +97,43 @@ __global__ void k_st_geo(double const * x, int64_t xsize, double * geo)
     double const width = xp - xm;
     geo[G_HDX * xsize + xi] = hdx;
     geo[G_WIDTH * xsize + xi] = width;
-    geo[G_RDXNEG * xsize + xi] = scg::dev::rcp_tab(dn);
-    geo[G_RDXPOS * xsize + xi] = scg::dev::rcp_tab(dp);
-    geo[G_RHDX * xsize + xi] = scg::dev::rcp_tab(hdx);
-    geo[G_RWIDTH * xsize + xi] = scg::dev::rcp_tab(width);
+    geo[G_RDXNEG * xsize + xi] = rcp_bits(dn);
+    geo[G_RDXPOS * xsize + xi] = rcp_bits(dp);
+    geo[G_RHDX * xsize + xi] = rcp_bits(hdx);
+    geo[G_RWIDTH * xsize + xi] = rcp_bits(width);
 }
 
 __device__ __forceinline__ double gq(STArgs const & a, int k, int64_t xi) { return a.geo[k * a.xsize + xi]; }
 
-// The parts of solution element xi that the conservation elements on either
+// The grid quantities of solution element xi.
+struct SelmGrid
+{
+    double dxneg, dxpos, dmneg, dmpos, disp;
+
+    __device__ __forceinline__ SelmGrid(STArgs const & a, int64_t xi)
+        : dxneg(gq(a, G_DXNEG, xi))
+        , dxpos(gq(a, G_DXPOS, xi))
+        , dmneg(gq(a, G_DMNEG, xi))
+        , dmpos(gq(a, G_DMPOS, xi))
+        , disp(gq(a, G_DISP, xi))
+    {
+    }
+};
+
+// The parts of a solution element that the conservation elements on either
 // side of it use (LinearScalarSelm / InviscidBurgersSelm, xn, xp, tp, so0p):
 // ll = xp + tp (to the element on its right), ur = xn - tp (to the element on
-// its left), the value so0p at the next time level and dxneg, dxpos with
-// their reciprocals.
+// its left) and the value so0p at the next time level.
 template <int KIND>
 struct SelmParts
 {
-    double ll, ur, so0p, dxneg, dxpos, rdxneg, rdxpos;
+    double ll, ur, so0p;
 
-    __device__ SelmParts(STArgs const & a, int64_t xi)
+    __device__ __forceinline__ SelmParts(STArgs const & a, double u, double ux, SelmGrid const & x)
     {
-        double const u = a.so0[xi];
-        double const ux = a.so1[xi];
-        dxneg = gq(a, G_DXNEG, xi);
-        dxpos = gq(a, G_DXPOS, xi);
-        rdxneg = gq(a, G_RDXNEG, xi);
-        rdxpos = gq(a, G_RDXPOS, xi);
-        double const disp = gq(a, G_DISP, xi);
-        double const xn = dxneg * (u + gq(a, G_DMNEG, xi) * ux);
-        double const xp = dxpos * (u + gq(a, G_DMPOS, xi) * ux);
+        double const disp = x.disp;
+        double const xn = x.dxneg * (u + x.dmneg * ux);
+        double const xp = x.dxpos * (u + x.dmpos * ux);
         double tp;
         if constexpr (KIND == 0)
         {
@@ -146,17 +167,18 @@ __global__ void k_st_cfl_tab(double * geo, int64_t xsize, double hdt)
     int64_t const xi = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (xi < xsize)
     {
-        geo[G_CFLLIN * xsize + xi] = scg::dev::div_rcp(hdt, geo[G_HDX * xsize + xi], geo[G_RHDX * xsize + xi]);
+        geo[G_CFLLIN * xsize + xi] = div_bits(hdt, geo[G_HDX * xsize + xi], geo[G_RHDX * xsize + xi]);
     }
 }
 
+// update_cfl at point xi of value u.
 template <int KIND>
-__device__ __forceinline__ void cfl_at(STArgs const & a, int64_t xi)
+__device__ __forceinline__ double cfl_at(STArgs const & a, int64_t xi, double u)
 {
     if constexpr (KIND == 0)
-        a.cfl[xi] = gq(a, G_CFLLIN, xi);
+        return gq(a, G_CFLLIN, xi);
     else
-        a.cfl[xi] = scg::dev::div_rcp(fabs(a.so0[xi]) * a.hdt, gq(a, G_HDX, xi), gq(a, G_RHDX, xi));
+        return div_bits(fabs(u) * a.hdt, gq(a, G_HDX, xi), gq(a, G_RHDX, xi));
 }
 
 template <int ALPHA>
@@ -168,65 +190,44 @@ __device__ __forceinline__ double wgrad(double duxn, double duxp)
         fan *= fan;
         fap *= fap;
     }
-    return (fap * duxn + fan * duxp) / (fap + fan + DBL_MIN);
+    double const den = fap + fan + DBL_MIN;
+    return scg::dev::div_fix(fap * duxn + fan * duxp, den, scg::dev::rcp_fix(den));
 }
 
-constexpr int BST = 256;
+constexpr int WOUT = 31; // conservation elements per warp
 
 // One half step; STAGE bits: 1 so0, 2 cfl of the top element, 4 so1,
-// 8 periodic ghost copies (first half only).  Thread t of a block derives
-// the parts of the lower-left solution element of conservation element
-// ic = block * BST + t - odd; the element's lower-right solution element is
-// the next thread's (or, for the last thread, one extra derived by thread 0),
-// shared through shared memory, so each solution element is derived once.
+// 8 periodic ghost copies (first half only).  Lane l of warp w derives the
+// parts of the lower-left solution element of conservation element
+// ic = 31 w + l - odd; lanes 0 .. 30 form the element's top from those and the
+// next lane's, by shuffles: warps share nothing.
 template <int KIND, int ALPHA, int STAGE>
-__global__ void __launch_bounds__(BST) k_st_half(STArgs a, int odd)
+__global__ void __launch_bounds__(128) k_st_half(STArgs a, int odd)
 {
-    __shared__ double s_ur[BST + 1];
-    __shared__ double s_so0p[BST + 1];
-    __shared__ double s_dxneg[BST + 1];
-    __shared__ double s_rdxneg[BST + 1];
-    int64_t const ic0 = static_cast<int64_t>(blockIdx.x) * BST - (odd ? 1 : 0);
-    int64_t const ic = ic0 + threadIdx.x;
-    // Solution elements exist for ic <= ncelm (the last one is the
-    // lower-right element of conservation element ncelm - 1).
-    bool const selm = ic <= a.ncelm;
-    double ll = 0.0, so0pn = 0.0, dxposn = 1.0, rdxposn = 1.0;
-    if (selm)
-    {
-        SelmParts<KIND> const sn(a, 2 + 2 * ic + odd);
-        ll = sn.ll;
-        so0pn = sn.so0p;
-        dxposn = sn.dxpos;
-        rdxposn = sn.rdxpos;
-        s_ur[threadIdx.x] = sn.ur;
-        s_so0p[threadIdx.x] = sn.so0p;
-        s_dxneg[threadIdx.x] = sn.dxneg;
-        s_rdxneg[threadIdx.x] = sn.rdxneg;
-    }
-    if (threadIdx.x == 0)
-    {
-        int64_t const ich = ic0 + BST;
-        if (ich <= a.ncelm)
-        {
-            SelmParts<KIND> const sh(a, 2 + 2 * ich + odd);
-            s_ur[BST] = sh.ur;
-            s_so0p[BST] = sh.so0p;
-            s_dxneg[BST] = sh.dxneg;
-            s_rdxneg[BST] = sh.rdxneg;
-        }
-    }
-    __syncthreads();
-    if (ic >= a.ncelm)
+    int const lane = static_cast<int>(threadIdx.x) & 31;
+    int64_t const w = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / 32;
+    int64_t const first = w * WOUT - odd;
+    if (first >= a.ncelm)
     {
         return;
     }
-    int64_t const xt = 3 + 2 * ic + odd;
+    // Solution elements exist for ic <= ncelm (the last one is the lower-right
+    // element of conservation element ncelm - 1); lanes past it repeat it.
+    int64_t const ic = first + lane < a.ncelm ? first + lane : a.ncelm;
+    int64_t const xi = 2 + 2 * ic + odd;
+    SelmParts<KIND> const sn(a, a.so0[xi], a.so1[xi], SelmGrid(a, xi));
+    double const ur = __shfl_down_sync(0xffffffffu, sn.ur, 1);
+    double const so0p = __shfl_down_sync(0xffffffffu, sn.so0p, 1);
+    if (lane >= WOUT || ic >= a.ncelm)
+    {
+        return;
+    }
+    int64_t const xt = xi + 1;
     int64_t const last = 2 * a.ncelm + 1; // selm(ncelm - 1, odd plane)
     double utp;
     if (STAGE & 1)
     {
-        utp = scg::dev::div_rcp(ll + s_ur[threadIdx.x + 1], gq(a, G_WIDTH, xt), gq(a, G_RWIDTH, xt));
+        utp = div_bits(sn.ll + ur, gq(a, G_WIDTH, xt), gq(a, G_RWIDTH, xt));
         a.so0[xt] = utp;
         if (STAGE & 8)
         {
@@ -242,20 +243,19 @@ __global__ void __launch_bounds__(BST) k_st_half(STArgs a, int odd)
     }
     if (STAGE & 2)
     {
-        cfl_at<KIND>(a, xt);
+        a.cfl[xt] = cfl_at<KIND>(a, xt, utp);
         if (STAGE & 8)
         {
             if (xt == last)
-                cfl_at<KIND>(a, 1);
+                a.cfl[1] = cfl_at<KIND>(a, 1, utp);
             if (xt == 3)
-                cfl_at<KIND>(a, last + 2);
+                a.cfl[last + 2] = cfl_at<KIND>(a, last + 2, utp);
         }
     }
     if (STAGE & 4)
     {
-        double const duxn = scg::dev::div_rcp(utp - so0pn, dxposn, rdxposn);
-        double const duxp =
-            scg::dev::div_rcp(s_so0p[threadIdx.x + 1] - utp, s_dxneg[threadIdx.x + 1], s_rdxneg[threadIdx.x + 1]);
+        double const duxn = div_bits(utp - sn.so0p, gq(a, G_DXPOS, xi), gq(a, G_RDXPOS, xi));
+        double const duxp = div_bits(so0p - utp, gq(a, G_DXNEG, xi + 2), gq(a, G_RDXNEG, xi + 2));
         double const g = wgrad<ALPHA>(duxn, duxp);
         a.so1[xt] = g;
         if (STAGE & 8)
@@ -268,6 +268,107 @@ __global__ void __launch_bounds__(BST) k_st_half(STArgs a, int odd)
     }
 }
 
+// Small grids: a whole march in one launch of one cluster (cluster.cuh), thread
+// t keeping the even point 2t and the odd point 2t + 1.  The first half step
+// writes the odd points of threads 1 .. ncelm from the even points of t and
+// t + 1, and copies the end ones to the ghosts of threads ncelm + 1 and 0; the
+// second the even points of threads 1 .. ncelm + 1 from the odd points of t - 1
+// and t.  A point's CFL number is overwritten by the next step's, so it is
+// formed in the last step.
+constexpr int ST_WARPS = 8;
+
+template <int KIND, int ALPHA>
+__global__ void __launch_bounds__(32 * ST_WARPS) k_st_cluster(STArgs a, int64_t steps)
+{
+    using namespace scg::cluster;
+    __shared__ double slots[2][ST_WARPS][2];
+    __shared__ double ghost[2][2]; // so0 and so1 of the first and of the last odd point
+    int64_t const nt = a.ncelm + 2;
+    int64_t const t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    int64_t const k = t < nt ? t : nt - 1; // threads past the grid repeat its last pair, and write nothing
+    int64_t const e = 2 * k, o = 2 * k + 1;
+    int64_t const lo = k > 0 ? e - 1 : o;
+    double ue = a.so0[e], xe = a.so1[e], uo = a.so0[o], xo = a.so1[o];
+    SelmGrid const ge(a, e), go(a, o);
+    double const wide_o = gq(a, G_WIDTH, o), rwide_o = gq(a, G_RWIDTH, o);
+    double const wide_e = gq(a, G_WIDTH, e), rwide_e = gq(a, G_RWIDTH, e);
+    double const rpe = gq(a, G_RDXPOS, e);
+    double const dne = gq(a, G_DXNEG, e + 2), rne = gq(a, G_RDXNEG, e + 2); // of the next even point
+    double const dpo = gq(a, G_DXPOS, lo), rpo = gq(a, G_RDXPOS, lo);       // of the odd point before
+    double const rno = gq(a, G_RDXNEG, o);
+    bool const out1 = t >= 1 && t <= a.ncelm, out2 = t >= 1 && t < nt;
+    // The other end's ghost: thread ncelm's odd point is thread 0's, thread 1's
+    // is thread ncelm + 1's.
+    unsigned const to_lo = slot_of(ghost[0], 0);
+    unsigned const to_hi = slot_of(ghost[1], static_cast<unsigned>((nt - 1) / blockDim.x));
+    cluster_sync(); // every block runs before any stores to another's slots
+    for (int64_t s = 0; s < steps; ++s)
+    {
+        bool const end = s + 1 == steps;
+        {
+            SelmParts<KIND> const p(a, ue, xe, ge);
+            double const v[2] = {p.ur, p.so0p};
+            double w[2];
+            hand_over<2, 1>(v, w, slots[0]);
+            if (out1)
+            {
+                uo = div_bits(p.ll + w[0], wide_o, rwide_o);
+                xo = wgrad<ALPHA>(div_bits(uo - p.so0p, ge.dxpos, rpe), div_bits(w[1] - uo, dne, rne));
+                if (t == a.ncelm)
+                {
+                    slot_put(to_lo, uo);
+                    slot_put(to_lo + 8u, xo);
+                }
+                if (t == 1)
+                {
+                    slot_put(to_hi, uo);
+                    slot_put(to_hi + 8u, xo);
+                }
+            }
+            cluster_sync();
+            if (t == 0)
+            {
+                uo = ghost[0][0];
+                xo = ghost[0][1];
+            }
+            else if (t == nt - 1)
+            {
+                uo = ghost[1][0];
+                xo = ghost[1][1];
+            }
+            if (end && t < nt)
+            {
+                a.cfl[o] = cfl_at<KIND>(a, o, uo);
+            }
+        }
+        {
+            SelmParts<KIND> const p(a, uo, xo, go);
+            double const v[2] = {p.ll, p.so0p};
+            double w[2];
+            hand_over<2, 0>(v, w, slots[1]);
+            if (out2)
+            {
+                ue = div_bits(w[0] + p.ur, wide_e, rwide_e);
+                xe = wgrad<ALPHA>(div_bits(ue - w[1], dpo, rpo), div_bits(p.so0p - ue, go.dxneg, rno));
+                if (end)
+                {
+                    a.cfl[e] = cfl_at<KIND>(a, e, ue);
+                }
+            }
+        }
+    }
+    if (t < nt)
+    {
+        if (t > 0)
+        {
+            a.so0[e] = ue;
+            a.so1[e] = xe;
+        }
+        a.so0[o] = uo;
+        a.so1[o] = xo;
+    }
+}
+
 template <int KIND>
 __global__ void k_st_cfl(STArgs a, int odd)
 {
@@ -275,7 +376,8 @@ __global__ void k_st_cfl(STArgs a, int odd)
     int64_t const ic = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x - (odd ? 1 : 0);
     if (ic <= a.ncelm)
     {
-        cfl_at<KIND>(a, 2 + 2 * ic + odd);
+        int64_t const xi = 2 + 2 * ic + odd;
+        a.cfl[xi] = cfl_at<KIND>(a, xi, a.so0[xi]);
     }
 }
 
@@ -382,20 +484,25 @@ public:
     void half_t(int alpha, int odd)
     {
         int64_t const n = ncelm + (odd ? 1 : 0);
-        unsigned const grid = static_cast<unsigned>((n + BST - 1) / BST);
+        // Blocks of one warp while they all are resident at once, as the 1D
+        // Euler core's, beyond that blocks of four.
+        int64_t const warps = (n + WOUT - 1) / WOUT;
+        int const wpb = warps <= 152 * 32 ? 1 : 4;
+        unsigned const grid = static_cast<unsigned>((warps + wpb - 1) / wpb);
+        int const threads = 32 * wpb;
         if (kind == 0)
         {
             if (alpha == 1)
-                k_st_half<0, 1, STAGE><<<grid, BST, 0, stream>>>(args(), odd);
+                k_st_half<0, 1, STAGE><<<grid, threads, 0, stream>>>(args(), odd);
             else
-                k_st_half<0, 2, STAGE><<<grid, BST, 0, stream>>>(args(), odd);
+                k_st_half<0, 2, STAGE><<<grid, threads, 0, stream>>>(args(), odd);
         }
         else
         {
             if (alpha == 1)
-                k_st_half<1, 1, STAGE><<<grid, BST, 0, stream>>>(args(), odd);
+                k_st_half<1, 1, STAGE><<<grid, threads, 0, stream>>>(args(), odd);
             else
-                k_st_half<1, 2, STAGE><<<grid, BST, 0, stream>>>(args(), odd);
+                k_st_half<1, 2, STAGE><<<grid, threads, 0, stream>>>(args(), odd);
         }
         scg::launched(stream, "spacetime_half");
     }
@@ -446,6 +553,11 @@ public:
         {
             throw std::invalid_argument("spacetime: alpha must be 1 or 2");
         }
+        if (kind == 0 ? (alpha == 1 ? cluster_march<0, 1>(steps) : cluster_march<0, 2>(steps))
+                      : (alpha == 1 ? cluster_march<1, 1>(steps) : cluster_march<1, 2>(steps)))
+        {
+            return;
+        }
         int64_t const chunks = steps / GRAPH_STEPS;
         if (chunks > 0)
         {
@@ -463,6 +575,25 @@ public:
         {
             step(alpha);
         }
+    }
+
+    // A small grid's steps in launches of one cluster.
+    template <int KIND, int ALPHA>
+    bool cluster_march(int64_t steps)
+    {
+        using namespace scg::cluster;
+        int blocks, warps;
+        if (!cluster_shape<k_st_cluster<KIND, ALPHA>, ST_WARPS>(ncelm + 2, blocks, warps))
+        {
+            return false;
+        }
+        for (int64_t s = 0; s < steps; s += CLUSTER_STEPS)
+        {
+            launch_cluster(k_st_cluster<KIND, ALPHA>, blocks, 32 * warps, stream, args(),
+                           std::min(CLUSTER_STEPS, steps - s));
+            scg::launched(stream, "spacetime_cluster");
+        }
+        return true;
     }
 
     void capture(int alpha)
@@ -526,7 +657,7 @@ private:
     int graph_alpha = 0;
 };
 
-// One quotient per thread, by div_rcp from the tabulated reciprocal and by
+// One quotient per thread, by div_fix from the tabulated reciprocal and by
 // the division itself, and the FP64 march's reciprocal of d.
 __global__ void k_divide_check(double const * x, double const * d, double * q, double * qdiv, double * rcp,
                                int64_t n)
@@ -534,7 +665,7 @@ __global__ void k_divide_check(double const * x, double const * d, double * q, d
     int64_t const i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i < n)
     {
-        q[i] = scg::dev::div_rcp(x[i], d[i], scg::dev::rcp_tab(d[i]));
+        q[i] = scg::dev::div_fix(x[i], d[i], scg::dev::rcp_fix(d[i]));
         qdiv[i] = x[i] / d[i];
         rcp[i] = scg::dev::recip(d[i]);
     }

@@ -1,6 +1,7 @@
-"""Whole marches of 1D tubes in one launch (the tube in the registers of a
-cluster of blocks) against the same steps taken one method at a time, at the
-sizes where threads, warps and blocks of the cluster begin and end."""
+"""Whole marches of 1D tubes and spacetime grids in one launch (the points in
+the registers of a cluster of blocks) against the same steps taken one method
+at a time, at the sizes where threads, warps and blocks of the cluster begin
+and end."""
 
 import numpy as np
 import pytest
@@ -47,4 +48,36 @@ def test_march_equals_its_half_steps(precision, sizes, alpha):
             np.testing.assert_array_equal(getattr(got, name)[...],
                                           getattr(want, name)[...],
                                           "%s n=%d" % (name, n))
+        assert np.isfinite(got.so0[...]).all()
+
+
+# Point pairs ncelm + 2: one element, a warp's end, two warps, 16 blocks, their
+# second and eighth warp, the last grid that fits (4,094) and the first that
+# does not.
+@pytest.mark.parametrize("solver", ["LinearScalarSolver",
+                                    "InviscidBurgersSolver"])
+@pytest.mark.parametrize("alpha", [1, 2])
+def test_spacetime_march_equals_its_half_steps(solver, alpha):
+    """march_alpha(3) leaves bit for bit what the half-step methods leave."""
+    import solvcon_gb300.spacetime as st
+    for n in (1, 2, 29, 30, 31, 62, 63, 510, 511, 4094, 4095):
+        rng = np.random.default_rng(n)
+        grid = st.Grid(np.cumsum(rng.uniform(0.5, 1.5, n + 1)))
+        cores = []
+        for _ in range(2):
+            core = getattr(st, solver)(grid, 0.2)
+            x = grid.xcoord
+            core.so0[...] = np.sin(x)[:, None]
+            core.so1[...] = np.cos(x)[:, None]
+            core.setup_march()
+            cores.append(core)
+        got, want = cores
+        getattr(got, "march_alpha%d" % alpha)(3)
+        for _ in range(3):
+            getattr(want, "march_half1_alpha%d" % alpha)()
+            getattr(want, "march_half2_alpha%d" % alpha)()
+        for name in ("so0", "so1", "cfl"):
+            np.testing.assert_array_equal(getattr(got, name)[...],
+                                          getattr(want, name)[...],
+                                          "%s ncelm=%d" % (name, n))
         assert np.isfinite(got.so0[...]).all()
