@@ -52,8 +52,7 @@ __device__ __forceinline__ void fused_batch_tiles(MarchArgs<R, G> const * descs,
             words[threadIdx.x] = reinterpret_cast<int const *>(descs + tl.x)[threadIdx.x];
         }
         __syncthreads();
-        scg::dev::fused_thread<ND, R, G, CT1, scg::dev::carry_shared<ND>() ? B : 0>(
-            a, static_cast<int64_t>(tl.y) + threadIdx.x);
+        scg::dev::fused_thread<ND, R, G, CT1, B>(a, static_cast<int64_t>(tl.y) + threadIdx.x, a.ncell + a.ngst);
     }
 }
 
@@ -119,6 +118,7 @@ class Batch : public BatchBase
 {
 public:
     using Args = MarchArgs<R, G>;
+    static constexpr int SMEM = scg::dev::stage_bytes<R, G, CT1, B>();
 
     Batch(std::vector<scg::EulerCoreBase *> cores_in, bool persistent)
         : cores(std::move(cores_in)), persistent(persistent)
@@ -130,7 +130,8 @@ public:
         int dev = 0, nsm = 0, occ = 0;
         scg::cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
         scg::cuda_check(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev), "attr");
-        scg::cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch_kernel<ND, R, G, B, CT1>(), B, 0),
+        scg::allow_shared<batch_kernel<ND, R, G, B, CT1>(), SMEM>();
+        scg::cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch_kernel<ND, R, G, B, CT1>(), B, SMEM),
                         "occupancy");
         resident = static_cast<int64_t>(nsm) * std::max(occ, 1);
         layout();
@@ -328,7 +329,7 @@ public:
     {
         for (int p = 0; p < 2; ++p)
         {
-            batch_kernel<ND, R, G, B, CT1>()<<<static_cast<unsigned>(grid), B, 0, stream>>>(
+            batch_kernel<ND, R, G, B, CT1>()<<<static_cast<unsigned>(grid), B, SMEM, stream>>>(
                 descs[p].ptr, tiles.ptr, static_cast<int>(ntiles));
             scg::launched(stream, "fused_batch");
         }

@@ -110,7 +110,11 @@ __device__ __forceinline__ void soln_any(MarchArgs<R, G> const & a, int64_t icl,
     if constexpr (sizeof(R) == 8)
         soln64<CT, false>(a, icl, so0n);
     else
-        soln_cell<CT, R, G>(a, icl, so0n);
+    {
+        CellHead<CellT<CT>::ND, CellT<CT>::NFC> const head(a, icl);
+        DirectRecs<CellT<CT>::ND> recs{a.cur, head.nbr};
+        soln_cell<CT>(a, geo_view(a, icl), head.nbr, recs, so0n);
+    }
 }
 template <int CT, typename R, typename G>
 __device__ __forceinline__ void dsoln_any(MarchArgs<R, G> const & a, int64_t icl, R const * so0n, R cflc, R * so1n)
@@ -118,7 +122,7 @@ __device__ __forceinline__ void dsoln_any(MarchArgs<R, G> const & a, int64_t icl
     if constexpr (sizeof(R) == 8)
         dsoln64<CT>(a, icl, so0n, cflc, so1n);
     else
-        dsoln_cell<CT, R, G>(a, icl, so0n, cflc, so1n);
+        dsoln_cell<CT>(a, geo_view(a, icl), icl, so0n, cflc, so1n);
 }
 
 template <int ND, typename R, typename G>
@@ -176,7 +180,7 @@ __global__ void k_cfl(MarchArgs<R, G> a)
     if constexpr (sizeof(R) == 8)
         cfl64<ND>(a, icl, row, s, rinv);
     else
-        cfl_cell<ND, R, G>(a, icl, row, s, rinv);
+        cfl_cell<ND>(a, geo_view(a, icl), row, s, rinv);
     out[NEQ - 1] = s[NEQ - 1];
 }
 
@@ -889,12 +893,11 @@ public:
         d_gint.alloc(std::max<int64_t>(ngstcell, 1));
 
         // Geometry: prepare_ce, then the compact march tables.
-        d_fgeo.alloc(static_cast<size_t>(std::max(nslot, 1)) * KF * std::max<int64_t>(ncell, 1));
-        d_cgeo.alloc(static_cast<size_t>(Dim<ND>::KC) * std::max<int64_t>(ncell, 1));
+        npl = Dim<ND>::KC + static_cast<int64_t>(std::max(nslot, 1)) * KF;
+        d_geo.alloc(static_cast<size_t>((std::max<int64_t>(ncell, 1) + GEO_TILE - 1) / GEO_TILE * GEO_TILE * npl));
         // Slots past a cell's own faces are never written; zero them so the
-        // whole tables hold defined values (the FP32 form checks them all).
-        cuda_check(cudaMemsetAsync(d_fgeo.ptr, 0, d_fgeo.bytes(), stream), "memset");
-        cuda_check(cudaMemsetAsync(d_cgeo.ptr, 0, d_cgeo.bytes(), stream), "memset");
+        // whole tables, the last tile included, hold defined values.
+        cuda_check(cudaMemsetAsync(d_geo.ptr, 0, d_geo.bytes(), stream), "memset");
         d_nbr.alloc(static_cast<size_t>(std::max(nslot, 1)) * std::max<int64_t>(ncell, 1));
         d_ctype.alloc(std::max<int64_t>(ncell, 1));
         prepare_ce(true);
@@ -942,7 +945,7 @@ public:
         size_t b = 0;
         for (auto const & r : rec)
             b += r.bytes();
-        b += d_fgeo.bytes() + d_cgeo.bytes() + d_nbr.bytes() + d_ctype.bytes();
+        b += d_geo.bytes() + d_nbr.bytes() + d_ctype.bytes();
         b += d_gamma.bytes() + d_cflo.bytes() + d_cflc.bytes() + d_comp.bytes();
         b += d_ndcrd.bytes() + d_fccnd.bytes() + d_clcnd.bytes() + d_fcnds.bytes() + d_fccls.bytes() +
              d_clfcs.bytes() + d_cltpn.bytes() + d_clvol.bytes();
@@ -1092,8 +1095,8 @@ public:
             cuda_check(cudaMemsetAsync(bad.ptr, 0, sizeof(unsigned long long), stream), "memset");
         }
         k_compact<ND, G><<<grid_for(ncell), BLOCK, 0, stream>>>(mv, ce[0].ptr, ce[1].ptr, ce[2].ptr, ce[3].ptr,
-                                                                0.5 * time_increment, std::max(nslot, 1),
-                                                                d_fgeo.ptr, d_cgeo.ptr, d_nbr.ptr, d_ctype.ptr,
+                                                                0.5 * time_increment, std::max(nslot, 1), npl,
+                                                                d_geo.ptr, d_nbr.ptr, d_ctype.ptr,
                                                                 bad.ptr);
         launched(stream, "compact");
         if constexpr (ROUNDS)
@@ -1195,8 +1198,8 @@ public:
         a.gamma = d_gamma.ptr;
         a.cflo = d_cflo.ptr;
         a.cflc = d_cflc.ptr;
-        a.fgeo = d_fgeo.ptr;
-        a.cgeo = d_cgeo.ptr;
+        a.geo = d_geo.ptr;
+        a.npl = npl;
         a.nbr = d_nbr.ptr;
         a.ctype = d_ctype.ptr;
         a.gkind = d_gkind.ptr;
@@ -1548,7 +1551,9 @@ public:
             constexpr int MINB = min_blocks<ND, R, SIMPLEX, BLOCK, G>();
             if constexpr (MINB > 0)
             {
-                k_fused_mb<ND, R, G, SIMPLEX, MINB><<<g, BLOCK, 0, stream>>>(args(), t0, t1);
+                constexpr int SMEM = stage_bytes<R, G, SIMPLEX, BLOCK>();
+                allow_shared<k_fused_mb<ND, R, G, SIMPLEX, MINB>, SMEM>();
+                k_fused_mb<ND, R, G, SIMPLEX, MINB><<<g, BLOCK, SMEM, stream>>>(args(), t0, t1);
             }
             else
             {
@@ -2008,6 +2013,7 @@ private:
 
     int64_t nrow = 0;
     int nslot = 0;
+    int64_t npl = 0;
     cudaStream_t own_stream = nullptr;
     // march_from_host: the upload stream, an event per upload chunk (and one
     // for the start), and the chunk plan.
@@ -2029,7 +2035,7 @@ private:
     DevBuf<double> d_ndcrd, d_fccnd, d_clcnd, d_clvol;
     DevBuf<int32_t> d_fcnds, d_fccls, d_clfcs, d_cltpn;
     DevBuf<double> ce[4]; // cevol, cecnd, sfcnd, sfnml (reference layout)
-    DevBuf<G> d_fgeo, d_cgeo;
+    DevBuf<G> d_geo;
     DevBuf<int32_t> d_nbr;
     DevBuf<int8_t> d_ctype;
     DevBuf<R> rec[2];

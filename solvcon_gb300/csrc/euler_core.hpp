@@ -85,6 +85,16 @@ enum Precision : int
     PREC_FP32 = 2,         // the same with displacements formed in FP32 from fewer stored values (faster variant)
 };
 
+// Let a kernel use `bytes` of dynamic shared memory (asked for once per kernel).
+template <auto KERNEL, int BYTES>
+inline void allow_shared()
+{
+    static cudaError_t const rc = BYTES <= 0 ? cudaSuccess
+                                             : cudaFuncSetAttribute(reinterpret_cast<void const *>(KERNEL),
+                                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, BYTES);
+    cuda_check(rc, "cudaFuncSetAttribute");
+}
+
 struct EulerBoundary
 {
     int kind;

@@ -162,20 +162,6 @@ __device__ __forceinline__ bool geo_r_takes(double v)
     return e <= 1150u;
 }
 
-// A stored geometry value in the march's precision R.
-template <typename R, typename G>
-__device__ __forceinline__ R geo_val(G v)
-{
-    if constexpr (std::is_same<G, Rounded>::value)
-    {
-        return v.v;
-    }
-    else
-    {
-        return R(v);
-    }
-}
-
 // The FP32 march's reciprocals and quotients.  2D: the approximate quotient
 // (div.approx.f32, one instruction and within 2 ulp for divisors of magnitude
 // in [2^-126, 2^126]; a zero divisor gives a signed infinity, or NaN over
@@ -428,8 +414,7 @@ struct MarchArgs
     R const * gamma;      // [nrow]
     R * cflo;             // [nrow]
     R * cflc;             // [nrow]
-    G const * fgeo;       // [NSLOT][KF][ncell]
-    G const * cgeo;       // [KC][ncell]
+    G const * geo;        // [tile of GEO_TILE cells][npl][GEO_TILE], see GeoView
     int32_t const * nbr;  // [NSLOT][ncell] neighbour row
     int8_t const * ctype; // [ncell]
     int8_t const * gkind; // [ngst] BC kind of the ghost row, -1 if none
@@ -445,6 +430,7 @@ struct MarchArgs
     R * comp;
     int64_t ncell;
     int64_t ngst;
+    int64_t npl; // geometry values per cell, KC + slots * KF
     R dt, hdt, qdt;
     R sigma0, taumin, tauscale;
 };
@@ -455,24 +441,50 @@ __device__ __forceinline__ T ldg(T const * p)
     return __ldg(p);
 }
 
-// A geometry table value, loaded once per cell-substep and streamed.
-template <int ND, typename R, typename G>
-__device__ __forceinline__ R geo_ld(G const * p)
+// One cell's geometry values.  The tables are kept in tiles of 32 consecutive
+// cells, tile-major: value (plane) k of cell i lies at
+//   ((i / 32) npl + k) 32 + i % 32,
+// so a warp's loads of one plane are one contiguous piece, and all the values
+// of a warp's cells are one too (6 KB for the FP32 form's triangles), which the
+// FP32 march copies to shared memory at once (SHARED: p points there).
+constexpr int GEO_TILE = 32;
+
+template <typename G, bool SHARED = false>
+struct GeoView
 {
-    if constexpr (std::is_same<G, Rounded>::value)
+    G const * p; // the cell's value 0
+
+    __device__ __forceinline__ auto at(int k) const
     {
-        return ldg(&p->v);
+        if constexpr (std::is_same<G, Rounded>::value)
+        {
+            float const * const q = &p[k * GEO_TILE].v;
+            return SHARED ? *q : ldg(q);
+        }
+        else
+        {
+            G const * const q = p + k * GEO_TILE;
+            return SHARED ? *q : ldg(q);
+        }
     }
-    else
-    {
-        return geo_val<R>(ldg(p));
-    }
+};
+
+template <typename R, typename G>
+__device__ __forceinline__ GeoView<G> geo_view(MarchArgs<R, G> const & a, int64_t icl)
+{
+    return GeoView<G>{a.geo + (icl / GEO_TILE) * a.npl * GEO_TILE + icl % GEO_TILE};
 }
 
-template <int ND, typename R, typename G>
-__device__ __forceinline__ R fg(MarchArgs<R, G> const & a, int f, int k, int64_t icl)
+// Value k of face f, and per-cell value k.
+template <int ND, typename G, bool SH>
+__device__ __forceinline__ auto fg(GeoView<G, SH> const & gv, int f, int k)
 {
-    return geo_ld<ND, R>(a.fgeo + (static_cast<int64_t>(f) * Geo<ND, G>::KF + k) * a.ncell + icl);
+    return gv.at(Dim<ND>::KC + f * Geo<ND, G>::KF + k);
+}
+template <int ND, typename G, bool SH>
+__device__ __forceinline__ auto cg(GeoView<G, SH> const & gv, int k)
+{
+    return gv.at(k);
 }
 
 } // namespace dev

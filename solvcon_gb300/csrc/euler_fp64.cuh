@@ -257,6 +257,7 @@ __device__ __forceinline__ void soln64(MarchArgs<double, double> const & a, int6
     using D = Geo<ND, double>;
     using RC = Rec<ND, double>;
     using F = FluxTerms<ND>;
+    GeoView<double> const gv = geo_view(a, icl);
     double acc[NEQ];
 #pragma unroll
     for (int f = 0; f < NFC; ++f)
@@ -281,7 +282,7 @@ __device__ __forceinline__ void soln64(MarchArgs<double, double> const & a, int6
             c = ct;
         }
         double const * const g = rec + 2 * NEQ;
-        double const bvol = fg<ND>(a, f, D::K_BVOL, icl);
+        double const bvol = fg<ND>(gv, f, D::K_BVOL);
 #pragma unroll
         for (int i = 0; i < NEQ; ++i)
         {
@@ -290,8 +291,8 @@ __device__ __forceinline__ void soln64(MarchArgs<double, double> const & a, int6
 #pragma unroll
         for (int d = 0; d < ND; ++d)
         {
-            double const vb = fg<ND>(a, f, D::K_DB + d, icl);
-            double const nh = fg<ND>(a, f, D::K_NH + d, icl);
+            double const vb = fg<ND>(gv, f, D::K_DB + d);
+            double const nh = fg<ND>(gv, f, D::K_NH + d);
             acc[0] = fm(-c[F::A0 + d], nh, fm(vb, g[d], acc[0]));
             acc[NEQ - 1] = fm(-c[F::AE + d], nh, fm(vb, g[(NEQ - 1) * ND + d], acc[NEQ - 1]));
 #pragma unroll
@@ -306,7 +307,7 @@ __device__ __forceinline__ void soln64(MarchArgs<double, double> const & a, int6
 #pragma unroll
             for (int d = 0; d < ND; ++d)
             {
-                double const m = fg<ND>(a, f, D::K_MH + e * ND + d, icl);
+                double const m = fg<ND>(gv, f, D::K_MH + e * ND + d);
                 acc[0] = fm(-g[(1 + d) * ND + e], m, acc[0]);
                 acc[NEQ - 1] = fm(-c[F::BE + d * ND + e], m, acc[NEQ - 1]);
 #pragma unroll
@@ -317,7 +318,7 @@ __device__ __forceinline__ void soln64(MarchArgs<double, double> const & a, int6
             }
         }
     }
-    double const ivol = __ldg(a.cgeo + icl);
+    double const ivol = cg<ND>(gv, 0);
 #pragma unroll
     for (int i = 0; i < NEQ; ++i)
     {
@@ -350,7 +351,7 @@ __device__ __forceinline__ double cfl64(MarchArgs<double, double> const & a, int
     bool const neg = hp >= 0x80000000u;
     double pra = neg ? (hp >= 0xfff00000u ? __longlong_as_double(0x7ff8000000000000ll) : 0.0) : pr;
     double const wspd = fm(sqr_t(momsq), ri, sqr_t(mu(mu(ga, pra), ri)));
-    double const cflo = mu(wspd, __ldg(a.cgeo + a.ncell + icl));
+    double const cflo = mu(wspd, cg<ND>(geo_view(a, icl), 1));
     // pra / (pra + TINY) is exactly 1 whenever TINY does not change pra, as it
     // does not above 1e-43: the division is taken only below.
     double f = 1.0;
@@ -420,6 +421,7 @@ __device__ __forceinline__ void dsoln64_simplex(MarchArgs<double, double> const 
     using RC = Rec<ND, double>;
     double const acfl = fabs(cflc);
     double const tau = fm(acfl, a.tauscale, a.taumin);
+    GeoView<double> const gv = geo_view(a, icl);
     // Solution deltas at the evaluation points: of the first ND faces, and
     // their sum over all.
     double uf[ND][NEQ], us[NEQ];
@@ -434,11 +436,11 @@ __device__ __forceinline__ void dsoln64_simplex(MarchArgs<double, double> const 
 #pragma unroll
         for (int d = 0; d < ND; ++d)
         {
-            double const qf = fg<ND>(a, f, D::K_Q + d, icl);
-            jd[d] = fm(tau, qf, fg<ND>(a, f, D::K_R + d, icl));
+            double const qf = fg<ND>(gv, f, D::K_Q + d);
+            jd[d] = fm(tau, qf, fg<ND>(gv, f, D::K_R + d));
             if (f < ND)
             {
-                x[f][d] = fm(tau, qf, fg<ND>(a, f, D::K_P + d, icl));
+                x[f][d] = fm(tau, qf, fg<ND>(gv, f, D::K_P + d));
             }
         }
 #pragma unroll
@@ -619,6 +621,7 @@ __device__ __forceinline__ void dsoln64_general(MarchArgs<double, double> const 
     using RC = Rec<ND, double>;
     double const acfl = fabs(cflc);
     double const tau = fm(acfl, a.tauscale, a.taumin);
+    GeoView<double> const gv = geo_view(a, icl);
     double x[NFC][ND];
 #pragma unroll
     for (int f = 0; f < NFC; ++f)
@@ -626,7 +629,7 @@ __device__ __forceinline__ void dsoln64_general(MarchArgs<double, double> const 
 #pragma unroll
         for (int d = 0; d < ND; ++d)
         {
-            x[f][d] = fm(tau, fg<ND>(a, f, D::K_Q + d, icl), fg<ND>(a, f, D::K_P + d, icl));
+            x[f][d] = fm(tau, fg<ND>(gv, f, D::K_Q + d), fg<ND>(gv, f, D::K_P + d));
         }
     }
     FacePairs<CT> pr;
@@ -692,7 +695,7 @@ __device__ __forceinline__ void dsoln64_general(MarchArgs<double, double> const 
 #pragma unroll
         for (int d = 0; d < ND; ++d)
         {
-            jd[d] = sb(fm(tau, fg<ND>(a, f, D::K_Q + d, icl), fg<ND>(a, f, D::K_R + d, icl)), delta[d]);
+            jd[d] = sb(fm(tau, fg<ND>(gv, f, D::K_Q + d), fg<ND>(gv, f, D::K_R + d)), delta[d]);
         }
 #pragma unroll
         for (int i = 0; i < NEQ; ++i)

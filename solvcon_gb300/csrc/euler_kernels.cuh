@@ -89,32 +89,11 @@ __host__ __device__ constexpr bool carries()
 }
 
 // Resident blocks of `block` threads to ask of the compiler for a fused
-// kernel whose cells carry (0: keep the one-argument launch bound).  The
-// carried sums hold 24 (2D) / 40 (3D) more floats; measured at 128 threads,
-// 2M triangles: 0.1727 ms per launch without carrying (64 registers), with
-// carrying 0.1771 ms at 5 blocks (96 registers), 0.1662 at 6, 0.1555 at 7
-// (72 registers, 28 bytes spilled), 0.1557 at 8 (64 registers, 60 bytes
-// spilled); 24.6M tetrahedra: 5.92 ms without, 4.75 ms at 5 blocks (96
-// registers, 80 bytes spilled), 4.66 ms at 4 (128 registers).  With the
-// FP32 delta form (u0, d0 below) 7 blocks stay best in 2D (0.1628 ms; 6:
-// 0.1688, 8: 0.1683) and 4 in 3D (4.80 ms).  The budget per thread (72 /
-// 128 registers) is kept for other block sizes.  The FP32 form (G = Rounded,
-// 15 / 25 stored values per face instead of 11 / 19) has its own budget: 2D,
-// 2M triangles, 0.2016 ms per launch at 96 registers against 0.2573 at 80,
-// 0.2750 at 72 and 0.3126 at 64 (spills); 3D, 1.3M tetrahedra, 0.299 ms at 128
-// and at 96, 0.334 at 80, 0.345 at 168.
-#ifndef SCG_CARRY_REGS_2D
-#define SCG_CARRY_REGS_2D 72
-#endif
-#ifndef SCG_CARRY_REGS_2D_ROUNDED
-#define SCG_CARRY_REGS_2D_ROUNDED 96
-#endif
-#ifndef SCG_CARRY_REGS_3D
-#define SCG_CARRY_REGS_3D 128
-#endif
-#ifndef SCG_CARRY_REGS_3D_ROUNDED
-#define SCG_CARRY_REGS_3D_ROUNDED 128
-#endif
+// kernel whose cells carry (0: keep the one-argument launch bound), from the
+// registers per thread that were fastest with what the kernel stages (Stage).
+// FP32 form, 2M triangles: 156 us per launch at 112 registers, 233 at 96 and
+// 252 at 80 (spills); fp32-geom32: 136 at 80, 138 at 96, 149 at 128.
+// Tetrahedra: 245 us per 1.3M at 128, 246 at 96.
 template <int ND, typename R, int CT, int BLOCK, typename G = R>
 __host__ __device__ constexpr int min_blocks()
 {
@@ -124,8 +103,7 @@ __host__ __device__ constexpr int min_blocks()
     }
     else
     {
-        constexpr int regs = ND == 3 ? (Geo<ND, G>::MID ? SCG_CARRY_REGS_3D : SCG_CARRY_REGS_3D_ROUNDED)
-                                     : (Geo<ND, G>::MID ? SCG_CARRY_REGS_2D : SCG_CARRY_REGS_2D_ROUNDED);
+        constexpr int regs = ND == 3 ? 128 : (Geo<ND, G>::MID ? 80 : 112);
         return 65536 / (BLOCK * regs);
     }
 }
@@ -174,8 +152,8 @@ struct CarrySh
 };
 
 // Face means of mid and dB (FP32 geometry; zero with FP64 geometry).
-template <int CT, typename R, typename G>
-__device__ __forceinline__ void face_means(MarchArgs<R, G> const & a, int64_t icl, R * mm, R * mb)
+template <int CT, typename R, typename G, bool SH>
+__device__ __forceinline__ void face_means(GeoView<G, SH> const & gv, R * mm, R * mb)
 {
     constexpr int ND = CellT<CT>::ND;
     constexpr int NFC = CellT<CT>::NFC;
@@ -194,8 +172,8 @@ __device__ __forceinline__ void face_means(MarchArgs<R, G> const & a, int64_t ic
 #pragma unroll
             for (int d = 0; d < ND; ++d)
             {
-                mm[d] += fg<ND>(a, f, D::K_MID + d, icl);
-                mb[d] += fg<ND>(a, f, D::K_DB + d, icl);
+                mm[d] += fg<ND>(gv, f, D::K_MID + d);
+                mb[d] += fg<ND>(gv, f, D::K_DB + d);
             }
         }
         R const inv = R(1) / R(NFC);
@@ -216,9 +194,11 @@ __device__ __forceinline__ void face_means(MarchArgs<R, G> const & a, int64_t ic
 // values enter as differences from u0 and d0 receives so0n - u0: the absolute
 // rounding then scales with the change, not with the state (the gradients
 // calc_dsoln forms from these differences are O(h) of the state).
-template <int CT, typename R, typename G, typename CA = Carry<CellT<CT>::ND, CellT<CT>::NFC, R>>
-__device__ __forceinline__ void soln_cell(MarchArgs<R, G> const & a, int64_t icl, R * so0n, CA * carry = nullptr,
-                                          R const * u0 = nullptr, R * d0 = nullptr)
+// recs.load(f, rec) gives the record of face f's neighbour, nbr[f] its row.
+template <int CT, typename R, typename G, bool SH, typename RS, typename CA = Carry<CellT<CT>::ND, CellT<CT>::NFC, R>>
+__device__ __forceinline__ void soln_cell(MarchArgs<R, G> const & a, GeoView<G, SH> const & gv, int32_t const * nbr,
+                                          RS & recs, R * so0n, CA * carry = nullptr, R const * u0 = nullptr,
+                                          R * d0 = nullptr)
 {
     constexpr int ND = CellT<CT>::ND;
     constexpr int NEQ = ND + 2;
@@ -229,21 +209,21 @@ __device__ __forceinline__ void soln_cell(MarchArgs<R, G> const & a, int64_t icl
 #pragma unroll
     for (int f = 0; f < NFC; ++f)
     {
-        int64_t const jr = ldg(a.nbr + f * a.ncell + icl);
+        int64_t const jr = nbr[f];
         R rec[RC::NUSED];
-        load_rec<ND>(a.cur + jr * RC::RS, rec);
+        recs.load(f, rec);
         R const * u = rec;
         R const * t = rec + NEQ;
         R const * g = rec + 2 * NEQ;
         R const ga = ldg(a.gamma + jr);
 
-        R const bvol = fg<ND>(a, f, D::K_BVOL, icl);
+        R const bvol = fg<ND>(gv, f, D::K_BVOL);
         R dB[ND], nh[ND], qn[ND];
 #pragma unroll
         for (int d = 0; d < ND; ++d)
         {
-            dB[d] = fg<ND>(a, f, D::K_DB + d, icl);
-            nh[d] = fg<ND>(a, f, D::K_NH + d, icl);
+            dB[d] = fg<ND>(gv, f, D::K_DB + d);
+            nh[d] = fg<ND>(gv, f, D::K_NH + d);
             qn[d] = a.qdt * nh[d];
         }
         if (carry)
@@ -259,8 +239,8 @@ __device__ __forceinline__ void soln_cell(MarchArgs<R, G> const & a, int64_t icl
                 }
                 else
                 {
-                    A[d] = fg<ND>(a, f, D::K_R + d, icl);
-                    B[d] = fg<ND>(a, f, D::K_Q + d, icl);
+                    A[d] = fg<ND>(gv, f, D::K_R + d);
+                    B[d] = fg<ND>(gv, f, D::K_Q + d);
                 }
             }
 #pragma unroll
@@ -302,7 +282,7 @@ __device__ __forceinline__ void soln_cell(MarchArgs<R, G> const & a, int64_t icl
 #pragma unroll
                 for (int e = 0; e < ND; ++e)
                 {
-                    s += g[i * ND + e] * fg<ND>(a, f, D::K_MH + e * ND + d, icl);
+                    s += g[i * ND + e] * fg<ND>(gv, f, D::K_MH + e * ND + d);
                 }
                 w[i * ND + d] = s;
             }
@@ -317,7 +297,7 @@ __device__ __forceinline__ void soln_cell(MarchArgs<R, G> const & a, int64_t icl
             acc[i].add(-fl[i]);
         }
     }
-    R const ivol = geo_ld<ND, R>(a.cgeo + 0 * a.ncell + icl);
+    R const ivol = cg<ND>(gv, 0);
 #pragma unroll
     for (int i = 0; i < NEQ; ++i)
     {
@@ -340,8 +320,8 @@ __device__ __forceinline__ void soln_cell(MarchArgs<R, G> const & a, int64_t icl
 // reference's three divisions by rho use one reciprocal 1/(rho + TINY) (the
 // floor changes nothing unless rho is below 1e-23); it is returned in rinv for the
 // primitives of the same state.
-template <int ND, typename R, typename G>
-__device__ __forceinline__ R cfl_cell(MarchArgs<R, G> const & a, int64_t icl, int64_t row, R * so0n, R & rinv)
+template <int ND, typename R, typename G, bool SH>
+__device__ __forceinline__ R cfl_cell(MarchArgs<R, G> const & a, GeoView<G, SH> const & gv, int64_t row, R * so0n, R & rinv)
 {
     constexpr int NEQ = ND + 2;
     R const ga = ldg(a.gamma + row);
@@ -358,7 +338,7 @@ __device__ __forceinline__ R cfl_cell(MarchArgs<R, G> const & a, int64_t icl, in
     R const pr = ga1 * (so0n[NEQ - 1] - ke);
     R const pra = (pr + fabs(pr)) / R(2);
     R const wspd = sqr_t(ga * pra * ri) + sqr_t(momsq) * ri;
-    R const cflo = wspd * geo_ld<ND, R>(a.cgeo + 1 * a.ncell + icl);
+    R const cflo = wspd * cg<ND>(gv, 1);
     // pra / (pra + TINY) is exactly 1 whenever TINY does not change pra (any
     // pressure above ~1e-44 in FP64), so the division is taken only below.
     R const prt = pra + Tiny<R>::CFL;
@@ -381,8 +361,8 @@ __device__ __forceinline__ R cfl_cell(MarchArgs<R, G> const & a, int64_t icl, in
 // gathered a second time (calc_soln just read them, so the loads hit in
 // cache); carrying calc_soln's neighbour terms over instead costs more FP64
 // operations, but pays in FP32 for simplices (carry != nullptr, see Carry).
-template <int CT, typename R, typename G, typename CA = Carry<CellT<CT>::ND, CellT<CT>::NFC, R>>
-__device__ __forceinline__ void dsoln_cell(MarchArgs<R, G> const & a, int64_t icl, R const * so0n, R cflc,
+template <int CT, typename R, typename G, bool SH, typename CA = Carry<CellT<CT>::ND, CellT<CT>::NFC, R>>
+__device__ __forceinline__ void dsoln_cell(MarchArgs<R, G> const & a, GeoView<G, SH> const & gv, int64_t icl, R const * so0n, R cflc,
                                            R * so1n, CA const * carry = nullptr,
                                            R const * u0 = nullptr, R const * d0 = nullptr)
 {
@@ -413,7 +393,7 @@ __device__ __forceinline__ void dsoln_cell(MarchArgs<R, G> const & a, int64_t ic
     }
     else
     {
-        face_means<CT, R, G>(a, icl, mm, mb);
+        face_means<CT, R>(gv, mm, mb);
     }
     R idis[NFC][ND];
 #pragma unroll
@@ -424,12 +404,12 @@ __device__ __forceinline__ void dsoln_cell(MarchArgs<R, G> const & a, int64_t ic
         {
             if constexpr (D::MID)
             {
-                idis[f][d] = (fg<ND>(a, f, D::K_MID + d, icl) - mm[d]) +
-                             tau * (mb[d] - fg<ND>(a, f, D::K_DB + d, icl));
+                idis[f][d] = (fg<ND>(gv, f, D::K_MID + d) - mm[d]) +
+                             tau * (mb[d] - fg<ND>(gv, f, D::K_DB + d));
             }
             else
             {
-                idis[f][d] = fg<ND>(a, f, D::K_P + d, icl) + tau * fg<ND>(a, f, D::K_Q + d, icl);
+                idis[f][d] = fg<ND>(gv, f, D::K_P + d) + tau * fg<ND>(gv, f, D::K_Q + d);
             }
         }
     }
@@ -510,12 +490,12 @@ __device__ __forceinline__ void dsoln_cell(MarchArgs<R, G> const & a, int64_t ic
             {
                 if constexpr (D::MID)
                 {
-                    R const db = fg<ND>(a, f, D::K_DB + d, icl);
+                    R const db = fg<ND>(gv, f, D::K_DB + d);
                     jd[d] = (db - mm[d]) + tau * (mb[d] - db) - delta[d];
                 }
                 else
                 {
-                    jd[d] = fg<ND>(a, f, D::K_R + d, icl) + tau * fg<ND>(a, f, D::K_Q + d, icl) - delta[d];
+                    jd[d] = fg<ND>(gv, f, D::K_R + d) + tau * fg<ND>(gv, f, D::K_Q + d) - delta[d];
                 }
             }
 #pragma unroll
@@ -840,13 +820,185 @@ __device__ __forceinline__ void deliver_row(MarchArgs<R, G> const & a, int64_t r
     }
 }
 
+// What an FP32 cell's substep reads first: its neighbours' rows and its own
+// current state.
+template <int ND, int NFC>
+struct CellHead
+{
+    int32_t nbr[NFC];
+    float u0[ND + 2];
+
+    template <typename G>
+    __device__ __forceinline__ CellHead(MarchArgs<float, G> const & a, int64_t icl)
+    {
+#pragma unroll
+        for (int f = 0; f < NFC; ++f)
+        {
+            nbr[f] = ldg(a.nbr + f * a.ncell + icl);
+        }
+        load_rec<ND, ND + 2>(a.cur + (icl + a.ngst) * Rec<ND, float>::RS, u0);
+    }
+};
+
+// Neighbour records read, and a cell's own stored, by its thread.
+template <int ND>
+struct DirectRecs
+{
+    float const * cur;
+    int32_t const * nbr;
+
+    __device__ __forceinline__ void load(int f, float * rec)
+    {
+        load_rec<ND>(cur + static_cast<int64_t>(nbr[f]) * Rec<ND, float>::RS, rec);
+    }
+};
+template <int ND>
+struct DirectOut
+{
+    float * row;
+
+    __device__ __forceinline__ void store(float const * so0, float const * so0t, float const * so1)
+    {
+        store_rec<ND>(row, so0, so0t, so1);
+    }
+};
+
+__device__ __forceinline__ void copy_async16(unsigned to, void const * from)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(to), "l"(from) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// Wait until at most n of the committed groups are still on their way.
+__device__ __forceinline__ void copy_wait(int n)
+{
+    switch (n)
+    {
+    case 0: asm volatile("cp.async.wait_group 0;" ::: "memory"); break;
+    case 1: asm volatile("cp.async.wait_group 1;" ::: "memory"); break;
+    case 2: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
+    default: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
+    }
+}
+
+// The neighbour records of a warp's cells, fetched together: a record's 64
+// (2D) or 128 (3D) bytes by 4 or 8 neighbouring lanes, 16 bytes each, straight
+// into shared memory, so that a load instruction touches 8 or 4 whole records
+// instead of a piece of 32 (a warp's loads of its own records kept the L1's
+// data path 52% busy in 2D and 77% in 3D), and NB faces' records are on their
+// way at once without holding registers.  Chunk c of lane i's record lies at
+// chunk place c ^ (i's low bits), so neither the copies nor the reads of 8 lanes
+// meet in a bank.
+template <int ND, int NFC, int NB>
+struct StagedRecs
+{
+    static constexpr int LPR = ND == 2 ? 4 : 8;                       // lanes, and chunk places, per record
+    static constexpr int CH = (Rec<ND, float>::NUSED + 3) / 4;        // chunks used
+    static constexpr int BUF = 32 * LPR;                              // chunks of one face's records
+    static constexpr int BYTES = NB * BUF * 16;                       // per warp
+    float const * cur;
+    int32_t const * nbr;
+    float4 * buf;
+
+    __device__ __forceinline__ static int place(int lane, int c)
+    {
+        return lane * LPR + (c ^ (ND == 2 ? (lane >> 1) & 3 : lane & 7));
+    }
+    __device__ __forceinline__ void fetch(int f)
+    {
+        int const ln = static_cast<int>(threadIdx.x) & 31;
+        int const c = ln % LPR;
+        float4 * const b = buf + (f % NB) * BUF;
+#pragma unroll
+        for (int r = 0; r < LPR; ++r)
+        {
+            int const i = r * (32 / LPR) + ln / LPR;
+            int64_t const j = __shfl_sync(0xffffffffu, nbr[f], i);
+            if (CH == LPR || c < CH)
+            {
+                copy_async16(static_cast<unsigned>(__cvta_generic_to_shared(b + place(i, c))),
+                             cur + j * Rec<ND, float>::RS + 4 * c);
+            }
+        }
+    }
+    // Fetch the first NB faces (the first one's group holds what the caller
+    // has copied before).
+    __device__ __forceinline__ void begin()
+    {
+#pragma unroll
+        for (int f = 0; f < NB; ++f)
+        {
+            fetch(f);
+            copy_commit();
+        }
+    }
+    __device__ __forceinline__ void load(int f, float * rec)
+    {
+        int const ln = static_cast<int>(threadIdx.x) & 31;
+        float4 const * const b = buf + (f % NB) * BUF;
+        copy_wait(f + NB <= NFC ? NB - 1 : NFC - 1 - f);
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < CH; ++c)
+        {
+            float4 const v = b[place(ln, c)];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+            {
+                if (4 * c + k < Rec<ND, float>::NUSED)
+                {
+                    rec[4 * c + k] = k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w;
+                }
+            }
+        }
+        if (f + NB < NFC)
+        {
+            __syncwarp(); // every lane has read its record
+            fetch(f + NB);
+            copy_commit();
+        }
+    }
+};
+
+// A cell's new record into its place in shared memory, for the warp to store
+// together.
+template <int ND, int LPR>
+struct StagedOut
+{
+    float4 * buf;
+
+    __device__ __forceinline__ void store(float const * so0, float const * so0t, float const * so1)
+    {
+        constexpr int NEQ = ND + 2;
+        constexpr int CH = (Rec<ND, float>::NUSED + 3) / 4;
+        int const ln = static_cast<int>(threadIdx.x) & 31;
+        float v[4 * CH];
+#pragma unroll
+        for (int i = 0; i < 4 * CH; ++i)
+        {
+            v[i] = i < NEQ ? so0[i]
+                           : (i < 2 * NEQ ? so0t[i - NEQ] : (i < Rec<ND, float>::NUSED ? so1[i - 2 * NEQ] : 0.f));
+        }
+#pragma unroll
+        for (int c = 0; c < CH; ++c)
+        {
+            buf[StagedRecs<ND, ND + 1, 1>::place(ln, c)] =
+                make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+        }
+    }
+};
+
 // One fused CESE substep for one body cell: soln, bc_soln of its boundary
 // faces, cfl, dsoln, bc_dsoln of its boundary faces, and calc_solt of the next
 // substep for its own row and its ghost rows.  Reads only the current records
 // (neighbours' old values) and writes only rows it owns, so one launch covers
 // the whole substep with no grid-wide synchronisation.
-template <int CT, typename R, typename G, int SB = 0>
-__device__ __forceinline__ void fused_cell(MarchArgs<R, G> const & a, int64_t icl)
+// recs: see soln_cell; out.store(so0n, so0t, so1n) keeps the new record.  live:
+// false for a lane past the mesh, which takes part in calc_soln (whose records
+// the warp may fetch together) for its last cell, and does no more.
+template <int CT, typename R, typename G, bool SH, int SB, typename RS, typename OUT>
+__device__ __forceinline__ void fused_cell(MarchArgs<R, G> const & a, GeoView<G, SH> const & gv, int64_t icl,
+                                           CellHead<CellT<CT>::ND, CellT<CT>::NFC> const & head, RS & recs, OUT & out,
+                                           bool live)
 {
     constexpr int ND = CellT<CT>::ND;
     constexpr int NEQ = ND + 2;
@@ -870,13 +1022,17 @@ __device__ __forceinline__ void fused_cell(MarchArgs<R, G> const & a, int64_t ic
     }
     if constexpr (CARRY)
     {
-        face_means<CT, R, G>(a, icl, carry.mm, carry.mb);
+        face_means<CT, R>(gv, carry.mm, carry.mb);
     }
     // Work relative to the cell's own current state (delta form).
-    R u0[NEQ], d0[NEQ];
-    load_rec<ND, NEQ>(a.cur + row * Rec<ND, R>::RS, u0);
+    R const * const u0 = head.u0;
+    R d0[NEQ];
     R so0n[NEQ];
-    soln_cell<CT, R, G>(a, icl, so0n, CARRY ? &carry : nullptr, u0, d0);
+    soln_cell<CT>(a, gv, head.nbr, recs, so0n, CARRY ? &carry : nullptr, u0, d0);
+    if (!live)
+    {
+        return;
+    }
     // FP32 error feedback: what rounding the new so0 to FP32 drops is kept per
     // cell and equation (comp) and added back to the cell's next new value,
     // the rounding taken by an exact two-sum (Knuth) so the kept residual is
@@ -909,7 +1065,7 @@ __device__ __forceinline__ void fused_cell(MarchArgs<R, G> const & a, int64_t ic
 #pragma unroll
     for (int f = 0; f < NFC; ++f)
     {
-        int64_t const jr = ldg(a.nbr + f * a.ncell + icl);
+        int64_t const jr = head.nbr[f];
         if (jr < a.ngst)
         {
             int const kind = a.gkind[jr];
@@ -929,7 +1085,7 @@ __device__ __forceinline__ void fused_cell(MarchArgs<R, G> const & a, int64_t ic
 
     R rinv;
     R const e_soln = so0n[NEQ - 1];
-    R const cflc = cfl_cell<ND, R, G>(a, icl, row, so0n, rinv);
+    R const cflc = cfl_cell<ND>(a, gv, row, so0n, rinv);
     if (so0n[NEQ - 1] != e_soln)
     {
         d0[NEQ - 1] = so0n[NEQ - 1] - u0[NEQ - 1]; // calc_cfl rewrote the energy
@@ -958,11 +1114,11 @@ __device__ __forceinline__ void fused_cell(MarchArgs<R, G> const & a, int64_t ic
         }
     }
     R so1n[NEQ * ND];
-    dsoln_cell<CT, R, G>(a, icl, so0n, cflc, so1n, CARRY ? &carry : nullptr, u0, d0);
+    dsoln_cell<CT>(a, gv, icl, so0n, cflc, so1n, CARRY ? &carry : nullptr, u0, d0);
     R so0t[NEQ];
     Prim<ND, R> const q(so0n, ldg(a.gamma + row), rinv);
     solt_prim<ND, R>(q, so0n, so1n, so0t);
-    store_rec<ND>(a.nxt + row * Rec<ND, R>::RS, so0n, so0t, so1n);
+    out.store(so0n, so0t, so1n);
 }
 
 // The same in FP64 (euler_fp64.cuh).
@@ -1016,7 +1172,108 @@ __device__ __forceinline__ void substep_cell(MarchArgs<R, G> const & a, int64_t 
     }
     else
     {
-        fused_cell<CT, R, G, SB>(a, icl);
+        constexpr int ND = CellT<CT>::ND;
+        CellHead<ND, CellT<CT>::NFC> const head(a, icl);
+        DirectRecs<ND> recs{a.cur, head.nbr};
+        DirectOut<ND> out{a.nxt + (icl + a.ngst) * Rec<ND, float>::RS};
+        fused_cell<CT, R, G, false, SB>(a, geo_view(a, icl), icl, head, recs, out, true);
+    }
+}
+
+// What the single-type FP32 kernels stage in shared memory (staged_cell): the
+// neighbour records of NB faces at a time, and in 2D the geometry (6 KB per
+// warp; in 3D it is 13 KB, room for two blocks per SM).  Shared memory and
+// registers then set the resident blocks together; measured, 2M triangles, us
+// per launch at the best register budget for each: nothing staged 180 (FP32
+// form) and 159 (fp32-geom32); geometry alone 163 and 149; records alone
+// (one face) 182 and 177; geometry and the records of one, two, three faces
+// 161, 156, 157 and 136, 138, 151.  1.3M tetrahedra: nothing staged 271, the
+// records of one, two, four faces 245, 300, 372.
+template <int CT, typename G>
+struct Stage
+{
+    static constexpr int ND = CellT<CT>::ND;
+    static constexpr int NFC = CellT<CT>::NFC;
+    static constexpr bool GEO = ND == 2;
+    static constexpr int NB = ND == 2 && !Geo<ND, G>::MID ? 2 : 1;
+    using Recs = StagedRecs<ND, NFC, NB>;
+    static constexpr int NPL = Dim<ND>::KC + NFC * Geo<ND, G>::KF;
+    static constexpr int GEO_BYTES = GEO ? NPL * GEO_TILE * 4 : 0;
+    static constexpr int WARP_BYTES = Recs::BYTES + GEO_BYTES;
+};
+
+// Dynamic shared memory of a fused kernel with blocks of B threads.
+template <typename R, typename G, int CT1, int B>
+__host__ __device__ constexpr int stage_bytes()
+{
+    if constexpr (CT1 != 0 && sizeof(R) == 4)
+    {
+        return B / 32 * Stage<CT1, G>::WARP_BYTES;
+    }
+    else
+    {
+        return 0;
+    }
+}
+
+// An FP32 substep of a warp's cells with their neighbours' records (StagedRecs)
+// and, in 2D, their geometry (one contiguous tile, see GeoView) copied to
+// shared memory by 16-byte asynchronous copies, and their own new records
+// stored together from there.
+template <int CT, typename G, int SB>
+__device__ __forceinline__ void staged_cell(MarchArgs<float, G> const & a, int64_t t)
+{
+    using S = Stage<CT, G>;
+    constexpr int ND = S::ND;
+    constexpr int NFC = S::NFC;
+    constexpr int RS = Rec<ND, float>::RS;
+    static_assert(sizeof(G) == 4, "a tile of 4-byte values");
+    extern __shared__ __align__(16) char s_stage[];
+    char * const mine = s_stage + (threadIdx.x / 32) * S::WARP_BYTES;
+    int const lane = static_cast<int>(threadIdx.x) & 31;
+    int64_t const first = t - lane; // the warp's first cell, a multiple of 32
+    int64_t const icl = t < a.ncell ? t : a.ncell - 1;
+    CellHead<ND, NFC> const head(a, icl);
+    G * const geo = reinterpret_cast<G *>(mine + S::Recs::BYTES);
+    if constexpr (S::GEO)
+    {
+        G const * const tile = a.geo + (first / GEO_TILE) * (S::NPL * GEO_TILE);
+        constexpr int N = S::GEO_BYTES / 16;
+#pragma unroll
+        for (int k = 0; k < N; k += 32)
+        {
+            if (k + 32 <= N || k + lane < N)
+            {
+                copy_async16(static_cast<unsigned>(__cvta_generic_to_shared(geo + 4 * (k + lane))),
+                             tile + 4 * (k + lane));
+            }
+        }
+    }
+    typename S::Recs recs{a.cur, head.nbr, reinterpret_cast<float4 *>(mine)};
+    recs.begin();
+    StagedOut<ND, S::Recs::LPR> out{recs.buf};
+    bool const live = t < a.ncell;
+    constexpr int CB = carry_shared<ND>() ? SB : 0;
+    if constexpr (S::GEO)
+    {
+        copy_wait(S::NB - 1); // the geometry and the first face's records
+        __syncwarp();
+        fused_cell<CT, float, G, true, CB>(a, GeoView<G, true>{geo + lane}, icl, head, recs, out, live);
+    }
+    else
+    {
+        fused_cell<CT, float, G, false, CB>(a, geo_view(a, icl), icl, head, recs, out, live);
+    }
+    __syncwarp();
+    int const c = lane % S::Recs::LPR;
+#pragma unroll
+    for (int r = 0; r < S::Recs::LPR; ++r)
+    {
+        int const i = r * (32 / S::Recs::LPR) + lane / S::Recs::LPR;
+        if ((S::Recs::CH == S::Recs::LPR || c < S::Recs::CH) && first + i < a.ncell)
+        {
+            reinterpret_cast<float4 *>(a.nxt + (first + i + a.ngst) * RS)[c] = recs.buf[S::Recs::place(i, c)];
+        }
     }
 }
 
@@ -1024,16 +1281,23 @@ __device__ __forceinline__ void substep_cell(MarchArgs<R, G> const & a, int64_t 
 // t - ncell after that.  CT1 = 0 dispatches on each cell's type; a nonzero
 // CT1 compiles the one cell type of a single-type mesh, whose kernel then
 // needs only that type's registers.
-template <int ND, typename R, typename G, int CT1 = 0, int SB = 0>
-__device__ __forceinline__ void fused_thread(MarchArgs<R, G> const & a, int64_t t)
+template <int ND, typename R, typename G, int CT1, int SB>
+__device__ __forceinline__ void fused_thread(MarchArgs<R, G> const & a, int64_t t, int64_t t1)
 {
-    if (t < a.ncell)
+    if constexpr (CT1 != 0 && sizeof(R) == 4)
+    {
+        if ((t & ~static_cast<int64_t>(31)) < a.ncell) // the whole warp
+        {
+            staged_cell<CT1, G, SB>(a, t);
+        }
+    }
+    else if (t < a.ncell && t < t1)
     {
         int const ct = a.ctype[t];
         if constexpr (CT1 != 0)
         {
             (void)ct;
-            substep_cell<CT1, R, G, SB>(a, t);
+            substep_cell<CT1, R, G, carry_shared<ND>() ? SB : 0>(a, t);
         }
         else if constexpr (ND == 2)
         {
@@ -1053,7 +1317,7 @@ __device__ __forceinline__ void fused_thread(MarchArgs<R, G> const & a, int64_t 
             }
         }
     }
-    else if (t < a.ncell + a.ngst)
+    if (t >= a.ncell && t < a.ncell + a.ngst && t < t1)
     {
         // A ghost row without a boundary condition keeps its stale state; its
         // next so0t is still the Jacobian product of that state.
@@ -1093,9 +1357,9 @@ template <int ND, typename R, typename G, int CT1 = 0>
 __global__ void __launch_bounds__(128) k_fused(MarchArgs<R, G> a, int64_t t0, int64_t t1)
 {
     int64_t const t = t0 + static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (t < t1)
+    if ((t & ~static_cast<int64_t>(31)) < t1)
     {
-        fused_thread<ND, R, G, CT1, carry_shared<ND>() ? 128 : 0>(a, t);
+        fused_thread<ND, R, G, CT1, 128>(a, t, t1);
     }
 }
 
@@ -1107,9 +1371,9 @@ template <int ND, typename R, typename G, int CT1, int MINB>
 __global__ void __launch_bounds__(128, MINB) k_fused_mb(MarchArgs<R, G> a, int64_t t0, int64_t t1)
 {
     int64_t const t = t0 + static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (t < t1)
+    if ((t & ~static_cast<int64_t>(31)) < t1)
     {
-        fused_thread<ND, R, G, CT1, carry_shared<ND>() ? 128 : 0>(a, t);
+        fused_thread<ND, R, G, CT1, 128>(a, t, t1);
     }
 }
 

@@ -260,7 +260,7 @@ __device__ __forceinline__ G geo_store(double v, bool conv, unsigned long long *
 // neighbour-row table and the cell types.
 template <int ND, typename G>
 __global__ void k_compact(MeshView m, double const * cevol, double const * cecnd, double const * sfcnd,
-                          double const * sfnml, double hdt, int nslot, G * fgeo, G * cgeo, int32_t * nbr,
+                          double const * sfnml, double hdt, int nslot, int64_t npl, G * geo, int32_t * nbr,
                           int8_t * ctype, unsigned long long * bad)
 {
     using D = Geo<ND, G>;
@@ -286,9 +286,10 @@ __global__ void k_compact(MeshView m, double const * cevol, double const * cecnd
         B[d] = 0.0;
     }
     double dist = 1.79769313486231570815e+308;
+    G * const row_geo = geo + (icl / GEO_TILE) * npl * GEO_TILE + icl % GEO_TILE;
     auto put = [&](int f, int k, double v) {
         bool const conv = !D::MID && k >= D::K_P && k < D::K_P + ND;
-        fgeo[(static_cast<int64_t>(f) * D::KF + k) * nc + icl] = geo_store<ND, G>(v, conv, bad);
+        row_geo[(Dim<ND>::KC + f * D::KF + k) * GEO_TILE] = geo_store<ND, G>(v, conv, bad);
     };
     for (int f = 0; f < clnfc; ++f)
     {
@@ -375,8 +376,8 @@ __global__ void k_compact(MeshView m, double const * cevol, double const * cecnd
             put(f, k, 0.0);
         }
     }
-    cgeo[0 * nc + icl] = geo_store<ND, G>(1.0 / cevol[row * 7], true, bad);
-    cgeo[1 * nc + icl] = geo_store<ND, G>(hdt / dist, true, bad);
+    row_geo[0 * GEO_TILE] = geo_store<ND, G>(1.0 / cevol[row * 7], true, bad);
+    row_geo[1 * GEO_TILE] = geo_store<ND, G>(hdt / dist, true, bad);
 }
 
 } // namespace dev
