@@ -922,20 +922,26 @@ public:
             cudaStreamSynchronize(m_xfer);
             cudaStreamDestroy(m_xfer);
         }
-        if (m_side)
+        for (cudaStream_t s : {m_side, m_copy})
         {
-            cudaStreamSynchronize(m_side);
-            cudaStreamDestroy(m_side);
+            if (s)
+            {
+                cudaStreamSynchronize(s);
+                cudaStreamDestroy(s);
+            }
         }
         if (m_cev)
         {
             cudaEventDestroy(m_cev);
         }
-        for (auto & e : m_xev)
+        for (auto * list : {m_xev, m_cpev})
         {
-            if (e)
+            for (int k = 0; k < XCH + 1; ++k)
             {
-                cudaEventDestroy(e);
+                if (list[k])
+                {
+                    cudaEventDestroy(list[k]);
+                }
             }
         }
     }
@@ -1532,8 +1538,8 @@ public:
     }
 
     // The fused kernel specialised to the mesh's cell type when it has only
-    // triangles or only tetrahedra (the simplex paths), else the generic one,
-    // over rows [t0, t1) of its work order (body cells, then ghost rows).
+    // triangles, tetrahedra or (FP64) hexahedra, else the generic one, over
+    // rows [t0, t1) of its work order (body cells, then ghost rows).
     void launch_fused(int64_t t0 = 0, int64_t t1 = -1)
     {
         if (t1 < 0)
@@ -1544,7 +1550,10 @@ public:
         {
             return;
         }
-        unsigned const g = grid_for(t1 - t0);
+        // FP64: blocks of one warp, whose work is long and ends unevenly (48k
+        // tetrahedra 136 -> 120 us per launch against blocks of four).
+        int const block = sizeof(R) == 8 ? 32 : BLOCK;
+        unsigned const g = static_cast<unsigned>((t1 - t0 + block - 1) / block);
         constexpr int SIMPLEX = (ND == 2) ? CT_TRIANGLE : CT_TET;
         if (single_ct == SIMPLEX)
         {
@@ -1557,12 +1566,31 @@ public:
             }
             else
             {
-                k_fused<ND, R, G, SIMPLEX><<<g, BLOCK, 0, stream>>>(args(), t0, t1);
+                k_fused<ND, R, G, SIMPLEX><<<g, block, 0, stream>>>(args(), t0, t1);
             }
         }
         else
         {
-            k_fused<ND, R, G><<<g, BLOCK, 0, stream>>>(args(), t0, t1);
+            if constexpr (ND == 3 && sizeof(R) == 8)
+            {
+                // 255 registers would leave 8 warps per SM, too few to keep its
+                // FP64 pipes fed through their loads: a spilling kernel of 16
+                // (hexahedra) or 12 warps is faster.  64k / 343k hexahedra: 353 /
+                // 1,948 us per launch at 255 registers, 362 / 1,780 at 168, 335 /
+                // 1,717 at 128; 54k prisms 277, 223, 250.
+                if (single_ct == CT_HEX)
+                {
+                    k_fused_mb<ND, R, G, CT_HEX, 4><<<g, block, 0, stream>>>(args(), t0, t1);
+                }
+                else
+                {
+                    k_fused_mb<ND, R, G, 0, 3><<<g, block, 0, stream>>>(args(), t0, t1);
+                }
+            }
+            else
+            {
+                k_fused<ND, R, G><<<g, block, 0, stream>>>(args(), t0, t1);
+            }
         }
     }
 
@@ -1650,28 +1678,46 @@ public:
         constexpr int W = NEQ * ND;
         double * const st0 = staging(nrow * (NEQ + W));
         double * const st1 = st0 + nrow * NEQ;
-        // The records it writes may still be read by work queued on the
-        // core's stream (an earlier march): that goes first.
+        // The records and the staging table it writes may still be read by work
+        // queued on the core's stream (an earlier march): that goes first.
         cuda_check(cudaEventRecord(m_xev[XCH], stream), "record");
+        cuda_check(cudaStreamWaitEvent(m_copy, m_xev[XCH], 0), "wait");
         cuda_check(cudaStreamWaitEvent(m_xfer, m_xev[XCH], 0), "wait");
+        // The chunks of the substep write disjoint rows, so they alternate
+        // between the core's stream and a second one: a chunk's last partial
+        // wave overlaps the next chunk instead of idling SMs.
+        cuda_check(cudaStreamWaitEvent(m_side, m_xev[XCH], 0), "wait");
         R * base;
         int off, width;
         field_of(EA_SO0N, base, off, width);
         bool const solt = tbuf != (cur ^ 1);
         Residual const c = so0_written(EA_SO0N);
-        for (int j = 0; j < nch; ++j)
+        // What the two sets leave behind, and the substep's buffer swap.
+        next_valid = solt;
+        next_buf = cur ^ 1;
+        comp_ready();
+        cur ^= 1;
+        if (solt)
         {
+            tbuf = cur;
+        }
+        m_deliver_now = false;
+        // Upload chunk j: the copies on their own stream, so that they run
+        // back to back while the scatters of earlier chunks run.
+        auto upload = [&](int j) {
             int64_t const r0 = j == 0 ? 0 : ngstcell + m_plan.cell[j];
             int64_t const r1 = ngstcell + m_plan.cell[j + 1];
             int64_t const nr = r1 - r0;
             double * const in0 = st0 + r0 * NEQ;
             double * const in1 = st1 + r0 * W;
             cuda_check(cudaMemcpyAsync(in0, so0n + r0 * NEQ, sizeof(double) * static_cast<size_t>(nr * NEQ),
-                                       cudaMemcpyHostToDevice, m_xfer),
+                                       cudaMemcpyHostToDevice, m_copy),
                        "H2D");
             cuda_check(cudaMemcpyAsync(in1, so1n + r0 * W, sizeof(double) * static_cast<size_t>(nr * W),
-                                       cudaMemcpyHostToDevice, m_xfer),
+                                       cudaMemcpyHostToDevice, m_copy),
                        "H2D");
+            cuda_check(cudaEventRecord(m_cpev[j], m_copy), "record");
+            cuda_check(cudaStreamWaitEvent(m_xfer, m_cpev[j], 0), "wait");
             k_set_field_host<ND, R><<<grid_for((nr * NEQ + 1) / 2), BLOCK, 0, m_xfer>>>(
                 base + r0 * RS, in0, nr, 0, NEQ, reinterpret_cast<uintptr_t>(in0) % 16 == 0,
                 Residual{c.comp, c.ngst - r0, c.ncell});
@@ -1690,29 +1736,7 @@ public:
                 launched(m_xfer, "set_field_host");
             }
             cuda_check(cudaEventRecord(m_xev[j], m_xfer), "record");
-        }
-        // What the two sets leave behind.
-        next_valid = solt;
-        next_buf = cur ^ 1;
-        // The first substep, as march_substep with its fused launch in
-        // chunks.
-        comp_ready();
-        cur ^= 1;
-        if (next_valid && next_buf == cur)
-        {
-            tbuf = cur;
-        }
-        else
-        {
-            cuda_check(cudaStreamWaitEvent(stream, m_xev[nch - 1], 0), "wait");
-            run_solt();
-        }
-        m_deliver_now = false;
-        // The chunks write disjoint rows, so they alternate between the
-        // core's stream and a second one: a chunk's last partial wave
-        // overlaps the next chunk instead of idling SMs.
-        cuda_check(cudaEventRecord(m_cev, stream), "record");
-        cuda_check(cudaStreamWaitEvent(m_side, m_cev, 0), "wait");
+        };
         cudaStream_t const mine = stream;
         {
             // The core's stream is back to its own even if a launch throws.
@@ -1722,12 +1746,27 @@ public:
                 cudaStream_t v;
                 ~Restore() { s = v; }
             } const restore{stream, mine};
-            for (int k = 0; k < nch; ++k)
+            // Each chunk of the substep is queued right after the last upload
+            // chunk that it waits for.
+            int k = 0;
+            for (int j = 0; j < nch; ++j)
             {
-                stream = (k & 1) ? m_side : mine;
-                cuda_check(cudaStreamWaitEvent(stream, m_xev[m_plan.need[k]], 0), "wait");
-                launch_fused(m_plan.cell[k], m_plan.cell[k + 1]);
-                launched(stream, "fused_substep");
+                upload(j);
+                if (!solt && j + 1 == nch)
+                {
+                    stream = mine;
+                    cuda_check(cudaStreamWaitEvent(mine, m_xev[j], 0), "wait");
+                    run_solt();
+                    cuda_check(cudaEventRecord(m_cev, mine), "record");
+                    cuda_check(cudaStreamWaitEvent(m_side, m_cev, 0), "wait");
+                }
+                for (; k < nch && (solt ? m_plan.need[k] <= j : j + 1 == nch); ++k)
+                {
+                    stream = (k & 1) ? m_side : mine;
+                    cuda_check(cudaStreamWaitEvent(stream, m_xev[m_plan.need[k]], 0), "wait");
+                    launch_fused(m_plan.cell[k], m_plan.cell[k + 1]);
+                    launched(stream, "fused_substep");
+                }
             }
         }
         cuda_check(cudaEventRecord(m_cev, m_side), "record");
@@ -1769,10 +1808,14 @@ public:
         {
             cuda_check(cudaStreamCreateWithFlags(&m_xfer, cudaStreamNonBlocking), "cudaStreamCreate");
             cuda_check(cudaStreamCreateWithFlags(&m_side, cudaStreamNonBlocking), "cudaStreamCreate");
+            cuda_check(cudaStreamCreateWithFlags(&m_copy, cudaStreamNonBlocking), "cudaStreamCreate");
             cuda_check(cudaEventCreateWithFlags(&m_cev, cudaEventDisableTiming), "event");
-            for (auto & e : m_xev)
+            for (auto * list : {m_xev, m_cpev})
             {
-                cuda_check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
+                for (int k = 0; k < XCH + 1; ++k)
+                {
+                    cuda_check(cudaEventCreateWithFlags(list + k, cudaEventDisableTiming), "event");
+                }
             }
         }
         int64_t nch = ncell / 65536;
@@ -2021,7 +2064,9 @@ private:
     cudaStream_t m_xfer = nullptr;
     cudaStream_t m_side = nullptr; // the second stream of the chunked substep
     cudaEvent_t m_cev = nullptr;
+    cudaStream_t m_copy = nullptr; // the upload's copies
     cudaEvent_t m_xev[XCH + 1] = {};
+    cudaEvent_t m_cpev[XCH + 1] = {};
     struct ChunkPlan
     {
         bool valid = false;

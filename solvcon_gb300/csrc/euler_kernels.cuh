@@ -820,6 +820,51 @@ __device__ __forceinline__ void deliver_row(MarchArgs<R, G> const & a, int64_t r
     }
 }
 
+// N values v of each lane's row, into the host block's rows row0 .. row0 + 31
+// (those below nrow): the warp's rows are one contiguous piece of the block,
+// which its lanes store 16 (N even) or 8 bytes at a time in order, each taking
+// its values from their lanes by shuffles.  Whole lines then cross the host
+// link; a lane's own 16-byte pieces of its row kept the link below the rate
+// that the substep's time allows (2M triangles, the last substep with its
+// delivery: 2.7 ms against 1.5 without).
+template <int N>
+__device__ __forceinline__ void deliver_rows(double * out, int64_t row0, int nrow, double const * v)
+{
+    constexpr int W = N % 2 == 0 ? 2 : 1; // doubles per store
+    constexpr int PER = N / W;
+    int const ln = static_cast<int>(threadIdx.x) & 31;
+    double * const base = out + row0 * N;
+#pragma unroll
+    for (int r = 0; r < PER; ++r)
+    {
+        int const q = r * 32 + ln;
+        int const src = q / PER;
+        int const p = q % PER;
+        double x[W];
+#pragma unroll
+        for (int k = 0; k < PER; ++k)
+        {
+#pragma unroll
+            for (int w = 0; w < W; ++w)
+            {
+                double const y = __shfl_sync(0xffffffffu, v[k * W + w], src);
+                x[w] = k == 0 || k == p ? y : x[w];
+            }
+        }
+        if (src < nrow)
+        {
+            if constexpr (W == 2)
+            {
+                reinterpret_cast<double2 *>(base)[q] = make_double2(x[0], x[1]);
+            }
+            else
+            {
+                base[q] = x[0];
+            }
+        }
+    }
+}
+
 // What an FP32 cell's substep reads first: its neighbours' rows and its own
 // current state.
 template <int ND, int NFC>
@@ -1121,9 +1166,10 @@ __device__ __forceinline__ void fused_cell(MarchArgs<R, G> const & a, GeoView<G,
     out.store(so0n, so0t, so1n);
 }
 
-// The same in FP64 (euler_fp64.cuh).
+// The same in FP64 (euler_fp64.cuh); the new state is returned too.
 template <int CT>
-__device__ __forceinline__ void fused_cell64(MarchArgs<double, double> const & a, int64_t icl)
+__device__ __forceinline__ void fused_cell64(MarchArgs<double, double> const & a, int64_t icl, double * so0n,
+                                             double * so1n)
 {
     constexpr int ND = CellT<CT>::ND;
     constexpr int NEQ = ND + 2;
@@ -1131,7 +1177,6 @@ __device__ __forceinline__ void fused_cell64(MarchArgs<double, double> const & a
     using RC = Rec<ND, double>;
     using F = FluxTerms<ND>;
     int64_t const row = icl + a.ngst;
-    double so0n[NEQ];
     soln64<CT, true>(a, icl, so0n);
 #pragma unroll 1
     for (int f = 0; f < NFC; ++f)
@@ -1154,21 +1199,19 @@ __device__ __forceinline__ void fused_cell64(MarchArgs<double, double> const & a
     }
     double rinv;
     double const cflc = cfl64<ND>(a, icl, row, so0n, rinv);
-    double so1n[NEQ * ND];
     dsoln64<CT>(a, icl, so0n, cflc, so1n);
     double so0t[NEQ], c[F::N];
     solt_terms<ND>(so0n, so1n, ldg(a.gamma + row), rinv, a.qdt, so0t, c);
     store_row<ND>(a.nxt + row * RC::RS, so0n, so0t, so1n, c);
-    deliver_row<ND>(a, row, so0n, so1n);
 }
 
-// A cell's fused substep in either precision.
+// A cell's fused substep in either precision (so0n, so1n: the FP64 new state).
 template <int CT, typename R, typename G, int SB = 0>
-__device__ __forceinline__ void substep_cell(MarchArgs<R, G> const & a, int64_t icl)
+__device__ __forceinline__ void substep_cell(MarchArgs<R, G> const & a, int64_t icl, R * so0n, R * so1n)
 {
     if constexpr (sizeof(R) == 8)
     {
-        fused_cell64<CT>(a, icl);
+        fused_cell64<CT>(a, icl, so0n, so1n);
     }
     else
     {
@@ -1284,9 +1327,13 @@ __device__ __forceinline__ void staged_cell(MarchArgs<float, G> const & a, int64
 template <int ND, typename R, typename G, int CT1, int SB>
 __device__ __forceinline__ void fused_thread(MarchArgs<R, G> const & a, int64_t t, int64_t t1)
 {
+    constexpr int NEQ = ND + 2;
+    R so0n[NEQ], so1n[NEQ * ND];
+    (void)so0n;
+    (void)so1n;
     if constexpr (CT1 != 0 && sizeof(R) == 4)
     {
-        if ((t & ~static_cast<int64_t>(31)) < a.ncell) // the whole warp
+        if (t - (static_cast<int>(threadIdx.x) & 31) < a.ncell) // the whole warp
         {
             staged_cell<CT1, G, SB>(a, t);
         }
@@ -1297,23 +1344,41 @@ __device__ __forceinline__ void fused_thread(MarchArgs<R, G> const & a, int64_t 
         if constexpr (CT1 != 0)
         {
             (void)ct;
-            substep_cell<CT1, R, G, carry_shared<ND>() ? SB : 0>(a, t);
+            substep_cell<CT1, R, G, carry_shared<ND>() ? SB : 0>(a, t, so0n, so1n);
         }
         else if constexpr (ND == 2)
         {
             if (ct == 4)
-                substep_cell<4, R, G>(a, t);
+                substep_cell<4, R, G>(a, t, so0n, so1n);
             else
-                substep_cell<3, R, G>(a, t);
+                substep_cell<3, R, G>(a, t, so0n, so1n);
         }
         else
         {
             switch (ct)
             {
-            case 6: substep_cell<6, R, G>(a, t); break;
-            case 5: substep_cell<5, R, G>(a, t); break;
-            case 7: substep_cell<7, R, G>(a, t); break;
-            default: substep_cell<8, R, G>(a, t); break;
+            case 6: substep_cell<6, R, G>(a, t, so0n, so1n); break;
+            case 5: substep_cell<5, R, G>(a, t, so0n, so1n); break;
+            case 7: substep_cell<7, R, G>(a, t, so0n, so1n); break;
+            default: substep_cell<8, R, G>(a, t, so0n, so1n); break;
+            }
+        }
+    }
+    if constexpr (sizeof(R) == 8)
+    {
+        if (a.out0 || a.out1)
+        {
+            __syncwarp();
+            int64_t const first = t - (static_cast<int>(threadIdx.x) & 31);
+            int64_t const left = (a.ncell < t1 ? a.ncell : t1) - first;
+            int const nrow = left >= 32 ? 32 : (left > 0 ? static_cast<int>(left) : 0);
+            if (a.out0)
+            {
+                deliver_rows<NEQ>(a.out0, first + a.ngst, nrow, so0n);
+            }
+            if (a.out1)
+            {
+                deliver_rows<NEQ * ND>(a.out1, first + a.ngst, nrow, so1n);
             }
         }
     }
@@ -1324,7 +1389,6 @@ __device__ __forceinline__ void fused_thread(MarchArgs<R, G> const & a, int64_t 
         int64_t const g = t - a.ncell;
         if (a.gkind[g] < 0)
         {
-            constexpr int NEQ = ND + 2;
             R * const base = a.nxt + g * Rec<ND, R>::RS;
             R rec[Rec<ND, R>::NUSED], tt[NEQ];
 #pragma unroll
@@ -1357,7 +1421,7 @@ template <int ND, typename R, typename G, int CT1 = 0>
 __global__ void __launch_bounds__(128) k_fused(MarchArgs<R, G> a, int64_t t0, int64_t t1)
 {
     int64_t const t = t0 + static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if ((t & ~static_cast<int64_t>(31)) < t1)
+    if (t - (static_cast<int>(threadIdx.x) & 31) < t1) // whole warps
     {
         fused_thread<ND, R, G, CT1, 128>(a, t, t1);
     }
@@ -1371,7 +1435,7 @@ template <int ND, typename R, typename G, int CT1, int MINB>
 __global__ void __launch_bounds__(128, MINB) k_fused_mb(MarchArgs<R, G> a, int64_t t0, int64_t t1)
 {
     int64_t const t = t0 + static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if ((t & ~static_cast<int64_t>(31)) < t1)
+    if (t - (static_cast<int>(threadIdx.x) & 31) < t1) // whole warps
     {
         fused_thread<ND, R, G, CT1, 128>(a, t, t1);
     }
