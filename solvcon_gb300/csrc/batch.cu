@@ -62,8 +62,8 @@ __global__ void __launch_bounds__(B) k_fused_batch(MarchArgs<R, G> const * descs
     fused_batch_tiles<ND, R, G, B, CT1>(descs, tiles, ntiles);
 }
 
-// The same with the resident-block request of the single-core kernel whose
-// cells carry calc_soln's neighbour terms (scg::dev::min_blocks).
+// The same with the resident-block request of the single-core kernel
+// (scg::dev::min_blocks).
 template <int ND, typename R, typename G, int B, int CT1, int MINB>
 __global__ void __launch_bounds__(B, MINB) k_fused_batch_mb(MarchArgs<R, G> const * descs, int2 const * tiles,
                                                             int ntiles)
@@ -72,22 +72,9 @@ __global__ void __launch_bounds__(B, MINB) k_fused_batch_mb(MarchArgs<R, G> cons
 }
 
 template <int ND, typename R, typename G, int B, int CT1>
-constexpr int batch_min_blocks()
-{
-    if constexpr (CT1 == 0)
-    {
-        return 0;
-    }
-    else
-    {
-        return scg::dev::min_blocks<ND, R, CT1, B, G>();
-    }
-}
-
-template <int ND, typename R, typename G, int B, int CT1>
 constexpr auto batch_kernel()
 {
-    constexpr int MINB = batch_min_blocks<ND, R, G, B, CT1>();
+    constexpr int MINB = scg::dev::min_blocks<ND, R, CT1, B, G>();
     if constexpr (MINB > 0)
     {
         return &k_fused_batch_mb<ND, R, G, B, CT1, MINB>;

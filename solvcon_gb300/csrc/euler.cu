@@ -1537,9 +1537,10 @@ public:
         }
     }
 
-    // The fused kernel specialised to the mesh's cell type when it has only
-    // triangles, tetrahedra or (FP64) hexahedra, else the generic one, over
-    // rows [t0, t1) of its work order (body cells, then ghost rows).
+    // The fused kernel over rows [t0, t1) of its work order (body cells, then
+    // ghost rows): the one compiled for the mesh's cell type when it has only
+    // triangles, tetrahedra, hexahedra or (FP32) quadrilaterals, else the one
+    // for any mix.
     void launch_fused(int64_t t0 = 0, int64_t t1 = -1)
     {
         if (t1 < 0)
@@ -1550,47 +1551,41 @@ public:
         {
             return;
         }
-        // FP64: blocks of one warp, whose work is long and ends unevenly (48k
-        // tetrahedra 136 -> 120 us per launch against blocks of four).
-        int const block = sizeof(R) == 8 ? 32 : BLOCK;
-        unsigned const g = static_cast<unsigned>((t1 - t0 + block - 1) / block);
-        constexpr int SIMPLEX = (ND == 2) ? CT_TRIANGLE : CT_TET;
+        constexpr int SIMPLEX = ND == 2 ? CT_TRIANGLE : CT_TET;
+        constexpr int BOX = ND == 2 ? CT_QUAD : CT_HEX;
         if (single_ct == SIMPLEX)
         {
-            constexpr int MINB = min_blocks<ND, R, SIMPLEX, BLOCK, G>();
-            if constexpr (MINB > 0)
+            launch_fused_type<SIMPLEX>(t0, t1);
+            return;
+        }
+        if constexpr (ND == 3 || sizeof(R) == 4)
+        {
+            if (single_ct == BOX)
             {
-                constexpr int SMEM = stage_bytes<R, G, SIMPLEX, BLOCK>();
-                allow_shared<k_fused_mb<ND, R, G, SIMPLEX, MINB>, SMEM>();
-                k_fused_mb<ND, R, G, SIMPLEX, MINB><<<g, BLOCK, SMEM, stream>>>(args(), t0, t1);
+                launch_fused_type<BOX>(t0, t1);
+                return;
             }
-            else
-            {
-                k_fused<ND, R, G, SIMPLEX><<<g, block, 0, stream>>>(args(), t0, t1);
-            }
+        }
+        launch_fused_type<0>(t0, t1);
+    }
+
+    template <int CT>
+    void launch_fused_type(int64_t t0, int64_t t1)
+    {
+        // FP64: blocks of one warp, whose work is long and ends unevenly (48k
+        // tetrahedra 136 -> 120 us per launch against blocks of four).
+        constexpr int B = sizeof(R) == 8 ? 32 : BLOCK;
+        constexpr int SMEM = stage_bytes<R, G, CT, B>();
+        constexpr int MINB = min_blocks<ND, R, CT, BLOCK, G>();
+        unsigned const g = static_cast<unsigned>((t1 - t0 + B - 1) / B);
+        if constexpr (MINB > 0)
+        {
+            allow_shared<k_fused_mb<ND, R, G, CT, MINB>, SMEM>();
+            k_fused_mb<ND, R, G, CT, MINB><<<g, B, SMEM, stream>>>(args(), t0, t1);
         }
         else
         {
-            if constexpr (ND == 3 && sizeof(R) == 8)
-            {
-                // 255 registers would leave 8 warps per SM, too few to keep its
-                // FP64 pipes fed through their loads: a spilling kernel of 16
-                // (hexahedra) or 12 warps is faster.  64k / 343k hexahedra: 353 /
-                // 1,948 us per launch at 255 registers, 362 / 1,780 at 168, 335 /
-                // 1,717 at 128; 54k prisms 277, 223, 250.
-                if (single_ct == CT_HEX)
-                {
-                    k_fused_mb<ND, R, G, CT_HEX, 4><<<g, block, 0, stream>>>(args(), t0, t1);
-                }
-                else
-                {
-                    k_fused_mb<ND, R, G, 0, 3><<<g, block, 0, stream>>>(args(), t0, t1);
-                }
-            }
-            else
-            {
-                k_fused<ND, R, G><<<g, block, 0, stream>>>(args(), t0, t1);
-            }
+            k_fused<ND, R, G, CT><<<g, B, SMEM, stream>>>(args(), t0, t1);
         }
     }
 

@@ -88,24 +88,30 @@ __host__ __device__ constexpr bool carries()
     return CellT<CT>::SIMPLEX;
 }
 
-// Resident blocks of `block` threads to ask of the compiler for a fused
-// kernel whose cells carry (0: keep the one-argument launch bound), from the
-// registers per thread that were fastest with what the kernel stages (Stage).
-// FP32 form, 2M triangles: 156 us per launch at 112 registers, 233 at 96 and
-// 252 at 80 (spills); fp32-geom32: 136 at 80, 138 at 96, 149 at 128.
-// Tetrahedra: 245 us per 1.3M at 128, 246 at 96.
+// Resident blocks of BLOCK threads to ask of the compiler for the fused kernel
+// of cell type CT (0: any mix), from the registers per thread that were fastest
+// with what the kernel stages (Stage); 0 keeps the one-argument launch bound.
+// Per launch, at BLOCK = 128:
+//  FP32 form, 2M triangles 156 us at 112 registers, 233 at 96 (spills);
+//  fp32-geom32 136 at 80, 138 at 96, 149 at 128.  1.3M tetrahedra 245 us at 128,
+//  246 at 96.  490k quadrilaterals 58.7 / 55.7 us (FP32 form / fp32-geom32) at
+//  112, 60.9 / 54.3 at 96, 64.8 / 55.4 at 80.  176k hexahedra 82 us at 168, 90 at
+//  128, 98 at 254.  Any mix: 176k hexahedra 99 us at 168, 105 at 128, 118 at the
+//  243 that the compiler takes; 490k quadrilaterals 62 at 96, 66 at its 126.
+//  FP64: at its 255 registers 8 warps per SM are too few to keep the FP64 pipes
+//  fed through their loads, and a spilling kernel of more warps is faster: 343k
+//  hexahedra 1,948 us at 255, 1,780 at 168, 1,717 at 128; 54k prisms (any mix)
+//  277, 223, 250.  Triangles, tetrahedra and quadrilaterals gain nothing.
 template <int ND, typename R, int CT, int BLOCK, typename G = R>
 __host__ __device__ constexpr int min_blocks()
 {
-    if constexpr (sizeof(R) == 8 || !carries<CT>())
-    {
-        return 0;
-    }
-    else
-    {
-        constexpr int regs = ND == 3 ? 128 : (Geo<ND, G>::MID ? 80 : 112);
-        return 65536 / (BLOCK * regs);
-    }
+    constexpr int regs = sizeof(R) == 8 ? (CT == 5 ? 128 : (CT == 0 && ND == 3 ? 168 : 0))
+                         : CT == 0      ? (ND == 2 ? 96 : 168)
+                         : CT == 5      ? 168
+                         : CT == 6      ? 128
+                         : CT == 3      ? (Geo<ND, G>::MID ? 96 : 112)
+                                        : (Geo<ND, G>::MID ? 80 : 112);
+    return regs > 0 ? 65536 / (BLOCK * regs) : 0;
 }
 
 template <int ND, int NFC, typename R>
