@@ -111,6 +111,12 @@ __global__ void k_inv_spacing(double const * coord, int64_t n, double hdt, doubl
 // requires.
 __device__ __forceinline__ double fm(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ double mu(double a, double b) { return __dmul_rn(a, b); }
+// The same product by either pipe (mul_int's bits are the multiplication's).
+template <bool INT>
+__device__ __forceinline__ double mu(double a, double b)
+{
+    return INT ? scg::dev::mul_int(a, b) : __dmul_rn(a, b);
+}
 __device__ __forceinline__ double ad(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double sb(double a, double b) { return __dsub_rn(a, b); }
 
@@ -198,12 +204,13 @@ struct K1D
 
 // The W-alpha gradient (march_half_so1_alpha, Euler1DCore.hpp:284-320); for
 // alpha = 2 its numerator duxp^2 duxn + duxn^2 duxp is duxn duxp (duxn + duxp).
+template <bool INT>
 __device__ __forceinline__ double wgrad(int alpha, double duxn, double duxp)
 {
     double num, den;
     if (alpha == 2)
     {
-        num = mu(mu(duxn, duxp), ad(duxn, duxp));
+        num = mu<INT>(mu<INT>(duxn, duxp), ad(duxn, duxp));
         den = fm(duxn, duxn, fm(duxp, duxp, Tiny1D<double>::V));
     }
     else
@@ -211,7 +218,7 @@ __device__ __forceinline__ double wgrad(int alpha, double duxn, double duxp)
         num = fm(fabs(duxp), duxn, mu(fabs(duxn), duxp));
         den = ad(ad(fabs(duxp), fabs(duxn)), Tiny1D<double>::V);
     }
-    return mu(num, scg::dev::recip(den));
+    return mu<INT>(num, scg::dev::recip(den));
 }
 
 // What a half step does (its mask): so0, cfl, the copy-out boundary
@@ -227,6 +234,7 @@ constexpr unsigned h_alpha(int alpha) { return static_cast<unsigned>(alpha) << 8
 // one in 32 at the seams.
 constexpr int WOUT = 31; // outputs per warp
 
+template <bool INT>
 __device__ __forceinline__ void half_warp(E1DArgs const & a, int64_t start, int64_t nout, unsigned mask, int64_t w)
 {
     int const alpha = static_cast<int>(mask >> 8);
@@ -251,7 +259,7 @@ __device__ __forceinline__ void half_warp(E1DArgs const & a, int64_t start, int6
             double const idx = a.invd2[ic];
             for (int i = 0; i < 3; ++i)
             {
-                v[i] = mu(ad(k.ll[i], lr[i]), idx);
+                v[i] = mu<INT>(ad(k.ll[i], lr[i]), idx);
                 a.so0[(ic + 1) * 3 + i] = v[i];
             }
         }
@@ -271,7 +279,8 @@ __device__ __forceinline__ void half_warp(E1DArgs const & a, int64_t start, int6
             double const idn = a.invdx[ic];
             for (int i = 0; i < 3; ++i)
             {
-                a.so1[(ic + 1) * 3 + i] = wgrad(alpha, mu(sb(v[i], k.up[i]), idn), mu(sb(up[i], v[i]), idp));
+                a.so1[(ic + 1) * 3 + i] =
+                    wgrad<INT>(alpha, mu<INT>(sb(v[i], k.up[i]), idn), mu<INT>(sb(up[i], v[i]), idp));
             }
         }
     }
@@ -293,12 +302,13 @@ __device__ __forceinline__ void copy_out(E1DArgs const & a)
 
 // One half step: so0, cfl and so1 at one parity and the boundary treatment, as
 // the mask asks.
+template <bool INT>
 __global__ void __launch_bounds__(128) k_half(E1DArgs a, int64_t start, int64_t nout, unsigned mask)
 {
     int64_t const w = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / 32;
     if (w * WOUT < nout)
     {
-        half_warp(a, start, nout, mask, w);
+        half_warp<INT>(a, start, nout, mask, w);
     }
     if ((mask & H_BND) && blockIdx.x == 0 && threadIdx.x == 0)
     {
@@ -373,7 +383,7 @@ __global__ void __launch_bounds__(32 * TUBE_WARPS64) k_tube(E1DArgs a, int alpha
                 for (int i = 0; i < 3; ++i)
                 {
                     uo[i] = mu(ad(c.ll[i], w[i]), de);
-                    xo[i] = wgrad(alpha, mu(sb(uo[i], c.up[i]), ie), mu(sb(w[3 + i], uo[i]), io));
+                    xo[i] = wgrad<false>(alpha, mu(sb(uo[i], c.up[i]), ie), mu(sb(w[3 + i], uo[i]), io));
                 }
                 if (end)
                 {
@@ -393,7 +403,7 @@ __global__ void __launch_bounds__(32 * TUBE_WARPS64) k_tube(E1DArgs a, int alpha
                 for (int i = 0; i < 3; ++i)
                 {
                     ue[i] = mu(ad(w[i], c.lr[i]), dl);
-                    xe[i] = wgrad(alpha, mu(sb(ue[i], w[3 + i]), il), mu(sb(c.up[i], ue[i]), ie));
+                    xe[i] = wgrad<false>(alpha, mu(sb(ue[i], w[3 + i]), il), mu(sb(c.up[i], ue[i]), ie));
                 }
             }
             if (end && t < nout2)
@@ -453,6 +463,12 @@ struct Euler1DBase
     int precision = SCG_FP64;
     cudaStream_t stream = nullptr;
 };
+
+// Tubes above this many points take 18 of a point's FP64 multiplications on the
+// integer pipe (half_warp's INT, the same bits): there the FP64 pipes are full
+// (2M points 214.6 -> 160.9 us per half step, 100,001 points 12.7 -> 12.1), below
+// the longer chain of instructions shows (20,001 points 6.4 -> 8.0).
+constexpr int64_t INT_POINTS64 = 60000;
 
 // The FP64 core: the reference's arithmetic on the reference's [n][3] device
 // tables.  The FP32 core is Euler1D32 below.
@@ -593,7 +609,15 @@ public:
         // SMs as it has warps; beyond that blocks of four.
         int64_t const warps = std::max<int64_t>((nout + WOUT - 1) / WOUT, 1);
         int const wpb = warps <= 152 * 32 ? 1 : 4;
-        k_half<<<static_cast<unsigned>((warps + wpb - 1) / wpb), 32 * wpb, 0, stream>>>(args(), start, nout, mask);
+        unsigned const grid = static_cast<unsigned>((warps + wpb - 1) / wpb);
+        if (n > INT_POINTS64)
+        {
+            k_half<true><<<grid, 32 * wpb, 0, stream>>>(args(), start, nout, mask);
+        }
+        else
+        {
+            k_half<false><<<grid, 32 * wpb, 0, stream>>>(args(), start, nout, mask);
+        }
         scg::launched(stream, "e1d_half");
     }
 

@@ -68,6 +68,13 @@ enum
     G_COUNT
 };
 
+__device__ __forceinline__ double mu(double a, double b) { return __dmul_rn(a, b); }
+// The same product by either pipe (mul_int's bits are the multiplication's).
+template <bool INT>
+__device__ __forceinline__ double mu(double a, double b)
+{
+    return INT ? scg::dev::mul_int(a, b) : __dmul_rn(a, b);
+}
 __device__ __forceinline__ double rcp_bits(double d)
 {
     return __longlong_as_double(static_cast<long long>(scg::dev::rcp_fix(d)));
@@ -124,37 +131,37 @@ struct SelmGrid
 // side of it use (LinearScalarSelm / InviscidBurgersSelm, xn, xp, tp, so0p):
 // ll = xp + tp (to the element on its right), ur = xn - tp (to the element on
 // its left) and the value so0p at the next time level.
-template <int KIND>
+template <int KIND, bool INT>
 struct SelmParts
 {
     double ll, ur, so0p;
 
     __device__ __forceinline__ SelmParts(STArgs const & a, double u, double ux, SelmGrid const & x)
     {
-        double const disp = x.disp;
-        double const xn = x.dxneg * (u + x.dmneg * ux);
-        double const xp = x.dxpos * (u + x.dmpos * ux);
+        double const dux = mu<INT>(x.disp, ux);
+        double const xn = mu(x.dxneg, u + mu(x.dmneg, ux));
+        double const xp = mu(x.dxpos, u + mu(x.dmpos, ux));
         double tp;
         if constexpr (KIND == 0)
         {
             double r = u;
-            r += disp * ux;
-            r -= a.qdt * ux;
-            tp = a.hdt * r;
+            r += dux;
+            r -= mu<INT>(a.qdt, ux);
+            tp = mu(a.hdt, r);
         }
         else
         {
-            double const u2 = u * u;
-            double r = 0.5 * u2;
-            r += disp * u * ux;
-            r -= a.qdt * u2 * ux;
-            tp = a.hdt * r;
+            double const u2 = mu(u, u);
+            double r = mu(0.5, u2);
+            r += mu(mu(x.disp, u), ux);
+            r -= mu(mu(a.qdt, u2), ux);
+            tp = mu(a.hdt, r);
         }
         ll = xp + tp;
         ur = xn - tp;
         double q = u;
-        q += disp * ux;
-        q -= a.hdt * ux;
+        q += dux;
+        q -= mu<INT>(a.hdt, ux);
         so0p = q;
     }
 };
@@ -181,17 +188,17 @@ __device__ __forceinline__ double cfl_at(STArgs const & a, int64_t xi, double u)
         return div_bits(fabs(u) * a.hdt, gq(a, G_HDX, xi), gq(a, G_RHDX, xi));
 }
 
-template <int ALPHA>
+template <int ALPHA, bool INT>
 __device__ __forceinline__ double wgrad(double duxn, double duxp)
 {
     double fan = fabs(duxn), fap = fabs(duxp);
     if constexpr (ALPHA == 2)
     {
-        fan *= fan;
-        fap *= fap;
+        fan = mu<INT>(fan, fan);
+        fap = mu<INT>(fap, fap);
     }
     double const den = fap + fan + DBL_MIN;
-    return scg::dev::div_fix(fap * duxn + fan * duxp, den, scg::dev::rcp_fix(den));
+    return scg::dev::div_fix(mu<INT>(fap, duxn) + mu<INT>(fan, duxp), den, scg::dev::rcp_fix(den));
 }
 
 constexpr int WOUT = 31; // conservation elements per warp
@@ -201,7 +208,7 @@ constexpr int WOUT = 31; // conservation elements per warp
 // parts of the lower-left solution element of conservation element
 // ic = 31 w + l - odd; lanes 0 .. 30 form the element's top from those and the
 // next lane's, by shuffles: warps share nothing.
-template <int KIND, int ALPHA, int STAGE>
+template <int KIND, int ALPHA, int STAGE, bool INT>
 __global__ void __launch_bounds__(128) k_st_half(STArgs a, int odd)
 {
     int const lane = static_cast<int>(threadIdx.x) & 31;
@@ -215,7 +222,7 @@ __global__ void __launch_bounds__(128) k_st_half(STArgs a, int odd)
     // element of conservation element ncelm - 1); lanes past it repeat it.
     int64_t const ic = first + lane < a.ncelm ? first + lane : a.ncelm;
     int64_t const xi = 2 + 2 * ic + odd;
-    SelmParts<KIND> const sn(a, a.so0[xi], a.so1[xi], SelmGrid(a, xi));
+    SelmParts<KIND, INT> const sn(a, a.so0[xi], a.so1[xi], SelmGrid(a, xi));
     double const ur = __shfl_down_sync(0xffffffffu, sn.ur, 1);
     double const so0p = __shfl_down_sync(0xffffffffu, sn.so0p, 1);
     if (lane >= WOUT || ic >= a.ncelm)
@@ -256,7 +263,7 @@ __global__ void __launch_bounds__(128) k_st_half(STArgs a, int odd)
     {
         double const duxn = div_bits(utp - sn.so0p, gq(a, G_DXPOS, xi), gq(a, G_RDXPOS, xi));
         double const duxp = div_bits(so0p - utp, gq(a, G_DXNEG, xi + 2), gq(a, G_RDXNEG, xi + 2));
-        double const g = wgrad<ALPHA>(duxn, duxp);
+        double const g = wgrad<ALPHA, INT>(duxn, duxp);
         a.so1[xt] = g;
         if (STAGE & 8)
         {
@@ -306,14 +313,14 @@ __global__ void __launch_bounds__(32 * ST_WARPS) k_st_cluster(STArgs a, int64_t 
     {
         bool const end = s + 1 == steps;
         {
-            SelmParts<KIND> const p(a, ue, xe, ge);
+            SelmParts<KIND, false> const p(a, ue, xe, ge);
             double const v[2] = {p.ur, p.so0p};
             double w[2];
             hand_over<2, 1>(v, w, slots[0]);
             if (out1)
             {
                 uo = div_bits(p.ll + w[0], wide_o, rwide_o);
-                xo = wgrad<ALPHA>(div_bits(uo - p.so0p, ge.dxpos, rpe), div_bits(w[1] - uo, dne, rne));
+                xo = wgrad<ALPHA, false>(div_bits(uo - p.so0p, ge.dxpos, rpe), div_bits(w[1] - uo, dne, rne));
                 if (t == a.ncelm)
                 {
                     slot_put(to_lo, uo);
@@ -342,14 +349,14 @@ __global__ void __launch_bounds__(32 * ST_WARPS) k_st_cluster(STArgs a, int64_t 
             }
         }
         {
-            SelmParts<KIND> const p(a, uo, xo, go);
+            SelmParts<KIND, false> const p(a, uo, xo, go);
             double const v[2] = {p.ll, p.so0p};
             double w[2];
             hand_over<2, 0>(v, w, slots[1]);
             if (out2)
             {
                 ue = div_bits(w[0] + p.ur, wide_e, rwide_e);
-                xe = wgrad<ALPHA>(div_bits(ue - w[1], dpo, rpo), div_bits(p.so0p - ue, go.dxneg, rno));
+                xe = wgrad<ALPHA, false>(div_bits(ue - w[1], dpo, rpo), div_bits(p.so0p - ue, go.dxneg, rno));
                 if (end)
                 {
                     a.cfl[e] = cfl_at<KIND>(a, e, ue);
@@ -391,6 +398,12 @@ __global__ void k_st_bnd(STArgs a, int which)
     s[1] = right_in;
     s[last + 2] = left_in;
 }
+
+// Grids above this many elements take 7 of an element's FP64 multiplications on
+// the integer pipe (k_st_half's INT, the same bits), where the FP64 pipes are
+// full (1M elements, linear 54.0 -> 49.3 us per half step, Burgers 67.9 -> 61.2;
+// 100,000 elements 7.6 -> 7.3).
+constexpr int64_t INT_ELEMENTS = 80000;
 
 class Spacetime
 {
@@ -490,20 +503,13 @@ public:
         int const wpb = warps <= 152 * 32 ? 1 : 4;
         unsigned const grid = static_cast<unsigned>((warps + wpb - 1) / wpb);
         int const threads = 32 * wpb;
-        if (kind == 0)
-        {
-            if (alpha == 1)
-                k_st_half<0, 1, STAGE><<<grid, threads, 0, stream>>>(args(), odd);
-            else
-                k_st_half<0, 2, STAGE><<<grid, threads, 0, stream>>>(args(), odd);
-        }
-        else
-        {
-            if (alpha == 1)
-                k_st_half<1, 1, STAGE><<<grid, threads, 0, stream>>>(args(), odd);
-            else
-                k_st_half<1, 2, STAGE><<<grid, threads, 0, stream>>>(args(), odd);
-        }
+        bool const big = ncelm > INT_ELEMENTS;
+        auto * const kernel =
+            kind == 0 ? (alpha == 1 ? (big ? k_st_half<0, 1, STAGE, true> : k_st_half<0, 1, STAGE, false>)
+                                    : (big ? k_st_half<0, 2, STAGE, true> : k_st_half<0, 2, STAGE, false>))
+                      : (alpha == 1 ? (big ? k_st_half<1, 1, STAGE, true> : k_st_half<1, 1, STAGE, false>)
+                                    : (big ? k_st_half<1, 2, STAGE, true> : k_st_half<1, 2, STAGE, false>));
+        kernel<<<grid, threads, 0, stream>>>(args(), odd);
         scg::launched(stream, "spacetime_half");
     }
 
@@ -682,6 +688,16 @@ __global__ void k_root_check(double const * x, double * r, double * s, int64_t n
     }
 }
 
+// The integer pipe's product of a and b.
+__global__ void k_product_check(double const * a, double const * b, double * p, int64_t n)
+{
+    int64_t const i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i < n)
+    {
+        p[i] = scg::dev::mul_int(a[i], b[i]);
+    }
+}
+
 } // namespace
 
 struct scg_st
@@ -794,6 +810,27 @@ int scg_root_check(const double * x, double * r, double * s, int64_t n)
         scg::launched(nullptr, "root_check");
         scg::cuda_check(cudaMemcpy(r, dr.ptr, dr.bytes(), cudaMemcpyDeviceToHost), "D2H");
         scg::cuda_check(cudaMemcpy(s, ds.ptr, ds.bytes(), cudaMemcpyDeviceToHost), "D2H");
+    });
+}
+
+int scg_product_check(const double * a, const double * b, double * p, int64_t n)
+{
+    return scg::guarded([&] {
+        if (n < 0 || (n > 0 && (!a || !b || !p)))
+        {
+            throw std::invalid_argument("scg_product_check: null buffer or negative count");
+        }
+        if (n == 0)
+        {
+            return;
+        }
+        size_t const sz = static_cast<size_t>(n);
+        scg::DevBuf<double> da(sz), db(sz), dp(sz);
+        scg::cuda_check(cudaMemcpy(da.ptr, a, da.bytes(), cudaMemcpyHostToDevice), "H2D");
+        scg::cuda_check(cudaMemcpy(db.ptr, b, db.bytes(), cudaMemcpyHostToDevice), "H2D");
+        k_product_check<<<static_cast<unsigned>((n + 255) / 256), 256>>>(da.ptr, db.ptr, dp.ptr, n);
+        scg::launched(nullptr, "product_check");
+        scg::cuda_check(cudaMemcpy(p, dp.ptr, dp.bytes(), cudaMemcpyDeviceToHost), "D2H");
     });
 }
 
