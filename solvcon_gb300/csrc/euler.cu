@@ -1537,6 +1537,14 @@ public:
         }
     }
 
+    // FP64 meshes up to this many cells march with several lanes per cell
+    // (k_fused_split), larger ones with one.  Per substep, one lane -> several:
+    // 1,024 triangles 33.7 -> 16.6 us (up to 4,000 the same), 8,192 30.9 ->
+    // 21.3, 12,800 30.9 -> 28.9, 20,000 37.6 -> 41.2; 1,024 quadrilaterals 41.2 ->
+    // 20.7, 10,000 42.0 -> 33.0; 2,058 tetrahedra 57.6 -> 28.9, 4,374 57.6 -> 43.2,
+    // 7,986 59.5 -> 79.4; 512 hexahedra 111 -> 45, 2,744 121 -> 56, 5,832 122 -> 124.
+    static constexpr int64_t SPLIT_CELLS = ND == 2 ? 12800 : 5200;
+
     // The fused kernel over rows [t0, t1) of its work order (body cells, then
     // ghost rows): the one compiled for the mesh's cell type when it has only
     // triangles, tetrahedra, hexahedra or (FP32) quadrilaterals, else the one
@@ -1550,6 +1558,15 @@ public:
         if (t1 <= t0)
         {
             return;
+        }
+        if constexpr (sizeof(R) == 8)
+        {
+            if (t0 == 0 && t1 >= ncell && ncell <= SPLIT_CELLS)
+            {
+                int64_t const n = ncell * Split<ND>::LPC + t1 - ncell;
+                k_fused_split<ND><<<static_cast<unsigned>((n + 31) / 32), 32, 0, stream>>>(args(), t1);
+                return;
+            }
         }
         constexpr int SIMPLEX = ND == 2 ? CT_TRIANGLE : CT_TET;
         constexpr int BOX = ND == 2 ? CT_QUAD : CT_HEX;

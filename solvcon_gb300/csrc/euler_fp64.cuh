@@ -408,14 +408,57 @@ __device__ __forceinline__ double cap64(double * w, double acfl, double sigma0, 
     return mu(fire ? nn : sigma0, recip(fire ? dd : cw));
 }
 
+// What calc_dsoln reads of a neighbour's record for equations q .. q + E - 1:
+// their so0 and so0t (u, t) and gradients (g).
+template <int ND, int E>
+struct RowPart
+{
+    double u[E], t[E], g[E * ND];
+
+    __device__ __forceinline__ RowPart(double const * base, int q)
+    {
+        constexpr int NEQ = ND + 2;
+        if constexpr (E == NEQ)
+        {
+            double rec[Rec<ND, double>::NUSED + 1];
+            load_part<0, Rec<ND, double>::NUSED>(base, rec);
+#pragma unroll
+            for (int i = 0; i < NEQ; ++i)
+            {
+                u[i] = rec[i];
+                t[i] = rec[NEQ + i];
+            }
+#pragma unroll
+            for (int k = 0; k < NEQ * ND; ++k)
+            {
+                g[k] = rec[2 * NEQ + k];
+            }
+        }
+        else
+        {
+#pragma unroll
+            for (int i = 0; i < E; ++i)
+            {
+                u[i] = __ldg(base + q + i);
+                t[i] = __ldg(base + NEQ + q + i);
+            }
+#pragma unroll
+            for (int k = 0; k < E * ND; ++k)
+            {
+                g[k] = __ldg(base + 2 * NEQ + q * ND + k);
+            }
+        }
+    }
+};
+
 // calc_dsoln of one body cell (euler_gradient.cpp:23-130 with the gradient
-// element of GradientElement.cpp:137-290): a triangle or tetrahedron.
-template <int CT>
-__device__ __forceinline__ void dsoln64_simplex(MarchArgs<double, double> const & a, int64_t icl, double const * so0n,
-                                                double cflc, double * so1n)
+// element of GradientElement.cpp:137-290) for equations q .. q + E - 1 (so0n
+// and so1n: theirs): a triangle or tetrahedron.  Returns their firing bits.
+template <int CT, int E>
+__device__ __forceinline__ unsigned dsoln64_simplex(MarchArgs<double, double> const & a, int64_t icl, int q,
+                                                    double const * so0n, double cflc, double * so1n)
 {
     constexpr int ND = CellT<CT>::ND;
-    constexpr int NEQ = ND + 2;
     constexpr int N = ND + 1; // faces, and gradient elements
     using D = Geo<ND, double>;
     using RC = Rec<ND, double>;
@@ -424,14 +467,13 @@ __device__ __forceinline__ void dsoln64_simplex(MarchArgs<double, double> const 
     GeoView<double> const gv = geo_view(a, icl);
     // Solution deltas at the evaluation points: of the first ND faces, and
     // their sum over all.
-    double uf[ND][NEQ], us[NEQ];
+    double uf[ND][E], us[E];
     double x[ND][ND]; // displacements of the first ND faces
 #pragma unroll
     for (int f = 0; f < N; ++f)
     {
         int64_t const jr = __ldg(a.nbr + f * a.ncell + icl);
-        double rec[RC::NUSED + 1];
-        load_part<0, RC::NUSED>(a.cur + jr * RC::RS, rec);
+        RowPart<ND, E> const r(a.cur + jr * RC::RS, q);
         double jd[ND];
 #pragma unroll
         for (int d = 0; d < ND; ++d)
@@ -444,13 +486,13 @@ __device__ __forceinline__ void dsoln64_simplex(MarchArgs<double, double> const 
             }
         }
 #pragma unroll
-        for (int i = 0; i < NEQ; ++i)
+        for (int i = 0; i < E; ++i)
         {
-            double s = sb(fm(a.hdt, rec[NEQ + i], rec[i]), so0n[i]);
+            double s = sb(fm(a.hdt, r.t[i], r.u[i]), so0n[i]);
 #pragma unroll
             for (int d = 0; d < ND; ++d)
             {
-                s = fm(jd[d], rec[2 * NEQ + i * ND + d], s);
+                s = fm(jd[d], r.g[i * ND + d], s);
             }
             if (f < ND)
             {
@@ -491,9 +533,9 @@ __device__ __forceinline__ void dsoln64_simplex(MarchArgs<double, double> const 
             }
         }
     }
-    uint8_t fired = 0;
+    unsigned fired = 0;
 #pragma unroll
-    for (int i = 0; i < NEQ; ++i)
+    for (int i = 0; i < E; ++i)
     {
         // Element m < ND leaves out face m, element ND the last face.
         double g[ND], w[N];
@@ -525,7 +567,7 @@ __device__ __forceinline__ void dsoln64_simplex(MarchArgs<double, double> const 
         }
         bool fire;
         double const cc = cap64<N>(w, acfl, a.sigma0, fire);
-        fired |= fire ? static_cast<uint8_t>(1u << i) : uint8_t(0);
+        fired |= fire ? 1u << (q + i) : 0u;
         // sum_k (1/n + cc u_k) g_k, the weights summing to one.
 #pragma unroll
         for (int m = 0; m < ND; ++m)
@@ -543,10 +585,7 @@ __device__ __forceinline__ void dsoln64_simplex(MarchArgs<double, double> const 
             so1n[i * ND + d] = g[d];
         }
     }
-    if (a.limiter)
-    {
-        a.limiter[icl] = fired;
-    }
+    return fired;
 }
 
 // a x b, from the stored product of the lower- and higher-numbered face: each
@@ -608,13 +647,12 @@ __device__ __forceinline__ void dets64(double const x[][CellT<CT>::ND], FacePair
     }
 }
 
-// calc_dsoln of one body cell that is no simplex.
-template <int CT>
-__device__ __forceinline__ void dsoln64_general(MarchArgs<double, double> const & a, int64_t icl, double const * so0n,
-                                                double cflc, double * so1n)
+// calc_dsoln of one body cell that is no simplex, for equations q .. q + E - 1.
+template <int CT, int E>
+__device__ __forceinline__ unsigned dsoln64_general(MarchArgs<double, double> const & a, int64_t icl, int q,
+                                                    double const * so0n, double cflc, double * so1n)
 {
     constexpr int ND = CellT<CT>::ND;
-    constexpr int NEQ = ND + 2;
     constexpr int NFC = CellT<CT>::NFC;
     constexpr int NFGE = CellT<CT>::NFGE;
     using D = Geo<ND, double>;
@@ -684,13 +722,12 @@ __device__ __forceinline__ void dsoln64_general(MarchArgs<double, double> const 
         }
     }
     // Solution deltas at the evaluation points.
-    double uf[NFC][NEQ];
+    double uf[NFC][E];
 #pragma unroll
     for (int f = 0; f < NFC; ++f)
     {
         int64_t const jr = __ldg(a.nbr + f * a.ncell + icl);
-        double rec[RC::NUSED + 1];
-        load_part<0, RC::NUSED>(a.cur + jr * RC::RS, rec);
+        RowPart<ND, E> const r(a.cur + jr * RC::RS, q);
         double jd[ND];
 #pragma unroll
         for (int d = 0; d < ND; ++d)
@@ -698,13 +735,13 @@ __device__ __forceinline__ void dsoln64_general(MarchArgs<double, double> const 
             jd[d] = sb(fm(tau, fg<ND>(gv, f, D::K_Q + d), fg<ND>(gv, f, D::K_R + d)), delta[d]);
         }
 #pragma unroll
-        for (int i = 0; i < NEQ; ++i)
+        for (int i = 0; i < E; ++i)
         {
-            double s = sb(fm(a.hdt, rec[NEQ + i], rec[i]), so0n[i]);
+            double s = sb(fm(a.hdt, r.t[i], r.u[i]), so0n[i]);
 #pragma unroll
             for (int d = 0; d < ND; ++d)
             {
-                s = fm(jd[d], rec[2 * NEQ + i * ND + d], s);
+                s = fm(jd[d], r.g[i * ND + d], s);
             }
             uf[f][i] = s;
         }
@@ -737,9 +774,9 @@ __device__ __forceinline__ void dsoln64_general(MarchArgs<double, double> const 
             }
         }
     }
-    uint8_t fired = 0;
+    unsigned fired = 0;
 #pragma unroll
-    for (int i = 0; i < NEQ; ++i)
+    for (int i = 0; i < E; ++i)
     {
         double g[NFGE][ND], w[NFGE];
 #pragma unroll
@@ -762,7 +799,7 @@ __device__ __forceinline__ void dsoln64_general(MarchArgs<double, double> const 
         }
         bool fire;
         double const cc = cap64<NFGE>(w, acfl, a.sigma0, fire);
-        fired |= fire ? static_cast<uint8_t>(1u << i) : uint8_t(0);
+        fired |= fire ? 1u << (q + i) : 0u;
 #pragma unroll
         for (int d = 0; d < ND; ++d)
         {
@@ -775,9 +812,20 @@ __device__ __forceinline__ void dsoln64_general(MarchArgs<double, double> const 
             so1n[i * ND + d] = s;
         }
     }
-    if (a.limiter)
+    return fired;
+}
+
+template <int CT, int E>
+__device__ __forceinline__ unsigned dsoln64_part(MarchArgs<double, double> const & a, int64_t icl, int q,
+                                                 double const * so0n, double cflc, double * so1n)
+{
+    if constexpr (CellT<CT>::SIMPLEX)
     {
-        a.limiter[icl] = fired;
+        return dsoln64_simplex<CT, E>(a, icl, q, so0n, cflc, so1n);
+    }
+    else
+    {
+        return dsoln64_general<CT, E>(a, icl, q, so0n, cflc, so1n);
     }
 }
 
@@ -785,14 +833,77 @@ template <int CT>
 __device__ __forceinline__ void dsoln64(MarchArgs<double, double> const & a, int64_t icl, double const * so0n,
                                         double cflc, double * so1n)
 {
-    if constexpr (CellT<CT>::SIMPLEX)
+    unsigned const fired = dsoln64_part<CT, CellT<CT>::ND + 2>(a, icl, 0, so0n, cflc, so1n);
+    if (a.limiter)
     {
-        dsoln64_simplex<CT>(a, icl, so0n, cflc, so1n);
+        a.limiter[icl] = static_cast<uint8_t>(fired);
     }
-    else
+}
+
+// ---------------------------------------------------------------------------
+// One substep of a cell by LPC lanes, one equation each, for meshes too small to
+// fill the GPU.  An FP64 instruction takes a warp 64 cycles however many of its
+// lanes work, on its SM sub-partition's pipe, and the GPU has 608 of those: a
+// thousand cells at a thread each are 32 warps in which hundreds of
+// instructions follow one another.  Lane q takes equation q of calc_soln and
+// calc_dsoln; what all equations share (the gradient elements' geometry, the CFL
+// number, the flux terms) every lane forms for itself; the lanes of the faces
+// 0, 1, ... do the boundary work.  The operations and their order are those of
+// the one-thread routines, so the results are the same bits.
+template <int ND>
+struct Split
+{
+    static constexpr int LPC = ND == 2 ? 4 : 8; // lanes per cell (equations 0 .. NEQ - 1, the rest repeat the last)
+};
+
+// Equation q of calc_soln (soln64<CT, true>).
+template <int CT>
+__device__ __forceinline__ double soln64_eq(MarchArgs<double, double> const & a, int64_t icl, int q)
+{
+    constexpr int ND = CellT<CT>::ND;
+    constexpr int NEQ = ND + 2;
+    using D = Geo<ND, double>;
+    using RC = Rec<ND, double>;
+    using F = FluxTerms<ND>;
+    GeoView<double> const gv = geo_view(a, icl);
+    // Where the record keeps this equation's A_d and B_{d,e}.
+    int oa[ND], ob[ND];
+#pragma unroll
+    for (int d = 0; d < ND; ++d)
     {
-        dsoln64_general<CT>(a, icl, so0n, cflc, so1n);
+        int const k = q - 1;
+        int const lo = k < d ? k : d, hi = k < d ? d : k;
+        int const sym = lo * ND - lo * (lo - 1) / 2 + hi - lo;
+        oa[d] = RC::OP + (q == 0 ? F::A0 + d : (q == NEQ - 1 ? F::AE + d : F::AM + sym));
+        ob[d] = q == 0 ? 2 * NEQ + (1 + d) * ND : RC::OP + (q == NEQ - 1 ? F::BE + d * ND : F::BM + sym * ND);
     }
+    double acc = 0.0;
+#pragma unroll
+    for (int f = 0; f < CellT<CT>::NFC; ++f)
+    {
+        int64_t const jr = __ldg(a.nbr + f * a.ncell + icl);
+        double const * const base = a.cur + jr * RC::RS;
+        double const bvol = fg<ND>(gv, f, D::K_BVOL);
+        double const u = __ldg(base + q);
+        acc = f == 0 ? mu(bvol, u) : fm(bvol, u, acc);
+#pragma unroll
+        for (int d = 0; d < ND; ++d)
+        {
+            double const vb = fg<ND>(gv, f, D::K_DB + d);
+            double const nh = fg<ND>(gv, f, D::K_NH + d);
+            acc = fm(-__ldg(base + oa[d]), nh, fm(vb, __ldg(base + 2 * NEQ + q * ND + d), acc));
+        }
+#pragma unroll
+        for (int e = 0; e < ND; ++e)
+        {
+#pragma unroll
+            for (int d = 0; d < ND; ++d)
+            {
+                acc = fm(-__ldg(base + ob[d] + e), fg<ND>(gv, f, D::K_MH + e * ND + d), acc);
+            }
+        }
+    }
+    return mu(acc, cg<ND>(gv, 0));
 }
 
 } // namespace dev

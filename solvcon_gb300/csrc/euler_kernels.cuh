@@ -1172,6 +1172,28 @@ __device__ __forceinline__ void fused_cell(MarchArgs<R, G> const & a, GeoView<G,
     out.store(so0n, so0t, so1n);
 }
 
+// The FP64 ghost row jr of a body cell's boundary face: bc_soln from the cell's
+// so0n (before calc_cfl's rewrite), bc_dsoln from its so1c, and calc_solt of the
+// next substep.
+template <int ND>
+__device__ __forceinline__ void ghost64(MarchArgs<double, double> const & a, int64_t jr, int64_t row,
+                                        double const * so0n)
+{
+    constexpr int NEQ = ND + 2;
+    using RC = Rec<ND, double>;
+    int const kind = a.gkind[jr];
+    if (kind >= 0)
+    {
+        double own[RC::NUSED + 1], g0[NEQ], g1[NEQ * ND], gt[NEQ], gc[FluxTerms<ND>::N];
+        load_part<2 * NEQ, RC::NUSED>(a.cur + row * RC::RS, own);
+        bc0_ghost<ND, double>(kind, a.gnml + jr * ND, a.gval + jr * NEQ, so0n, g0);
+        bc1_ghost<ND, double>(kind, a.gnml + jr * ND, own + 2 * NEQ, g1);
+        solt_terms<ND>(g0, g1, ldg(a.gamma + jr), a.qdt, gt, gc);
+        store_row<ND>(a.nxt + jr * RC::RS, g0, gt, g1, gc);
+        deliver_row<ND>(a, jr, g0, g1);
+    }
+}
+
 // The same in FP64 (euler_fp64.cuh); the new state is returned too.
 template <int CT>
 __device__ __forceinline__ void fused_cell64(MarchArgs<double, double> const & a, int64_t icl, double * so0n,
@@ -1190,17 +1212,7 @@ __device__ __forceinline__ void fused_cell64(MarchArgs<double, double> const & a
         int64_t const jr = ldg(a.nbr + f * a.ncell + icl);
         if (jr < a.ngst)
         {
-            int const kind = a.gkind[jr];
-            if (kind >= 0)
-            {
-                double own[RC::NUSED + 1], g0[NEQ], g1[NEQ * ND], gt[NEQ], gc[F::N];
-                load_part<2 * NEQ, RC::NUSED>(a.cur + row * RC::RS, own);
-                bc0_ghost<ND, double>(kind, a.gnml + jr * ND, a.gval + jr * NEQ, so0n, g0);
-                bc1_ghost<ND, double>(kind, a.gnml + jr * ND, own + 2 * NEQ, g1);
-                solt_terms<ND>(g0, g1, ldg(a.gamma + jr), a.qdt, gt, gc);
-                store_row<ND>(a.nxt + jr * RC::RS, g0, gt, g1, gc);
-                deliver_row<ND>(a, jr, g0, g1);
-            }
+            ghost64<ND>(a, jr, row, so0n);
         }
     }
     double rinv;
@@ -1326,6 +1338,28 @@ __device__ __forceinline__ void staged_cell(MarchArgs<float, G> const & a, int64
     }
 }
 
+// A ghost row without a boundary condition keeps its stale state; its next so0t
+// is still the Jacobian product of that state.
+template <int ND>
+__device__ __forceinline__ void stale_ghost64(MarchArgs<double, double> const & a, int64_t g)
+{
+    constexpr int NEQ = ND + 2;
+    using RC = Rec<ND, double>;
+    if (a.gkind[g] < 0)
+    {
+        double * const base = a.nxt + g * RC::RS;
+        double rec[RC::NUSED], t[NEQ], c[FluxTerms<ND>::N];
+#pragma unroll
+        for (int i = 0; i < RC::NUSED; ++i)
+        {
+            rec[i] = base[i];
+        }
+        solt_terms<ND>(rec, rec + 2 * NEQ, ldg(a.gamma + g), a.qdt, t, c);
+        store_row<ND>(base, rec, t, rec + 2 * NEQ, c);
+        deliver_row<ND>(a, g, rec, rec + 2 * NEQ);
+    }
+}
+
 // The work of thread t of one substep: body cell t for t < ncell, ghost row
 // t - ncell after that.  CT1 = 0 dispatches on each cell's type; a nonzero
 // CT1 compiles the one cell type of a single-type mesh, whose kernel then
@@ -1393,7 +1427,11 @@ __device__ __forceinline__ void fused_thread(MarchArgs<R, G> const & a, int64_t 
         // A ghost row without a boundary condition keeps its stale state; its
         // next so0t is still the Jacobian product of that state.
         int64_t const g = t - a.ncell;
-        if (a.gkind[g] < 0)
+        if constexpr (sizeof(R) == 8)
+        {
+            stale_ghost64<ND>(a, g);
+        }
+        else if (a.gkind[g] < 0)
         {
             R * const base = a.nxt + g * Rec<ND, R>::RS;
             R rec[Rec<ND, R>::NUSED], tt[NEQ];
@@ -1402,19 +1440,137 @@ __device__ __forceinline__ void fused_thread(MarchArgs<R, G> const & a, int64_t 
             {
                 rec[i] = base[i];
             }
-            if constexpr (sizeof(R) == 8)
-            {
-                double c[FluxTerms<ND>::N];
-                solt_terms<ND>(rec, rec + 2 * NEQ, ldg(a.gamma + g), a.qdt, tt, c);
-                store_row<ND>(base, rec, tt, rec + 2 * NEQ, c);
-                deliver_row<ND>(a, g, rec, rec + 2 * NEQ);
-            }
+            Prim<ND, R> const q(rec, ldg(a.gamma + g));
+            solt_prim<ND, R>(q, rec, rec + 2 * NEQ, tt);
+            store_rec<ND>(base, rec, tt, rec + 2 * NEQ);
+        }
+    }
+}
+
+// One cell's substep by the LPC lanes of its group (q: the lane's place in it);
+// see Split.
+template <int CT>
+__device__ __forceinline__ void split_cell(MarchArgs<double, double> const & a, int64_t icl, int q)
+{
+    constexpr int ND = CellT<CT>::ND;
+    constexpr int NEQ = ND + 2;
+    constexpr int LPC = Split<ND>::LPC;
+    using RC = Rec<ND, double>;
+    using F = FluxTerms<ND>;
+    int64_t const row = icl + a.ngst;
+    int const lane = static_cast<int>(threadIdx.x) & 31;
+    int const lead = lane - q; // the group's first lane
+    unsigned const group = ((1u << LPC) - 1u) << lead;
+    int const eq = q < NEQ ? q : NEQ - 1;
+    double const mine = soln64_eq<CT>(a, icl, eq);
+    double so0n[NEQ];
+#pragma unroll
+    for (int i = 0; i < NEQ; ++i)
+    {
+        so0n[i] = __shfl_sync(group, mine, lead + i);
+    }
+    if (q < CellT<CT>::NFC)
+    {
+        int64_t const jr = ldg(a.nbr + q * a.ncell + icl);
+        if (jr < a.ngst)
+        {
+            ghost64<ND>(a, jr, row, so0n);
+        }
+    }
+    double rinv;
+    double const cflc = cfl64<ND>(a, icl, row, so0n, rinv);
+    // This lane's so0n, as calc_cfl left it.
+    double own0 = so0n[0];
+#pragma unroll
+    for (int i = 1; i < NEQ; ++i)
+    {
+        own0 = eq == i ? so0n[i] : own0;
+    }
+    double g[ND];
+    unsigned fired = dsoln64_part<CT, 1>(a, icl, eq, &own0, cflc, g);
+    double so1n[NEQ * ND];
+#pragma unroll
+    for (int i = 0; i < NEQ; ++i)
+    {
+#pragma unroll
+        for (int d = 0; d < ND; ++d)
+        {
+            so1n[i * ND + d] = __shfl_sync(group, g[d], lead + i);
+        }
+    }
+#pragma unroll
+    for (int k = 1; k < LPC; k *= 2)
+    {
+        fired |= __shfl_xor_sync(group, fired, k);
+    }
+    double so0t[NEQ], c[F::N];
+    solt_terms<ND>(so0n, so1n, ldg(a.gamma + row), rinv, a.qdt, so0t, c);
+    // The record, its 16-byte pieces dealt to the lanes in turn.
+    double * const base = a.nxt + row * RC::RS;
+#pragma unroll
+    for (int k = 0; k < (RC::NLOAD + 1) / 2; ++k)
+    {
+        double v[2];
+#pragma unroll
+        for (int w = 0; w < 2; ++w)
+        {
+            int const i = 2 * k + w;
+            v[w] = i < NEQ ? so0n[i]
+                           : (i < 2 * NEQ ? so0t[i - NEQ]
+                                          : (i < RC::NUSED ? so1n[i - 2 * NEQ]
+                                                           : (i < RC::NLOAD ? c[i - RC::OP] : 0.0)));
+        }
+        if (k % LPC == q)
+        {
+            reinterpret_cast<double2 *>(base)[k] = make_double2(v[0], v[1]);
+        }
+    }
+    if (q == 0)
+    {
+        if (a.limiter)
+        {
+            a.limiter[icl] = static_cast<uint8_t>(fired);
+        }
+        deliver_row<ND>(a, row, so0n, so1n);
+    }
+}
+
+// A whole FP64 substep of a small mesh: LPC lanes per body cell, then (rows up
+// to t1 of the work order) one per ghost row.
+template <int ND>
+__global__ void __launch_bounds__(32) k_fused_split(MarchArgs<double, double> a, int64_t t1)
+{
+    constexpr int LPC = Split<ND>::LPC;
+    int64_t const t = static_cast<int64_t>(blockIdx.x) * 32 + threadIdx.x;
+    int64_t const icl = t / LPC;
+    int const q = static_cast<int>(t % LPC);
+    if (icl < a.ncell)
+    {
+        int const ct = a.ctype[icl];
+        if constexpr (ND == 2)
+        {
+            if (ct == 4)
+                split_cell<4>(a, icl, q);
             else
+                split_cell<3>(a, icl, q);
+        }
+        else
+        {
+            switch (ct)
             {
-                Prim<ND, R> const q(rec, ldg(a.gamma + g));
-                solt_prim<ND, R>(q, rec, rec + 2 * NEQ, tt);
-                store_rec<ND>(base, rec, tt, rec + 2 * NEQ);
+            case 6: split_cell<6>(a, icl, q); break;
+            case 5: split_cell<5>(a, icl, q); break;
+            case 7: split_cell<7>(a, icl, q); break;
+            default: split_cell<8>(a, icl, q); break;
             }
+        }
+    }
+    else
+    {
+        int64_t const g = t - a.ncell * LPC;
+        if (g < a.ngst && a.ncell + g < t1)
+        {
+            stale_ghost64<ND>(a, g);
         }
     }
 }
