@@ -309,14 +309,31 @@ struct Residual
     int64_t ngst = 0, ncell = 0;
 };
 
+__device__ __noinline__ double widen_plain(float v) { return double(v); }
+
+// double(v): the conversion instruction goes through the FP64 pipe (the FP32
+// gradients of 1.3M tetrahedra left k_get_field in 111 us with it, FP64 ones in
+// 69); normal numbers and zeros are widened by the integer one.
+__device__ __forceinline__ double widen(float v)
+{
+    unsigned const u = __float_as_uint(v);
+    unsigned const sign = u & 0x80000000u, m = u ^ sign;
+    if (m - 0x00800000u < 0x7f000000u)
+    {
+        return __hiloint2double(static_cast<int>(sign | ((m >> 3) + 0x38000000u)), static_cast<int>(u << 29));
+    }
+    return m == 0u ? __hiloint2double(static_cast<int>(sign), 0) : widen_plain(v);
+}
+__device__ __forceinline__ double widen(double v) { return v; }
+
 // Value k of row r of a record field in FP64, the residual added.
 template <int ND, typename R>
 __device__ __forceinline__ double field_value(R const * rec, int64_t r, int off, int k, Residual c)
 {
-    double v = double(rec[r * Rec<ND, R>::RS + off + k]);
+    double v = widen(rec[r * Rec<ND, R>::RS + off + k]);
     if (c.comp && r >= c.ngst)
     {
-        v += double(static_cast<R const *>(c.comp)[k * c.ncell + (r - c.ngst)]);
+        v += widen(static_cast<R const *>(c.comp)[k * c.ncell + (r - c.ngst)]);
     }
     return v;
 }
@@ -334,59 +351,31 @@ __device__ __forceinline__ void field_store(R * rec, int64_t r, int off, int k, 
     }
 }
 
-// Record field <-> FP64 reference-layout table.
-template <int ND, typename R>
-__global__ void k_get_field(R const * rec, double * out, int64_t nrow, int off, int width, Residual c)
+// Record field <-> FP64 reference-layout table of W values a row, on the device
+// or in mapped host memory: one thread per pair of consecutive doubles of the
+// table, so the table is accessed in contiguous 16-byte pieces (vec: it is
+// 16-byte aligned) and the records are gathered.  A thread per row, its
+// stores W doubles apart, took 190 us for the gradients of 1.3M tetrahedra
+// (153 MB; FP32 records), 53 us with the pairs, of 912 us with the copy (1041 before).
+template <int ND, typename R, int W>
+__global__ void k_get_field(R const * rec, double * out, int64_t nrow, int off, bool vec, Residual c)
 {
-    int64_t const r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (r >= nrow)
-    {
-        return;
-    }
-    for (int k = 0; k < width; ++k)
-    {
-        out[r * width + k] = field_value<ND, R>(rec, r, off, k, c);
-    }
-}
-
-template <int ND, typename R>
-__global__ void k_set_field(R * rec, double const * in, int64_t nrow, int off, int width, Residual c)
-{
-    int64_t const r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (r >= nrow)
-    {
-        return;
-    }
-    for (int k = 0; k < width; ++k)
-    {
-        field_store<ND, R>(rec, r, off, k, in[r * width + k], c);
-    }
-}
-
-// The same record fields read from or written to mapped host memory: one
-// thread per pair of consecutive doubles of the host table, so the host side
-// is accessed in contiguous 16-byte pieces (vec: the host table is 16-byte
-// aligned) and the records are gathered on the device.
-template <int ND, typename R>
-__global__ void k_get_field_host(R const * rec, double * out, int64_t nrow, int off, int width, bool vec,
-                                 Residual c)
-{
-    int64_t const n = nrow * width;
+    int64_t const n = nrow * W;
     int64_t const i = 2 * (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x);
     if (i >= n)
     {
         return;
     }
-    int64_t const r0 = i / width;
-    int const k0 = static_cast<int>(i - r0 * width);
+    int64_t const r0 = i / W;
+    int const k0 = static_cast<int>(i - r0 * W);
     double const v0 = field_value<ND, R>(rec, r0, off, k0, c);
     if (i + 1 >= n)
     {
         out[i] = v0;
         return;
     }
-    int64_t const r1 = k0 + 1 < width ? r0 : r0 + 1;
-    int const k1 = k0 + 1 < width ? k0 + 1 : 0;
+    int64_t const r1 = k0 + 1 < W ? r0 : r0 + 1;
+    int const k1 = k0 + 1 < W ? k0 + 1 : 0;
     double const v1 = field_value<ND, R>(rec, r1, off, k1, c);
     if (vec)
     {
@@ -401,16 +390,15 @@ __global__ void k_get_field_host(R const * rec, double * out, int64_t nrow, int 
 
 // Two values per thread (grid-stride: a grid of one pass per pair is the
 // usual launch).
-template <int ND, typename R>
-__global__ void k_set_field_host(R * rec, double const * in, int64_t nrow, int off, int width, bool vec,
-                                 Residual c)
+template <int ND, typename R, int W>
+__global__ void k_set_field(R * rec, double const * in, int64_t nrow, int off, bool vec, Residual c)
 {
-    int64_t const n = nrow * width;
+    int64_t const n = nrow * W;
     int64_t const step = 2 * static_cast<int64_t>(gridDim.x) * blockDim.x;
     for (int64_t i = 2 * (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x); i < n; i += step)
     {
-        int64_t const r0 = i / width;
-        int const k0 = static_cast<int>(i - r0 * width);
+        int64_t const r0 = i / W;
+        int const k0 = static_cast<int>(i - r0 * W);
         if (i + 1 >= n)
         {
             field_store<ND, R>(rec, r0, off, k0, in[i], c);
@@ -425,8 +413,8 @@ __global__ void k_set_field_host(R * rec, double const * in, int64_t nrow, int o
         {
             v = make_double2(in[i], in[i + 1]);
         }
-        int64_t const r1 = k0 + 1 < width ? r0 : r0 + 1;
-        int const k1 = k0 + 1 < width ? k0 + 1 : 0;
+        int64_t const r1 = k0 + 1 < W ? r0 : r0 + 1;
+        int const k1 = k0 + 1 < W ? k0 + 1 : 0;
         field_store<ND, R>(rec, r0, off, k0, v.x, c);
         field_store<ND, R>(rec, r1, off, k1, v.y, c);
     }
@@ -485,7 +473,7 @@ __global__ void k_chunk_top_row(int32_t const * nbr, int8_t const * ctype, int64
 // pieces (vec: the table is 16-byte aligned; a block's stretch starts at a
 // multiple of 128 rows, so it is aligned too), then one thread per row
 // finishes the row.  The values and the arithmetic are those of
-// k_set_field_host followed by k_solt_rows.
+// k_set_field followed by k_solt_rows.
 template <int ND, typename R>
 __global__ void __launch_bounds__(BLOCK) k_set_so1_host_solt(R * rec, double const * in, R const * gamma,
                                                              int64_t nrow, bool vec, R qdt)
@@ -494,7 +482,7 @@ __global__ void __launch_bounds__(BLOCK) k_set_so1_host_solt(R * rec, double con
     constexpr int W = NEQ * ND;
     using RC = Rec<ND, R>;
     __shared__ double buf[BLOCK * W];
-    // Grid-stride over stretches of BLOCK rows (see k_set_field_host).
+    // Grid-stride over stretches of BLOCK rows (see k_set_field).
     for (int64_t r0 = static_cast<int64_t>(blockIdx.x) * BLOCK; r0 < nrow;
          r0 += static_cast<int64_t>(gridDim.x) * BLOCK)
     {
@@ -1239,6 +1227,37 @@ public:
         }
     }
 
+    // One field of all rows into a table, or of nr rows from one.
+    void get_field(R const * base, double * out, int off, int width, Residual c)
+    {
+        bool const vec = reinterpret_cast<uintptr_t>(out) % 16 == 0;
+        unsigned const grid = grid_for((nrow * width + 1) / 2);
+        if (width == NEQ)
+        {
+            k_get_field<ND, R, NEQ><<<grid, BLOCK, 0, stream>>>(base, out, nrow, off, vec, c);
+        }
+        else
+        {
+            k_get_field<ND, R, NEQ * ND><<<grid, BLOCK, 0, stream>>>(base, out, nrow, off, vec, c);
+        }
+        launched(stream, "get_field");
+    }
+
+    void set_field(R * base, double const * in, int64_t nr, int off, int width, Residual c, cudaStream_t on)
+    {
+        bool const vec = reinterpret_cast<uintptr_t>(in) % 16 == 0;
+        unsigned const grid = grid_for((nr * width + 1) / 2);
+        if (width == NEQ)
+        {
+            k_set_field<ND, R, NEQ><<<grid, BLOCK, 0, on>>>(base, in, nr, off, vec, c);
+        }
+        else
+        {
+            k_set_field<ND, R, NEQ * ND><<<grid, BLOCK, 0, on>>>(base, in, nr, off, vec, c);
+        }
+        launched(on, "set_field");
+    }
+
     void get_array(int which, double * out) override
     {
         upload_bc();
@@ -1273,15 +1292,11 @@ public:
             if (double * const dev = static_cast<double *>(mapped_host(out, nb)))
             {
                 // Mapped host table: the gather writes it directly.
-                k_get_field_host<ND, R><<<grid_for((n + 1) / 2), BLOCK, 0, stream>>>(
-                    base, dev, nrow, off, width, reinterpret_cast<uintptr_t>(dev) % 16 == 0, so0_residual(which));
-                launched(stream, "get_field_host");
+                get_field(base, dev, off, width, so0_residual(which));
                 sync();
                 return;
             }
-            k_get_field<ND, R><<<grid_for(nrow), BLOCK, 0, stream>>>(base, tmp, nrow, off, width,
-                                                                     so0_residual(which));
-            launched(stream, "get_field");
+            get_field(base, tmp, off, width, so0_residual(which));
         }
         cuda_check(cudaMemcpyAsync(out, tmp, nb, cudaMemcpyDeviceToHost, stream), "D2H");
         sync();
@@ -1322,10 +1337,7 @@ public:
                 }
                 else
                 {
-                    k_set_field_host<ND, R><<<grid_for((n + 1) / 2), BLOCK, 0, stream>>>(
-                        base, dev, nrow, off, width, reinterpret_cast<uintptr_t>(dev) % 16 == 0,
-                        so0_written(which));
-                    launched(stream, "set_field_host");
+                    set_field(base, dev, nrow, off, width, so0_written(which), stream);
                     next_valid = false;
                 }
                 sync();
@@ -1351,9 +1363,7 @@ public:
             R * base;
             int off, width;
             field_of(which, base, off, width);
-            k_set_field<ND, R><<<grid_for(nrow), BLOCK, 0, stream>>>(base, tmp, nrow, off, width,
-                                                                     so0_written(which));
-            launched(stream, "set_field");
+            set_field(base, tmp, nrow, off, width, so0_written(which), stream);
         }
         next_valid = false;
         sync();
@@ -1647,9 +1657,7 @@ public:
                 int off, width;
                 field_of(k == 0 ? EA_SO0N : EA_SO1N, base, off, width);
                 int64_t const n = static_cast<int64_t>(d.nbytes / sizeof(double));
-                k_get_field_host<ND, R><<<grid_for((n + 1) / 2), BLOCK, 0, stream>>>(
-                    base, d.dev, nrow, off, width, true, so0_residual(k == 0 ? EA_SO0N : EA_SO1N));
-                launched(stream, "get_field_host");
+                get_field(base, d.dev, off, width, so0_residual(k == 0 ? EA_SO0N : EA_SO1N));
             }
         }
     }
@@ -1730,10 +1738,7 @@ public:
                        "H2D");
             cuda_check(cudaEventRecord(m_cpev[j], m_copy), "record");
             cuda_check(cudaStreamWaitEvent(m_xfer, m_cpev[j], 0), "wait");
-            k_set_field_host<ND, R><<<grid_for((nr * NEQ + 1) / 2), BLOCK, 0, m_xfer>>>(
-                base + r0 * RS, in0, nr, 0, NEQ, reinterpret_cast<uintptr_t>(in0) % 16 == 0,
-                Residual{c.comp, c.ngst - r0, c.ncell});
-            launched(m_xfer, "set_field_host");
+            set_field(base + r0 * RS, in0, nr, 0, NEQ, Residual{c.comp, c.ngst - r0, c.ncell}, m_xfer);
             if (solt)
             {
                 k_set_so1_host_solt<ND, R><<<grid_for(nr), BLOCK, 0, m_xfer>>>(
@@ -1743,9 +1748,7 @@ public:
             }
             else
             {
-                k_set_field_host<ND, R><<<grid_for((nr * W + 1) / 2), BLOCK, 0, m_xfer>>>(
-                    base + r0 * RS, in1, nr, 2 * NEQ, W, reinterpret_cast<uintptr_t>(in1) % 16 == 0, Residual{});
-                launched(m_xfer, "set_field_host");
+                set_field(base + r0 * RS, in1, nr, 2 * NEQ, W, Residual{}, m_xfer);
             }
             cuda_check(cudaEventRecord(m_xev[j], m_xfer), "record");
         };
