@@ -408,6 +408,124 @@ __device__ __forceinline__ double cap64(double * w, double acfl, double sigma0, 
     return mu(fire ? nn : sigma0, recip(fire ? dd : cw));
 }
 
+// The weights of N gradient elements from their squared magnitudes sq in FP64,
+// for operands weights64 does not take.
+template <int N>
+__device__ __noinline__ bool weights64_plain(double const * sq, double acfl, double sigma0, double * wt)
+{
+    for (int k = 0; k < N; ++k)
+    {
+        wt[k] = rsq(sq[k]);
+    }
+    bool fire;
+    double const cc = cap64<N>(wt, acfl, sigma0, fire);
+    for (int k = 0; k < N; ++k)
+    {
+        wt[k] = fm(cc, wt[k], 1.0 / N);
+    }
+    return fire;
+}
+
+// n 2^e for n in [2^63, 2^64), rounded down to a double.
+__device__ __forceinline__ double compose(unsigned long long n, int e)
+{
+    return __longlong_as_double(static_cast<long long>((n >> 11) + (static_cast<unsigned long long>(1085 + e) << 52)));
+}
+
+// The same weights, 1/N + (N-1)/N U_k / max(t S, M), in integers but for one
+// multiplication: w_k = 1/sqrt(sq_k) aligned to the largest of them, S their sum,
+// U_k = N w_k - S, M = max(max U, (N-1) max(-U)), and t = (N-1) acfl / sigma0; the
+// cap fires where t S < M.  This is cap64's 1/N + cc (w_k - mean w) with the
+// common factors taken out, and w_k's scale with them.  The smallest bit kept
+// is 2^-57 of the largest w, a sixteenth of its rounding in FP64.  Takes
+// normal sq_k > 0 and t in 2^[-400, 400); others by the call.  Some 180 integer
+// instructions for 15 FP64 ones (N = 3; 19 at 4, 31 at 8); substep 2M triangles
+// 1527 -> 1330 us, 490,000 quadrilaterals 568 -> 524, 384,000 tetrahedra 783 -> 737,
+// 64,000 hexahedra 328 -> 322.
+template <int N>
+__device__ __forceinline__ bool weights64(double const * sq, double t, double acfl, double sigma0, double * wt)
+{
+    // (N-1) N 2^(62-P) < 2^63.
+    constexpr int P = N <= 3 ? 2 : (N == 4 ? 3 : (N <= 6 ? 4 : 5));
+    static_assert(N <= 8, "P");
+    bool plain = (static_cast<unsigned>(__double2hiint(t)) >> 20) - 623u > 799u;
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+    {
+        plain = plain || !pos_normal(static_cast<unsigned>(__double2hiint(sq[k])));
+    }
+    if (plain)
+    {
+        double s[N], w[N];
+#pragma unroll
+        for (int k = 0; k < N; ++k)
+        {
+            s[k] = sq[k];
+        }
+        bool const fire = weights64_plain<N>(s, acfl, sigma0, w);
+#pragma unroll
+        for (int k = 0; k < N; ++k)
+        {
+            wt[k] = w[k];
+        }
+        return fire;
+    }
+    unsigned long long w[N]; // w_k 2^(62 + h_k), then aligned
+    int h[N], low;
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+    {
+        unsigned long long x;
+        w[k] = rsq_fixed(static_cast<unsigned>(__double2hiint(sq[k])), static_cast<unsigned>(__double2loint(sq[k])), x,
+                         h[k]);
+        low = k == 0 ? h[0] : min(low, h[k]);
+    }
+    unsigned long long sum = 0;
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+    {
+        w[k] = w[k] >> min(P + h[k] - low, 63);
+        sum += w[k];
+    }
+    long long u[N], most = 0, least = 0;
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+    {
+        u[k] = static_cast<long long>(w[k] * N - sum);
+        most = u[k] > most ? u[k] : most;
+        least = u[k] < least ? u[k] : least;
+    }
+    long long const side = -least * (N - 1);
+    unsigned long long const big = static_cast<unsigned long long>(side > most ? side : most);
+    int const ls = __clzll(static_cast<long long>(sum));
+    double const ts = mu(t, compose(sum << ls, -ls));
+    // max(t S, M) = n 2^(e - 63) with n in [2^63, 2^64).
+    unsigned const th = static_cast<unsigned>(__double2hiint(ts));
+    unsigned long long n = sig53(th, static_cast<unsigned>(__double2loint(ts))) << 11;
+    int e = static_cast<int>(th >> 20) - 1023;
+    int const lb = __clzll(static_cast<long long>(big));
+    unsigned long long const nb = big << (lb & 63);
+    int const eb = big == 0 ? -2000 : 63 - lb;
+    bool const fire = eb > e || (eb == e && nb > n);
+    n = fire ? nb : n;
+    e = fire ? eb : e;
+    unsigned long long r = rcp_sig(static_cast<unsigned>(n >> 43), static_cast<unsigned>(n >> 11)); // 2^62 / (n 2^-63)
+    r -= r / N;
+    // |u_k| < 2^(e + 1), so that u_k 2^(61 - e) fits; zero where e < 0.
+    int const left = min(max(61 - e, 0), 63), right = min(max(e - 61, 0), 63);
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+    {
+        bool const neg = u[k] < 0;
+        unsigned long long const m = static_cast<unsigned long long>(neg ? -u[k] : u[k]) << left >> right;
+        long long const q = static_cast<long long>(mul_hi64(m, r)); // 2^59
+        long long const v = static_cast<long long>((1ull << 59) / N) + (neg ? -q : q);
+        int const lv = __clzll(v);
+        wt[k] = v > 0 ? compose(static_cast<unsigned long long>(v) << lv, -59 - lv) : 0.0;
+    }
+    return fire;
+}
+
 // What calc_dsoln reads of a neighbour's record for equations q .. q + E - 1:
 // their so0 and so0t (u, t) and gradients (g).
 template <int ND, int E>
@@ -463,6 +581,7 @@ __device__ __forceinline__ unsigned dsoln64_simplex(MarchArgs<double, double> co
     using D = Geo<ND, double>;
     using RC = Rec<ND, double>;
     double const acfl = fabs(cflc);
+    double const ts = mu(mu(acfl, double(N - 1)), recip(a.sigma0));
     double const tau = fm(acfl, a.tauscale, a.taumin);
     GeoView<double> const gv = geo_view(a, icl);
     // Solution deltas at the evaluation points: of the first ND faces, and
@@ -538,8 +657,8 @@ __device__ __forceinline__ unsigned dsoln64_simplex(MarchArgs<double, double> co
     for (int i = 0; i < E; ++i)
     {
         // Element m < ND leaves out face m, element ND the last face.
-        double g[ND], w[N];
-        double sq = Tiny<double>::AZ;
+        double g[ND], sq[N], w[N];
+        sq[ND] = Tiny<double>::AZ;
 #pragma unroll
         for (int d = 0; d < ND; ++d)
         {
@@ -550,29 +669,25 @@ __device__ __forceinline__ unsigned dsoln64_simplex(MarchArgs<double, double> co
                 s = fm(uf[f][i], c[f][d], s);
             }
             g[d] = s;
-            sq = fm(s, s, sq);
+            sq[ND] = fm(s, s, sq[ND]);
         }
-        w[ND] = rsq(sq); // W-1/2: inverse gradient magnitude
 #pragma unroll
         for (int m = 0; m < ND; ++m)
         {
-            sq = Tiny<double>::AZ;
+            sq[m] = Tiny<double>::AZ;
 #pragma unroll
             for (int d = 0; d < ND; ++d)
             {
                 double const s = fm(-us[i], c[m][d], g[d]);
-                sq = fm(s, s, sq);
+                sq[m] = fm(s, s, sq[m]);
             }
-            w[m] = rsq(sq);
         }
-        bool fire;
-        double const cc = cap64<N>(w, acfl, a.sigma0, fire);
-        fired |= fire ? 1u << (q + i) : 0u;
-        // sum_k (1/n + cc u_k) g_k, the weights summing to one.
+        fired |= weights64<N>(sq, ts, acfl, a.sigma0, w) ? 1u << (q + i) : 0u;
+        // sum_k w_k g_k, the weights summing to one.
 #pragma unroll
         for (int m = 0; m < ND; ++m)
         {
-            double const ws = mu(fm(cc, w[m], 1.0 / N), us[i]);
+            double const ws = mu(w[m], us[i]);
 #pragma unroll
             for (int d = 0; d < ND; ++d)
             {
@@ -658,6 +773,7 @@ __device__ __forceinline__ unsigned dsoln64_general(MarchArgs<double, double> co
     using D = Geo<ND, double>;
     using RC = Rec<ND, double>;
     double const acfl = fabs(cflc);
+    double const ts = mu(mu(acfl, double(NFGE - 1)), recip(a.sigma0));
     double const tau = fm(acfl, a.tauscale, a.taumin);
     GeoView<double> const gv = geo_view(a, icl);
     double x[NFC][ND];
@@ -778,11 +894,11 @@ __device__ __forceinline__ unsigned dsoln64_general(MarchArgs<double, double> co
 #pragma unroll
     for (int i = 0; i < E; ++i)
     {
-        double g[NFGE][ND], w[NFGE];
+        double g[NFGE][ND], sq[NFGE], w[NFGE];
 #pragma unroll
         for (int k = 0; k < NFGE; ++k)
         {
-            double sq = Tiny<double>::AZ;
+            sq[k] = Tiny<double>::AZ;
 #pragma unroll
             for (int d = 0; d < ND; ++d)
             {
@@ -793,21 +909,18 @@ __device__ __forceinline__ unsigned dsoln64_general(MarchArgs<double, double> co
                     s = fm(uf[CellT<CT>::fge(k, v)][i], C[k][v][d], s);
                 }
                 g[k][d] = s;
-                sq = fm(s, s, sq);
+                sq[k] = fm(s, s, sq[k]);
             }
-            w[k] = rsq(sq); // W-1/2: inverse gradient magnitude
         }
-        bool fire;
-        double const cc = cap64<NFGE>(w, acfl, a.sigma0, fire);
-        fired |= fire ? 1u << (q + i) : 0u;
+        fired |= weights64<NFGE>(sq, ts, acfl, a.sigma0, w) ? 1u << (q + i) : 0u;
 #pragma unroll
         for (int d = 0; d < ND; ++d)
         {
-            double s = mu(fm(cc, w[0], 1.0 / NFGE), g[0][d]);
+            double s = mu(w[0], g[0][d]);
 #pragma unroll
             for (int k = 1; k < NFGE; ++k)
             {
-                s = fm(fm(cc, w[k], 1.0 / NFGE), g[k][d], s);
+                s = fm(w[k], g[k][d], s);
             }
             so1n[i * ND + d] = s;
         }
