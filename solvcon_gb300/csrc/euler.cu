@@ -1549,10 +1549,10 @@ public:
 
     // FP64 meshes up to this many cells march with several lanes per cell
     // (k_fused_split), larger ones with one.  Per substep, one lane -> several:
-    // 1,024 triangles 33.7 -> 16.6 us (up to 4,000 the same), 8,192 30.9 ->
-    // 21.3, 12,800 30.9 -> 28.9, 20,000 37.6 -> 41.2; 1,024 quadrilaterals 41.2 ->
-    // 20.7, 10,000 42.0 -> 33.0; 2,058 tetrahedra 57.6 -> 28.9, 4,374 57.6 -> 43.2,
-    // 7,986 59.5 -> 79.4; 512 hexahedra 111 -> 45, 2,744 121 -> 56, 5,832 122 -> 124.
+    // 1,058 triangles 35.0 -> 16.6 us, 8,192 31.0 -> 20.8, 12,800 31.1 -> 26.9
+    // (20,000 37 -> 41); 10,000 quadrilaterals 45.1 -> 33.0; 2,058 tetrahedra 58.1 ->
+    // 28.9, 4,374 57.7 -> 41.2 (7,986 60 -> 79); 1,331 hexahedra 119 -> 43, 4,913 121 ->
+    // 86.
     static constexpr int64_t SPLIT_CELLS = ND == 2 ? 12800 : 5200;
 
     // The fused kernel over rows [t0, t1) of its work order (body cells, then

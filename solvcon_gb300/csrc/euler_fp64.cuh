@@ -45,6 +45,15 @@ namespace dev
 __device__ __forceinline__ double fm(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ double mu(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double ad(double a, double b) { return __dadd_rn(a, b); }
+// A product of the loop over equations, E of them: in 2D on the integer pipe,
+// the same bits (2M triangles 1252 -> 1198 us, 490,000 quadrilaterals 465 -> 453);
+// in 3D the longer loop costs more (64,000 hexahedra 285 -> 310), as it does
+// outside the loop (1198 -> 1280 with the flux terms' products).
+template <int ND, int E>
+__device__ __forceinline__ double mx(double a, double b)
+{
+    return ND == 2 && E > 1 ? mul_int(a, b) : mu(a, b);
+}
 __device__ __forceinline__ double sb(double a, double b) { return __dsub_rn(a, b); }
 
 // Layout of a record's flux terms: the time-centred fluxes A_d (f_d + dt/4 J_d
@@ -260,6 +269,17 @@ __device__ __forceinline__ void soln64(MarchArgs<double, double> const & a, int6
     GeoView<double> const gv = geo_view(a, icl);
     double acc[NEQ];
 #pragma unroll
+    for (int i = 0; i < NEQ; ++i)
+    {
+        acc[i] = -0.0; // -0 + a = a, zeros of both signs too
+    }
+    // Not unrolled, as the loops over faces and equations of calc_dsoln (which
+    // index uf in local memory for it): a substep's instructions in one stretch
+    // are more than the instruction caches hold, and FP64 tetrahedra and
+    // hexahedra waited for them a fifth of the time.  384k tetrahedra 740 ->
+    // 688 us, 64k hexahedra 323 -> 298, 64k prisms 510 -> 440, 490k quadrilaterals
+    // 527 -> 490, 2M triangles 1348 -> 1331; most of it from the equations' loop.
+#pragma unroll 1
     for (int f = 0; f < NFC; ++f)
     {
         int64_t const jr = __ldg(a.nbr + f * a.ncell + icl);
@@ -286,7 +306,7 @@ __device__ __forceinline__ void soln64(MarchArgs<double, double> const & a, int6
 #pragma unroll
         for (int i = 0; i < NEQ; ++i)
         {
-            acc[i] = f == 0 ? mu(bvol, rec[i]) : fm(bvol, rec[i], acc[i]);
+            acc[i] = fm(bvol, rec[i], acc[i]);
         }
 #pragma unroll
         for (int d = 0; d < ND; ++d)
@@ -433,52 +453,31 @@ __device__ __forceinline__ double compose(unsigned long long n, int e)
 }
 
 // The same weights, 1/N + (N-1)/N U_k / max(t S, M), in integers but for one
-// multiplication: w_k = 1/sqrt(sq_k) aligned to the largest of them, S their sum,
+// multiplication: w_k = w[k] 2^(-62 - h[k]), the inverse gradient magnitudes
+// (inverse_norm), aligned to the largest of them, S their sum,
 // U_k = N w_k - S, M = max(max U, (N-1) max(-U)), and t = (N-1) acfl / sigma0; the
 // cap fires where t S < M.  This is cap64's 1/N + cc (w_k - mean w) with the
 // common factors taken out, and w_k's scale with them.  The smallest bit kept
-// is 2^-57 of the largest w, a sixteenth of its rounding in FP64.  Takes
-// normal sq_k > 0 and t in 2^[-400, 400); others by the call.  Some 180 integer
+// is 2^-57 of the largest w, a sixteenth of its rounding in FP64.  For t in
+// 2^[-400, 400) (cap_in_range).  Some 180 integer
 // instructions for 15 FP64 ones (N = 3; 19 at 4, 31 at 8); substep 2M triangles
 // 1527 -> 1330 us, 490,000 quadrilaterals 568 -> 524, 384,000 tetrahedra 783 -> 737,
 // 64,000 hexahedra 328 -> 322.
+__device__ __forceinline__ bool cap_in_range(double t)
+{
+    return (static_cast<unsigned>(__double2hiint(t)) >> 20) - 623u <= 799u;
+}
 template <int N>
-__device__ __forceinline__ bool weights64(double const * sq, double t, double acfl, double sigma0, double * wt)
+__device__ __forceinline__ bool weights64(unsigned long long * w, int const * h, double t, double * wt)
 {
     // (N-1) N 2^(62-P) < 2^63.
     constexpr int P = N <= 3 ? 2 : (N == 4 ? 3 : (N <= 6 ? 4 : 5));
     static_assert(N <= 8, "P");
-    bool plain = (static_cast<unsigned>(__double2hiint(t)) >> 20) - 623u > 799u;
+    int low = h[0];
 #pragma unroll
-    for (int k = 0; k < N; ++k)
+    for (int k = 1; k < N; ++k)
     {
-        plain = plain || !pos_normal(static_cast<unsigned>(__double2hiint(sq[k])));
-    }
-    if (plain)
-    {
-        double s[N], w[N];
-#pragma unroll
-        for (int k = 0; k < N; ++k)
-        {
-            s[k] = sq[k];
-        }
-        bool const fire = weights64_plain<N>(s, acfl, sigma0, w);
-#pragma unroll
-        for (int k = 0; k < N; ++k)
-        {
-            wt[k] = w[k];
-        }
-        return fire;
-    }
-    unsigned long long w[N]; // w_k 2^(62 + h_k), then aligned
-    int h[N], low;
-#pragma unroll
-    for (int k = 0; k < N; ++k)
-    {
-        unsigned long long x;
-        w[k] = rsq_fixed(static_cast<unsigned>(__double2hiint(sq[k])), static_cast<unsigned>(__double2loint(sq[k])), x,
-                         h[k]);
-        low = k == 0 ? h[0] : min(low, h[k]);
+        low = min(low, h[k]);
     }
     unsigned long long sum = 0;
 #pragma unroll
@@ -580,6 +579,7 @@ __device__ __forceinline__ unsigned dsoln64_simplex(MarchArgs<double, double> co
     constexpr int N = ND + 1; // faces, and gradient elements
     using D = Geo<ND, double>;
     using RC = Rec<ND, double>;
+    constexpr int UF = E > 1 ? 1 : N;
     double const acfl = fabs(cflc);
     double const ts = mu(mu(acfl, double(N - 1)), recip(a.sigma0));
     double const tau = fm(acfl, a.tauscale, a.taumin);
@@ -587,8 +587,12 @@ __device__ __forceinline__ unsigned dsoln64_simplex(MarchArgs<double, double> co
     // Solution deltas at the evaluation points: of the first ND faces, and
     // their sum over all.
     double uf[ND][E], us[E];
-    double x[ND][ND]; // displacements of the first ND faces
 #pragma unroll
+    for (int i = 0; i < E; ++i)
+    {
+        us[i] = -0.0;
+    }
+#pragma unroll UF
     for (int f = 0; f < N; ++f)
     {
         int64_t const jr = __ldg(a.nbr + f * a.ncell + icl);
@@ -597,12 +601,7 @@ __device__ __forceinline__ unsigned dsoln64_simplex(MarchArgs<double, double> co
 #pragma unroll
         for (int d = 0; d < ND; ++d)
         {
-            double const qf = fg<ND>(gv, f, D::K_Q + d);
-            jd[d] = fm(tau, qf, fg<ND>(gv, f, D::K_R + d));
-            if (f < ND)
-            {
-                x[f][d] = fm(tau, qf, fg<ND>(gv, f, D::K_P + d));
-            }
+            jd[d] = fm(tau, fg<ND>(gv, f, D::K_Q + d), fg<ND>(gv, f, D::K_R + d));
         }
 #pragma unroll
         for (int i = 0; i < E; ++i)
@@ -617,7 +616,17 @@ __device__ __forceinline__ unsigned dsoln64_simplex(MarchArgs<double, double> co
             {
                 uf[f][i] = s;
             }
-            us[i] = f == 0 ? s : ad(us[i], s);
+            us[i] = ad(us[i], s);
+        }
+    }
+    double x[ND][ND]; // displacements of the first ND faces
+#pragma unroll
+    for (int f = 0; f < ND; ++f)
+    {
+#pragma unroll
+        for (int d = 0; d < ND; ++d)
+        {
+            x[f][d] = fm(tau, fg<ND>(gv, f, D::K_Q + d), fg<ND>(gv, f, D::K_P + d));
         }
     }
     // Columns of the inverse of the displacement rows.
@@ -653,41 +662,69 @@ __device__ __forceinline__ unsigned dsoln64_simplex(MarchArgs<double, double> co
         }
     }
     unsigned fired = 0;
-#pragma unroll
+#pragma unroll 1
     for (int i = 0; i < E; ++i)
     {
         // Element m < ND leaves out face m, element ND the last face.
-        double g[ND], sq[N], w[N];
-        sq[ND] = Tiny<double>::AZ;
+        double g[ND], w[N];
+        unsigned long long r[N];
+        int h[N];
 #pragma unroll
         for (int d = 0; d < ND; ++d)
         {
-            double s = mu(uf[0][i], c[0][d]);
+            double s = mx<ND, E>(uf[0][i], c[0][d]);
 #pragma unroll
             for (int f = 1; f < ND; ++f)
             {
                 s = fm(uf[f][i], c[f][d], s);
             }
             g[d] = s;
-            sq[ND] = fm(s, s, sq[ND]);
         }
+        bool fixed = cap_in_range(ts);
+        fixed = inverse_norm<ND>(g, r[ND], h[ND]) && fixed; // W-1/2: inverse gradient magnitude
 #pragma unroll
         for (int m = 0; m < ND; ++m)
         {
-            sq[m] = Tiny<double>::AZ;
+            double s[ND];
 #pragma unroll
             for (int d = 0; d < ND; ++d)
             {
-                double const s = fm(-us[i], c[m][d], g[d]);
-                sq[m] = fm(s, s, sq[m]);
+                s[d] = fm(-us[i], c[m][d], g[d]);
+            }
+            fixed = inverse_norm<ND>(s, r[m], h[m]) && fixed;
+        }
+        bool fire;
+        if (fixed)
+        {
+            fire = weights64<N>(r, h, ts, w);
+        }
+        else
+        {
+            double sq[N], wp[N];
+#pragma unroll
+            for (int m = 0; m < N; ++m)
+            {
+                sq[m] = Tiny<double>::AZ;
+#pragma unroll
+                for (int d = 0; d < ND; ++d)
+                {
+                    double const s = m < ND ? fm(-us[i], c[m < ND ? m : 0][d], g[d]) : g[d];
+                    sq[m] = fm(s, s, sq[m]);
+                }
+            }
+            fire = weights64_plain<N>(sq, acfl, a.sigma0, wp);
+#pragma unroll
+            for (int m = 0; m < N; ++m)
+            {
+                w[m] = wp[m];
             }
         }
-        fired |= weights64<N>(sq, ts, acfl, a.sigma0, w) ? 1u << (q + i) : 0u;
+        fired |= fire ? 1u << (q + i) : 0u;
         // sum_k w_k g_k, the weights summing to one.
 #pragma unroll
         for (int m = 0; m < ND; ++m)
         {
-            double const ws = mu(w[m], us[i]);
+            double const ws = mx<ND, E>(w[m], us[i]);
 #pragma unroll
             for (int d = 0; d < ND; ++d)
             {
@@ -772,6 +809,7 @@ __device__ __forceinline__ unsigned dsoln64_general(MarchArgs<double, double> co
     constexpr int NFGE = CellT<CT>::NFGE;
     using D = Geo<ND, double>;
     using RC = Rec<ND, double>;
+    constexpr int UF = E > 1 ? 1 : NFC;
     double const acfl = fabs(cflc);
     double const ts = mu(mu(acfl, double(NFGE - 1)), recip(a.sigma0));
     double const tau = fm(acfl, a.tauscale, a.taumin);
@@ -839,7 +877,7 @@ __device__ __forceinline__ unsigned dsoln64_general(MarchArgs<double, double> co
     }
     // Solution deltas at the evaluation points.
     double uf[NFC][E];
-#pragma unroll
+#pragma unroll UF
     for (int f = 0; f < NFC; ++f)
     {
         int64_t const jr = __ldg(a.nbr + f * a.ncell + icl);
@@ -891,32 +929,59 @@ __device__ __forceinline__ unsigned dsoln64_general(MarchArgs<double, double> co
         }
     }
     unsigned fired = 0;
-#pragma unroll
+#pragma unroll 1
     for (int i = 0; i < E; ++i)
     {
-        double g[NFGE][ND], sq[NFGE], w[NFGE];
+        double g[NFGE][ND], w[NFGE];
+        unsigned long long r[NFGE];
+        int h[NFGE];
+        bool fixed = cap_in_range(ts);
 #pragma unroll
         for (int k = 0; k < NFGE; ++k)
         {
-            sq[k] = Tiny<double>::AZ;
 #pragma unroll
             for (int d = 0; d < ND; ++d)
             {
-                double s = mu(uf[CellT<CT>::fge(k, 0)][i], C[k][0][d]);
+                double s = mx<ND, E>(uf[CellT<CT>::fge(k, 0)][i], C[k][0][d]);
 #pragma unroll
                 for (int v = 1; v < ND; ++v)
                 {
                     s = fm(uf[CellT<CT>::fge(k, v)][i], C[k][v][d], s);
                 }
                 g[k][d] = s;
-                sq[k] = fm(s, s, sq[k]);
+            }
+            fixed = inverse_norm<ND>(g[k], r[k], h[k]) && fixed; // W-1/2: inverse gradient magnitude
+        }
+        bool fire;
+        if (fixed)
+        {
+            fire = weights64<NFGE>(r, h, ts, w);
+        }
+        else
+        {
+            double sq[NFGE], wp[NFGE];
+#pragma unroll
+            for (int k = 0; k < NFGE; ++k)
+            {
+                sq[k] = Tiny<double>::AZ;
+#pragma unroll
+                for (int d = 0; d < ND; ++d)
+                {
+                    sq[k] = fm(g[k][d], g[k][d], sq[k]);
+                }
+            }
+            fire = weights64_plain<NFGE>(sq, acfl, a.sigma0, wp);
+#pragma unroll
+            for (int k = 0; k < NFGE; ++k)
+            {
+                w[k] = wp[k];
             }
         }
-        fired |= weights64<NFGE>(sq, ts, acfl, a.sigma0, w) ? 1u << (q + i) : 0u;
+        fired |= fire ? 1u << (q + i) : 0u;
 #pragma unroll
         for (int d = 0; d < ND; ++d)
         {
-            double s = mu(w[0], g[0][d]);
+            double s = mx<ND, E>(w[0], g[0][d]);
 #pragma unroll
             for (int k = 1; k < NFGE; ++k)
             {

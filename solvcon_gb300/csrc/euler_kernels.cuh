@@ -98,14 +98,19 @@ __host__ __device__ constexpr bool carries()
 //  112, 60.9 / 54.3 at 96, 64.8 / 55.4 at 80.  176k hexahedra 82 us at 168, 90 at
 //  128, 98 at 254.  Any mix: 176k hexahedra 99 us at 168, 105 at 128, 118 at the
 //  243 that the compiler takes; 490k quadrilaterals 62 at 96, 66 at its 126.
-//  FP64: at its 255 registers 8 warps per SM are too few to keep the FP64 pipes
-//  fed through their loads, and a spilling kernel of more warps is faster: 343k
-//  hexahedra 1,948 us at 255, 1,780 at 168, 1,717 at 128; 54k prisms (any mix)
-//  277, 223, 250.  Triangles, tetrahedra and quadrilaterals gain nothing.
+//  FP64: enough warps to keep the FP64 pipes fed through their loads, spilling
+//  for it where a cell has many faces: 64k hexahedra 284 us at 128 (with its
+//  spills), 325 at 168, 314 at 255; 64k prisms (any mix) 430 at 168, 432 at 128,
+//  441 at 255; 384k tetrahedra 648 at 128, 657 at the 138 that the compiler takes,
+//  655 at 102; 490k quadrilaterals (any mix) 446 at 102, 451 at 124; triangles
+//  the same from 85 to 106.
 template <int ND, typename R, int CT, int BLOCK, typename G = R>
 __host__ __device__ constexpr int min_blocks()
 {
-    constexpr int regs = sizeof(R) == 8 ? (CT == 5 ? 128 : (CT == 0 && ND == 3 ? 168 : 0))
+    constexpr int regs = sizeof(R) == 8 ? (CT == 5 || CT == 6  ? 128
+                                             : CT == 0 && ND == 3 ? 168
+                                             : CT == 0            ? 102
+                                                                  : 0)
                          : CT == 0      ? (ND == 2 ? 96 : 168)
                          : CT == 5      ? 168
                          : CT == 6      ? 128
