@@ -46,12 +46,12 @@ sys.path.insert(0, ROOT)
 
 # Algorithmic HBM bytes of one cell-substep of the fused march: compulsory
 # reads of the neighbour-summed state, the cell's geometry and ids, and writes
-# of so0n, so1n, cflo, cflc.  2D triangles: FP64 520 B, FP32 state with FP64
-# geometry (the FP32 form, "fp32") 412 B, FP32 geometry too ("fp32-geom32")
-# 268 B; 3D tetrahedra: 1,100 / 928 / 560 B.
-ALG_BYTES = {("tri2d", "fp64"): 520, ("tri2d", "fp32"): 412,
+# of so0n, so1n, cflo, cflc.  2D triangles: FP64 520 B, FP32 268 B (both
+# forms' marches read FP32 geometry: "fp32" computes it in FP64 and rounds it
+# once); 3D tetrahedra: 1,100 / 560 B.
+ALG_BYTES = {("tri2d", "fp64"): 520, ("tri2d", "fp32"): 268,
              ("tri2d", "fp32-geom32"): 268, ("tet3d", "fp64"): 1100,
-             ("tet3d", "fp32"): 928, ("tet3d", "fp32-geom32"): 560}
+             ("tet3d", "fp32"): 560, ("tet3d", "fp32-geom32"): 560}
 ALG_BYTES.update({(w, "fp32-geom64"): ALG_BYTES[(w, "fp32")]
                   for w in ("tri2d", "tet3d")})
 
@@ -59,16 +59,16 @@ ALG_BYTES.update({(w, "fp32-geom64"): ALG_BYTES[(w, "fp32")]
 # substep kernel per cell-substep, each from one ncu capture of the kernel on
 # a smaller mesh of the same workload, larger than L2 (tri2d: 500^2 x 2 cells
 # FP64, 700^2 x 2 FP32; tet3d: 40^3 x 6 FP64, 60^3 x 6 FP32), divided by its
-# cells; absent until captured.  The FP64 records carry a primitive cache
-# (192 B instead of 128 B), which trades DRAM bytes, idle in the FP64-bound
+# cells; absent until captured.  The FP64 records carry the state's flux terms
+# (288 B instead of 128 B), which trades DRAM bytes, idle in the FP64-bound
 # march, for FP64 operations.
-NCU_TRAFFIC_PER_CELL = {("tri2d", "fp64"): 769.5,
-                        ("tri2d", "fp32"): 546.6,
-                        ("tri2d", "fp32-geom32"): 270.2,
-                        ("tet3d", "fp64"): 1337.3,
-                        ("tet3d", "fp32"): 1199.1,
-                        ("tet3d", "fp32-geom32"): 627.1}
-NCU_DP_FLOPS_PER_CELL = {("tri2d", "fp64"): 1159.6, ("tet3d", "fp64"): 2717.4}
+NCU_TRAFFIC_PER_CELL = {("tri2d", "fp64"): 1068.7,
+                        ("tri2d", "fp32"): 351.7,
+                        ("tri2d", "fp32-geom32"): 300.0,
+                        ("tet3d", "fp64"): 2135.7,
+                        ("tet3d", "fp32"): 754.5,
+                        ("tet3d", "fp32-geom32"): 656.3}
+NCU_DP_FLOPS_PER_CELL = {("tri2d", "fp64"): 569.7, ("tet3d", "fp64"): 1479.7}
 
 WORKLOADS = {
     "tri2d": dict(ndim=2, nside=1000, jitter=0.2, cfl=0.8, seed=2026),
@@ -1267,9 +1267,9 @@ def main():
                     sorted(LINE_WORKLOADS))
     ap.add_argument("--precision", default=None,
                     choices=["fp64", "fp32", "fp32-geom64", "fp32-geom32"],
-                    help="fp32: FP32 state and flux with FP64 geometry "
-                    "tables (fp32-geom64 is the same); fp32-geom32 also "
-                    "stores the geometry in FP32")
+                    help="fp32: FP32 state and flux, geometry computed in FP64 "
+                    "and rounded once (fp32-geom64 is the same); fp32-geom32 "
+                    "stores fewer values, the rest formed in FP32")
     ap.add_argument("--nside", type=int, default=None)
     ap.add_argument("--cpu-nside", type=int, default=None)
     ap.add_argument("--cpu-steps", type=int, default=20)

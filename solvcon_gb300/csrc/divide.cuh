@@ -3,13 +3,12 @@
  *
  * GB300 issues one FP64 instruction per SM every 19 cycles (measured; 64 on one
  * SM sub-partition alone), and the FP64 marches keep that pipe full while the
- * integer and FP32 pipes idle (8% of the issue slots used), so these
+ * integer and FP32 pipes idle (8% of the issue slots used, 16% with these), so these
  * functions form their results with integer instructions alone, half a cycle
  * each: Newton's iteration in fixed point from the FP32 hardware
  * approximation, the residual kept exactly or to 62 bits, the result rounded
  * once to 53 bits.  recip, rsq and sqr_t are within 0.52 ulp, in about 30, 40
- * and 48 instructions (4, 5 and 8 on the FP64 pipe before; a triangle's
- * substep takes 6, 12 and 2 of them, a hexahedron's 15, 40 and 2).  div_fix is
+ * and 48 instructions (4, 5 and 8 on the FP64 pipe before).  div_fix is
  * the IEEE quotient bit for bit, in about 50 (5 on the FP64 pipe from a
  * tabulated reciprocal by Markstein's method before, more without).
  * scg_divide_check, scg_root_check and scg_product_check compare them on the device.

@@ -4,9 +4,10 @@
  * The FP64 march's per-cell routines: calc_soln, calc_cfl, calc_dsoln and
  * calc_solt of the reference EulerCore (cpp/solvcon/multidim/euler_march.cpp,
  * euler_solution.cpp, euler_gradient.cpp, GradientElement.cpp), arranged for
- * the fewest instructions on the FP64 pipe, which bounds these kernels: one
- * FP64 instruction takes an SM 16 cycles, and everything else together fills a
- * tenth of the issue slots.
+ * the fewest instructions on the FP64 pipe, which bounds these kernels: with
+ * the pipe full a warp's FP64 instruction takes an SM 19 cycles (64 on its
+ * sub-partition alone), and everything else together fills a sixth of the
+ * issue slots.
  *
  *  - Flux terms once per cell instead of once per face.  calc_soln's temporal
  *    flux through a face from neighbour j is
@@ -23,12 +24,14 @@
  *    solution deltas over all faces, the gradient without face m is
  *    g - s c_m, g = sum_f delta_f c_f being the one without the last face.
  *    The weights sum to one, so their mean needs only g, s and the c_m.
- *  - Reciprocals, roots and comparisons on the integer pipe (divide.cuh).
+ *  - Reciprocals, roots and comparisons, the gradient elements' norms and
+ *    weights, and in 2D some products on the integer pipe (divide.cuh,
+ *    weights64).
  *
- * FP64-pipe instructions per cell-substep (ncu), before -> with these: triangle
- * 743 -> 430, tetrahedron 1,701 -> 1,041, hexahedron 3,060 -> 2,171; 500k
- * triangles 694 -> 407 us per launch, 384k tetrahedra 1,199 -> 781 us, 216k
- * hexahedra 1,310 -> 1,020 us, the FP64 pipe 89%, 87% and 79% busy.
+ * FP64-pipe instructions per cell-substep (ncu), with the neighbours' fluxes
+ * formed per face and all of this on the FP64 pipe -> now: triangle 743 -> 340,
+ * tetrahedron 1,701 -> 903, hexahedron 3,060 -> 1,903; 500k triangles 694 -> 326 us
+ * per launch, 384k tetrahedra 1,199 -> 648 us.
  *
  * Every operation is written as the instruction it is (fused multiply-add,
  * multiply, add), so the kernels that inline these routines (one cell type or

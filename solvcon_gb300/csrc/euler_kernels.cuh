@@ -1596,7 +1596,7 @@ __global__ void __launch_bounds__(128) k_fused(MarchArgs<R, G> a, int64_t t0, in
 
 // The same kernel asking the compiler for MINB resident blocks of 128
 // (min_blocks).  A stated minimum of 1 would instead free the compiler to use
-// up to 255 registers, so the kernels that do not carry keep the one-argument
+// up to 255 registers, so the kernels without a budget keep the one-argument
 // bound.
 template <int ND, typename R, typename G, int CT1, int MINB>
 __global__ void __launch_bounds__(128, MINB) k_fused_mb(MarchArgs<R, G> a, int64_t t0, int64_t t1)
