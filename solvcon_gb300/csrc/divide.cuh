@@ -3,7 +3,7 @@
  *
  * GB300 issues one FP64 instruction per SM every 19 cycles (measured; 64 on one
  * SM sub-partition alone), and the FP64 marches keep that pipe full while the
- * integer and FP32 pipes idle (8% of the issue slots used, 16% with these), so these
+ * integer and FP32 pipes idle (8% of the issue slots used, 14 to 25% with these), so these
  * functions form their results with integer instructions alone, half a cycle
  * each: Newton's iteration in fixed point from the FP32 hardware
  * approximation, the residual kept exactly or to 62 bits, the result rounded

@@ -6,7 +6,7 @@
  * euler_solution.cpp, euler_gradient.cpp, GradientElement.cpp), arranged for
  * the fewest instructions on the FP64 pipe, which bounds these kernels: with
  * the pipe full a warp's FP64 instruction takes an SM 19 cycles (64 on its
- * sub-partition alone), and everything else together fills a sixth of the
+ * sub-partition alone), and all instructions together fill 14 to 23% of the
  * issue slots.
  *
  *  - Flux terms once per cell instead of once per face.  calc_soln's temporal
