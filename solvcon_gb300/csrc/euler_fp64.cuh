@@ -449,10 +449,12 @@ __device__ __noinline__ bool weights64_plain(double const * sq, double acfl, dou
     return fire;
 }
 
-// n 2^e for n in [2^63, 2^64), rounded down to a double.
+// n 2^e for n in [2^63, 2^64), rounded to the nearest double (a half away from
+// zero; rounding up to 2^64 carries into the exponent).
 __device__ __forceinline__ double compose(unsigned long long n, int e)
 {
-    return __longlong_as_double(static_cast<long long>((n >> 11) + (static_cast<unsigned long long>(1085 + e) << 52)));
+    return __longlong_as_double(
+        static_cast<long long>((n >> 11) + ((n >> 10) & 1ull) + (static_cast<unsigned long long>(1085 + e) << 52)));
 }
 
 // The same weights, 1/N + (N-1)/N U_k / max(t S, M), in integers but for one
@@ -511,6 +513,7 @@ __device__ __forceinline__ bool weights64(unsigned long long * w, int const * h,
     bool const fire = eb > e || (eb == e && nb > n);
     n = fire ? nb : n;
     e = fire ? eb : e;
+    n += n < 0ull - 1024ull ? 1024ull : 0ull; // to 53 bits, to the nearest
     unsigned long long r = rcp_sig(static_cast<unsigned>(n >> 43), static_cast<unsigned>(n >> 11)); // 2^62 / (n 2^-63)
     r -= r / N;
     // |u_k| < 2^(e + 1), so that u_k 2^(61 - e) fits; zero where e < 0.
