@@ -447,8 +447,8 @@ int scg_geometry_round(const double * in, float * out, int64_t n);
 int scg_divide_check(const double * x, const double * d, double * q, double * qdiv, double * rcp, int64_t n);
 /* Not in the reference: the FP64 march's reciprocal roots r[i] = 1 / sqrt(x[i])
  * and roots s[i] = sqrt(x[i]) on the device, formed on the integer pipe for
- * positive normal x (within 0.52 ulp; other x by the library functions), for
- * checking them.  Synchronous; allocates its own device buffers. */
+ * positive normal x (r within 0.52 ulp, s rounded to nearest; other x by the
+ * library functions), for checking them.  Synchronous; allocates its own device buffers. */
 int scg_root_check(const double * x, double * r, double * s, int64_t n);
 /* Not in the reference: the products p[i] = a[i] * b[i] on the device by the
  * 1D marches' multiplication on the integer pipe (bit for bit the FP64 product),

@@ -7,10 +7,10 @@
  * functions form their results with integer instructions alone, half a cycle
  * each: Newton's iteration in fixed point from the FP32 hardware
  * approximation, the residual kept exactly or to 62 bits, the result rounded
- * once to 53 bits.  recip, rsq and sqr_t are within 0.52 ulp, in about 30, 40
- * and 48 instructions (4, 5 and 8 on the FP64 pipe before).  div_fix is
- * the IEEE quotient bit for bit, in about 50 (5 on the FP64 pipe from a
- * tabulated reciprocal by Markstein's method before, more without).
+ * once to 53 bits.  recip and rsq are within 0.52 ulp, in about 30 and 40
+ * instructions (4 and 5 on the FP64 pipe before).  sqr_t and div_fix are the
+ * IEEE root and quotient bit for bit, in about 60 and 50 (8 on the FP64 pipe
+ * before; 5 from a tabulated reciprocal by Markstein's method, more without).
  * scg_divide_check, scg_root_check and scg_product_check compare them on the device.
  *
  * Operands outside the stated ranges take the division or the library
@@ -262,8 +262,10 @@ __device__ __forceinline__ double rsq(double x)
 }
 __device__ __forceinline__ float rsq(float x) { return rsqrtf(x); }
 
-// sqrt(x) = x / sqrt(x): FP64 positive normal x and zero, else the library's;
-// FP32 the library's.
+// sqrt(x): FP64 positive normal x rounded to nearest, as the library's root is,
+// and zero; else, and in FP32, the library's.  With x / sqrt(x) rounded to S, in
+// units of its 53 bits within 0.52 of the root, the exact remainder of S^2,
+// modulo 2^64, says whether S is one off: a root is never half-way between two.
 __device__ __forceinline__ double sqr_t(double x)
 {
     unsigned const hi = static_cast<unsigned>(__double2hiint(x));
@@ -275,9 +277,12 @@ __device__ __forceinline__ double sqr_t(double x)
     unsigned long long X;
     int h;
     unsigned long long const r = rsq_fixed(hi, lo, X, h);
-    unsigned long long const q = mul_hi64(X, r); // sqrt(m) 2^60
+    unsigned long long S = (mul_hi64(X, r) + 128u) >> 8; // sqrt(m) 2^52
+    long long const rem = static_cast<long long>((X << 42) - S * S);
+    long long const s = static_cast<long long>(S);
+    S += static_cast<unsigned long long>((rem > s ? 1 : 0) - (rem <= -s ? 1 : 0));
     return __longlong_as_double(
-        static_cast<long long>(((q + 128u) >> 8) + (static_cast<unsigned long long>(1022 + h) << 52)));
+        static_cast<long long>(S + (static_cast<unsigned long long>(1022 + h) << 52)));
 }
 __device__ __forceinline__ float sqr_t(float x) { return sqrtf(x); }
 
