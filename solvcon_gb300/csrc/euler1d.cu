@@ -139,14 +139,18 @@ struct P1D
     }
 
     // update_cfl at the point (Euler1DCore.cpp:70-94), times the table's
-    // dt / 2 / dx.  The reference's sqrt(m * m) / rho is |v|.
+    // dt / 2 / dx.  The reference's sqrt(m * m) / rho is |v| with the density's
+    // sign.
     __device__ __forceinline__ double cfl(double cflr) const
     {
         // (p + |p|) / 2: zero for a negative p, NaN for -infinity and NaN.
         unsigned const hp = static_cast<unsigned>(__double2hiint(p));
         double const pr =
             hp >= 0x80000000u ? (hp >= 0xfff00000u ? __longlong_as_double(0x7ff8000000000000ll) : 0.0) : p;
-        return mu(ad(scg::dev::sqr_t(mu(mu(ga, pr), r)), fabs(v)), cflr);
+        double const speed =
+            __hiloint2double((__double2hiint(v) & 0x7fffffff) | (__double2hiint(r) & static_cast<int>(0x80000000u)),
+                             __double2loint(v));
+        return mu(ad(scg::dev::sqr_t(mu(mu(ga, pr), r)), speed), cflr);
     }
 };
 
