@@ -85,12 +85,14 @@ __device__ __forceinline__ void hand_over(R const * v, R * w, R (*slots)[N])
     }
 }
 
-// The largest cluster this GPU schedules for a kernel at `threads` threads a
-// block: 16 where it can (a non-portable size), else 8.  Asked once per kernel.
+// The largest cluster the current device schedules for a kernel at THREADS
+// threads a block: 16 where it can (a non-portable size), else 8.  Asked once per
+// kernel and device, where the permission for 16 holds.
 template <auto KERNEL, int THREADS>
 inline int cluster_limit()
 {
-    static int const limit = [] {
+    static PerDevice<int> limit;
+    return limit.get([] {
         cudaLaunchAttribute attr{};
         attr.id = cudaLaunchAttributeClusterDimension;
         attr.val.clusterDim = {16, 1, 1};
@@ -107,8 +109,7 @@ inline int cluster_limit()
         }
         (void)cudaGetLastError();
         return 8;
-    }();
-    return limit;
+    });
 }
 
 // Launch a kernel as one cluster of `blocks` blocks.

@@ -9,6 +9,7 @@
 
 #include <atomic>
 #include <cstdint>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 
@@ -56,6 +57,32 @@ inline void cuda_check(cudaError_t rc, char const * what)
         throw CudaError(std::string(what) + ": " + cudaGetErrorString(rc));
     }
 }
+
+// A value that holds for one device (a limit asked of the driver, an attribute
+// set on a kernel): made by `make` on the first call with that device current,
+// and again there if it threw.  Safe with several threads.
+template <typename T>
+class PerDevice
+{
+public:
+    template <typename F>
+    T get(F && make)
+    {
+        int dev = 0;
+        cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
+        if (dev < 0 || dev >= COUNT)
+        {
+            return make();
+        }
+        std::call_once(m_once[dev], [&] { m_value[dev] = make(); });
+        return m_value[dev];
+    }
+
+private:
+    static constexpr int COUNT = 64;
+    std::once_flag m_once[COUNT];
+    T m_value[COUNT] = {};
+};
 
 inline void launched(cudaStream_t s, char const * what)
 {

@@ -85,14 +85,21 @@ enum Precision : int
     PREC_FP32 = 2,         // the same with displacements formed in FP32 from fewer stored values (faster variant)
 };
 
-// Let a kernel use `bytes` of dynamic shared memory (asked for once per kernel).
+// Let a kernel use BYTES of dynamic shared memory on the current device (asked
+// for once per kernel and device, where the attribute holds).
 template <auto KERNEL, int BYTES>
 inline void allow_shared()
 {
-    static cudaError_t const rc = BYTES <= 0 ? cudaSuccess
-                                             : cudaFuncSetAttribute(reinterpret_cast<void const *>(KERNEL),
-                                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, BYTES);
-    cuda_check(rc, "cudaFuncSetAttribute");
+    if constexpr (BYTES > 0)
+    {
+        static PerDevice<bool> allowed;
+        allowed.get([] {
+            cuda_check(cudaFuncSetAttribute(reinterpret_cast<void const *>(KERNEL),
+                                            cudaFuncAttributeMaxDynamicSharedMemorySize, BYTES),
+                       "cudaFuncSetAttribute");
+            return true;
+        });
+    }
 }
 
 struct EulerBoundary
