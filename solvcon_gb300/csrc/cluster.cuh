@@ -86,29 +86,36 @@ __device__ __forceinline__ void hand_over(R const * v, R * w, R (*slots)[N])
 }
 
 // The largest cluster the current device schedules for a kernel at THREADS
-// threads a block: 16 where it can (a non-portable size), else 8.  Asked once per
-// kernel and device, where the permission for 16 holds.
+// threads a block: 16 where it can (a non-portable size), else a smaller power of
+// two, 0 where it schedules none (part of a GPU may have fewer SMs than a
+// portable cluster wants).  Asked once per kernel and device, where the
+// permission for 16 holds.
 template <auto KERNEL, int THREADS>
 inline int cluster_limit()
 {
     static PerDevice<int> limit;
     return limit.get([] {
-        cudaLaunchAttribute attr{};
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim = {16, 1, 1};
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(16);
-        cfg.blockDim = dim3(THREADS);
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        int n = 0;
-        if (cudaFuncSetAttribute(KERNEL, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-            cudaOccupancyMaxActiveClusters(&n, KERNEL, &cfg) == cudaSuccess && n > 0)
-        {
-            return 16;
-        }
+        bool const wide =
+            cudaFuncSetAttribute(KERNEL, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
         (void)cudaGetLastError();
-        return 8;
+        for (unsigned size = wide ? 16 : 8; size > 0; size /= 2)
+        {
+            cudaLaunchAttribute attr{};
+            attr.id = cudaLaunchAttributeClusterDimension;
+            attr.val.clusterDim = {size, 1, 1};
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3(size);
+            cfg.blockDim = dim3(THREADS);
+            cfg.attrs = &attr;
+            cfg.numAttrs = 1;
+            int n = 0;
+            if (cudaOccupancyMaxActiveClusters(&n, KERNEL, &cfg) == cudaSuccess && n > 0)
+            {
+                return static_cast<int>(size);
+            }
+            (void)cudaGetLastError(); // a refusal is no error of the launch to come
+        }
+        return 0;
     });
 }
 
@@ -138,6 +145,10 @@ template <auto KERNEL, int MAX_WARPS>
 bool cluster_shape(int64_t threads, int & blocks, int & warps)
 {
     int const limit = cluster_limit<KERNEL, 32 * MAX_WARPS>();
+    if (limit == 0)
+    {
+        return false;
+    }
     int64_t const w = (threads + 31) / 32;
     blocks = 1;
     while (blocks < limit && blocks < w)

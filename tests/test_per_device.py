@@ -16,10 +16,11 @@ RUNTIME = r"""
 #include <map>
 
 static int g_device = 0;
-static int g_largest[4] = {16, 16, 8, 4}; // cluster that each device schedules
+static int g_largest[6] = {16, 16, 8, 4, 1, 0}; // cluster that each device schedules
 static int g_calls = 0;
 static std::map<int, int> g_shared, g_wide; // by device
 static bool g_refuse = false;
+static cudaError_t g_last = cudaSuccess;
 
 extern "C"
 {
@@ -28,14 +29,19 @@ cudaError_t cudaGetDevice(int * dev)
     *dev = g_device;
     return cudaSuccess;
 }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
-cudaError_t cudaPeekAtLastError() { return cudaSuccess; }
+cudaError_t cudaGetLastError()
+{
+    cudaError_t const rc = g_last;
+    g_last = cudaSuccess;
+    return rc;
+}
+cudaError_t cudaPeekAtLastError() { return g_last; }
 char const * cudaGetErrorString(cudaError_t) { return "refused"; }
 cudaError_t cudaFuncSetAttribute(void const *, cudaFuncAttribute attr, int value)
 {
     if (g_refuse)
     {
-        return cudaErrorInvalidValue;
+        return g_last = cudaErrorInvalidValue;
     }
     ++g_calls;
     (attr == cudaFuncAttributeMaxDynamicSharedMemorySize ? g_shared : g_wide)[g_device] = value;
@@ -44,9 +50,9 @@ cudaError_t cudaFuncSetAttribute(void const *, cudaFuncAttribute attr, int value
 cudaError_t cudaOccupancyMaxActiveClusters(int * n, void const *, cudaLaunchConfig_t const * cfg)
 {
     int const size = static_cast<int>(cfg->attrs[0].val.clusterDim.x);
-    if (size > 8 && !g_wide[g_device])
+    if ((size > 8 && !g_wide[g_device]) || size > 2 * g_largest[g_device])
     {
-        return cudaErrorInvalidClusterSize;
+        return g_last = cudaErrorInvalidClusterSize;
     }
     *n = size <= g_largest[g_device] ? 1 : 0;
     return cudaSuccess;
@@ -75,6 +81,11 @@ std::atomic<int64_t> g_launches{0}, g_device_allocs{0};
 static void kernel_a(int) {}
 static void kernel_b(int) {}
 
+extern "C" int fits(int64_t threads)
+{
+    int blocks = 0, warps = 0;
+    return scg::cluster::cluster_shape<kernel_a, 4>(threads, blocks, warps) ? blocks * warps : 0;
+}
 extern "C" int limit() { return scg::cluster::cluster_limit<kernel_a, 128>(); }
 extern "C" int allow()
 {
@@ -130,3 +141,15 @@ def test_a_refusal_is_reported_and_asked_again(host):
     assert host.allow() == 1 and host.allow() == 1
     host.refuse(0)
     assert host.allow() == 0 and host.shared_of(0) == 65536
+
+
+@pytest.mark.parametrize("dev,size", [(0, 16), (2, 8), (3, 4), (4, 1), (5, 0)])
+def test_no_cluster_is_larger_than_the_device_schedules(host, dev, size):
+    """A march takes one cluster only where its threads fit the largest one,
+    four warps to a block, and none where the device schedules none."""
+    host.use(dev)
+    host.fits.argtypes = [ctypes.c_int64]
+    assert host.limit() == size
+    assert host.fits(size * 128) == 4 * size
+    assert host.fits(size * 128 + 1) == 0
+    assert host.cudaPeekAtLastError() == 0  # what the next launch looks at
