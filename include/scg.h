@@ -44,6 +44,10 @@ int64_t scg_launch_count(void);
  * process for its solver objects and per-call scratch (the device mesh
  * builder's Thrust buffers are not counted). */
 int64_t scg_device_alloc_count(void);
+/* The most bytes of device memory that this library's buffers have held at
+ * once since the last call with a non-zero reset (which starts it again from
+ * what they hold now). */
+int64_t scg_device_peak_bytes(int reset);
 /* Library version string. */
 const char * scg_version(void);
 

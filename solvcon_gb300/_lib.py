@@ -27,6 +27,7 @@ _SIGS = {
     "scg_last_error": ([], ctypes.c_char_p),
     "scg_launch_count": ([], ctypes.c_int64),
     "scg_device_alloc_count": ([], ctypes.c_int64),
+    "scg_device_peak_bytes": ([ctypes.c_int], ctypes.c_int64),
     "scg_geometry_round": ([_vp, _vp, ctypes.c_int64], ctypes.c_int),
     "scg_divide_check": ([_vp, _vp, _vp, _vp, _vp, ctypes.c_int64], ctypes.c_int),
     "scg_root_check": ([_vp, _vp, _vp, ctypes.c_int64], ctypes.c_int),

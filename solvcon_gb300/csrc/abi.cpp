@@ -18,6 +18,7 @@ namespace scg
 
 std::atomic<int64_t> g_launches{0};
 std::atomic<int64_t> g_device_allocs{0};
+std::atomic<int64_t> g_device_bytes{0}, g_device_peak{0};
 
 namespace
 {
@@ -54,6 +55,11 @@ const char * scg_last_error(void) { return scg::last_error().c_str(); }
 
 int64_t scg_launch_count(void) { return scg::g_launches.load(); }
 int64_t scg_device_alloc_count(void) { return scg::g_device_allocs.load(); }
+
+int64_t scg_device_peak_bytes(int reset)
+{
+    return reset ? scg::g_device_peak.exchange(scg::g_device_bytes.load()) : scg::g_device_peak.load();
+}
 
 const char * scg_version(void) { return "solvcon-gb300 0.1"; }
 

@@ -41,6 +41,16 @@ extern std::atomic<int64_t> g_launches;
 // Count of device allocations made through DevBuf (every device buffer of the
 // cores, batches, 1D and spacetime solvers, and per-call scratch).
 extern std::atomic<int64_t> g_device_allocs;
+// Bytes that DevBuf holds on the device, and the most that it has held.
+extern std::atomic<int64_t> g_device_bytes, g_device_peak;
+
+inline void device_held(int64_t change)
+{
+    int64_t const now = g_device_bytes.fetch_add(change) + change;
+    for (int64_t peak = g_device_peak.load(); now > peak && !g_device_peak.compare_exchange_weak(peak, now);)
+    {
+    }
+}
 
 // The device address of the host range [p, p + nbytes) when the whole range
 // lies inside one block from scg_host_alloc (page-locked and mapped into the
@@ -168,12 +178,14 @@ struct DevBuf
         }
         g_device_allocs.fetch_add(1, std::memory_order_relaxed);
         n = count;
+        device_held(static_cast<int64_t>(bytes()));
     }
     void release()
     {
         if (ptr)
         {
             cudaFree(ptr);
+            device_held(-static_cast<int64_t>(bytes()));
         }
         ptr = nullptr;
         n = 0;

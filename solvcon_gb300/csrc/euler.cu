@@ -853,7 +853,25 @@ public:
             single_ct = (icl == 0 || single_ct == t) ? t : -1;
         }
 
-        // Solution state.
+        // Boundary tables.
+        d_gkind.alloc(std::max<int64_t>(ngstcell, 1));
+        d_gnml.alloc(std::max<int64_t>(ngstcell * ND, 1));
+        d_gval.alloc(std::max<int64_t>(ngstcell * NEQ, 1));
+        d_gint.alloc(std::max<int64_t>(ngstcell, 1));
+
+        // Geometry: prepare_ce, then the compact march tables.
+        npl = Dim<ND>::KC + static_cast<int64_t>(std::max(nslot, 1)) * KF;
+        d_geo.alloc(static_cast<size_t>((std::max<int64_t>(ncell, 1) + GEO_TILE - 1) / GEO_TILE * GEO_TILE * npl));
+        // Slots past a cell's own faces are never written; zero them so the
+        // whole tables, the last tile included, hold defined values.
+        cuda_check(cudaMemsetAsync(d_geo.ptr, 0, d_geo.bytes(), stream), "memset");
+        d_nbr.alloc(static_cast<size_t>(std::max(nslot, 1)) * std::max<int64_t>(ncell, 1));
+        d_ctype.alloc(std::max<int64_t>(ncell, 1));
+        prepare_ce(true);
+
+        // Solution state: after prepare_ce has released its sub-face tables (768 B a
+        // cell in 2D, 1,152 in 3D), so that setting up a mesh needs no more memory
+        // at once than the tables or the records (576 and 1,024 B in FP64) do.
         for (auto & r : rec)
         {
             r.alloc(static_cast<size_t>(nrow * RS));
@@ -874,21 +892,6 @@ public:
             comp_live = true;
         }
 
-        // Boundary tables.
-        d_gkind.alloc(std::max<int64_t>(ngstcell, 1));
-        d_gnml.alloc(std::max<int64_t>(ngstcell * ND, 1));
-        d_gval.alloc(std::max<int64_t>(ngstcell * NEQ, 1));
-        d_gint.alloc(std::max<int64_t>(ngstcell, 1));
-
-        // Geometry: prepare_ce, then the compact march tables.
-        npl = Dim<ND>::KC + static_cast<int64_t>(std::max(nslot, 1)) * KF;
-        d_geo.alloc(static_cast<size_t>((std::max<int64_t>(ncell, 1) + GEO_TILE - 1) / GEO_TILE * GEO_TILE * npl));
-        // Slots past a cell's own faces are never written; zero them so the
-        // whole tables, the last tile included, hold defined values.
-        cuda_check(cudaMemsetAsync(d_geo.ptr, 0, d_geo.bytes(), stream), "memset");
-        d_nbr.alloc(static_cast<size_t>(std::max(nslot, 1)) * std::max<int64_t>(ncell, 1));
-        d_ctype.alloc(std::max<int64_t>(ncell, 1));
-        prepare_ce(true);
         upload_bc();
         sync();
     }
