@@ -77,6 +77,7 @@ class _MeshSpec:
         self.faces = faces
         self.gamma = gamma
         self.dt = dt
+        self.nbytes = None  # of a solver, once one was made
 
 
 class _Slot:
@@ -128,8 +129,10 @@ class Server:
         self.meshes[key] = _MeshSpec(mesh, state, faces, gamma, dt)
 
     @staticmethod
-    def tube_bytes(ncoord):
-        return 11 * 8 * int(ncoord)
+    def tube_bytes(ncoord, precision="fp32"):
+        # FP64: 17 tables of a point; FP32: 48 B and the 24 B that its state
+        # passes through to and from the host.
+        return (17 if precision == "fp64" else 11) * 8 * int(ncoord)
 
     def _evict_idle(self, need):
         """Free idle slots (least recently created first) until ``need``
@@ -153,21 +156,25 @@ class Server:
             if not s.busy:
                 return s
         if req.kind == "2d":
+            # A mesh's solver is made before its size is known exactly, so the
+            # first one may turn out not to fit; later ones are not made then.
             spec = self.meshes[req.mesh_key]
-            est = int(spec.mesh.ncell * 1200)
+            est = spec.nbytes or int(spec.mesh.ncell * 1200)
             if not self._evict_idle(est):
                 return None
             core = EulerCore(spec.mesh, spec.dt, precision=self.precision)
+            spec.nbytes = core.device_bytes
+            if not self._evict_idle(spec.nbytes):
+                return None
             core.add_slipwall(spec.faces)
-            slot = _Slot(key, core, core.device_bytes)
+            slot = _Slot(key, core, spec.nbytes)
         else:
-            est = self.tube_bytes(req.ncoord)
+            precision = _tube_precision(self.precision)
+            est = self.tube_bytes(req.ncoord, precision)
             if not self._evict_idle(est):
                 return None
             slot = _Slot(key, Euler1DCore(req.ncoord, tube_dt(req.ncoord),
-                                          precision=_tube_precision(
-                                              self.precision)),
-                         est)
+                                          precision=precision), est)
         self.held += slot.nbytes
         self.slots[key].append(slot)
         return slot
