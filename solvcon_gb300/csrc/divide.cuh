@@ -77,8 +77,7 @@ __device__ __forceinline__ unsigned long long rcp_sig(unsigned hi, unsigned lo)
 }
 
 // Reciprocal.  FP64: |d| in [2^-1022, 2^1022) as above; outside it (zero,
-// subnormals, the largest magnitudes, infinities, NaN) the division.  FP32: the
-// division.
+// subnormals, the largest magnitudes, infinities, NaN) the division.
 __device__ __forceinline__ double recip(double d)
 {
     unsigned const hi = static_cast<unsigned>(__double2hiint(d));
@@ -92,7 +91,6 @@ __device__ __forceinline__ double recip(double d)
         ((rcp_sig(hi, lo) + 256u) >> 9) + (static_cast<unsigned long long>(2044u - e) << 52);
     return __longlong_as_double(static_cast<long long>(bits | (static_cast<unsigned long long>(hi & 0x80000000u) << 32)));
 }
-__device__ __forceinline__ float recip(float d) { return 1.0f / d; }
 
 // The significand's reciprocal of a divisor, for div_fix: 2^62 / m of a normal
 // d, else 0 (div_fix then divides).

@@ -1659,7 +1659,6 @@ public:
                 R * base;
                 int off, width;
                 field_of(k == 0 ? EA_SO0N : EA_SO1N, base, off, width);
-                int64_t const n = static_cast<int64_t>(d.nbytes / sizeof(double));
                 get_field(base, d.dev, off, width, so0_residual(k == 0 ? EA_SO0N : EA_SO1N));
             }
         }

@@ -310,12 +310,6 @@ __device__ __forceinline__ void solt_prim(Prim<ND, R> const & q, R const * u, R 
     }
 }
 
-template <int ND, typename R>
-__device__ __forceinline__ void solt_row(R const * u, R const * g, R ga, R * t)
-{
-    solt_prim<ND, R>(Prim<ND, R>(u, ga), u, g, t);
-}
-
 // Fundamental gradient element tables (1-based in GradientElement.cpp:
 // 16-79, 0-based here), per cell type.
 template <int CT>
