@@ -94,6 +94,18 @@ private:
     T m_value[COUNT] = {};
 };
 
+// SMs of the current device.
+inline int sm_count()
+{
+    static PerDevice<int> count;
+    return count.get([] {
+        int dev = 0, n = 0;
+        cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
+        cuda_check(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev), "attr");
+        return n;
+    });
+}
+
 inline void launched(cudaStream_t s, char const * what)
 {
     g_launches.fetch_add(1, std::memory_order_relaxed);

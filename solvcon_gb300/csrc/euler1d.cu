@@ -609,10 +609,10 @@ public:
         int64_t start, nout;
         range(odd, start, nout);
         // Blocks of one warp while they all are resident at once (32 blocks
-        // on each of 152 SMs), so that a tube takes the FP64 pipes of as many
-        // SMs as it has warps; beyond that blocks of four.
+        // on each SM), so that a tube takes the FP64 pipes of as many SMs as it
+        // has warps; beyond that blocks of four.
         int64_t const warps = std::max<int64_t>((nout + WOUT - 1) / WOUT, 1);
-        int const wpb = warps <= 152 * 32 ? 1 : 4;
+        int const wpb = warps <= int64_t(scg::sm_count()) * 32 ? 1 : 4;
         unsigned const grid = static_cast<unsigned>((warps + wpb - 1) / wpb);
         if (n > INT_POINTS64)
         {

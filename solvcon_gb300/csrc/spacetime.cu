@@ -500,7 +500,7 @@ public:
         // Blocks of one warp while they all are resident at once, as the 1D
         // Euler core's, beyond that blocks of four.
         int64_t const warps = (n + WOUT - 1) / WOUT;
-        int const wpb = warps <= 152 * 32 ? 1 : 4;
+        int const wpb = warps <= int64_t(scg::sm_count()) * 32 ? 1 : 4;
         unsigned const grid = static_cast<unsigned>((warps + wpb - 1) / wpb);
         int const threads = 32 * wpb;
         bool const big = ncelm > INT_ELEMENTS;
