@@ -1221,7 +1221,8 @@ def headline_figures(local):
                         "log-uniform in [2k, 200k], per-mesh quadrant "
                         "states, gamma in [1.1, 1.67], CFL 0.8, slip walls)",
             "cells": r["ncell"],
-            "precision": "fp32 (FP32 state and flux, FP64 geometry)",
+            "precision": "fp32 (FP32 state and flux, geometry formed in "
+                         "FP64 and rounded once)",
             "steps": steps, "warmup": warmup,
             "ms_per_step": r["ms_per_step"], "tiles": r["best"],
             "plain_fp64_sequential": r["seq_value"],
@@ -1243,8 +1244,8 @@ def headline_figures(local):
                         "batched distribution, 200-2000 steps; HBM budget "
                         "120 GB; continuous batching, ticks of at most 32 "
                         "steps)" % (nreq, rate),
-            "precision": "fp32 (FP32 state and flux, FP64 geometry; FP32 "
-                         "tubes)",
+            "precision": "fp32 (FP32 state and flux, geometry formed in "
+                         "FP64 and rounded once; FP32 tubes)",
             "p50_latency_s": st["p50_latency_s"],
             "p99_latency_s": st["p99_latency_s"],
             "makespan_s": st["makespan_s"],

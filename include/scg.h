@@ -455,8 +455,8 @@ int scg_divide_check(const double * x, const double * d, double * q, double * qd
  * library functions), for checking them.  Synchronous; allocates its own device buffers. */
 int scg_root_check(const double * x, double * r, double * s, int64_t n);
 /* Not in the reference: the products p[i] = a[i] * b[i] on the device by the
- * 1D marches' multiplication on the integer pipe (bit for bit the FP64 product),
- * for checking it.  Synchronous; allocates its own device buffers. */
+ * multiplication on the integer pipe of the 1D Euler, the spacetime and the 2D
+ * FP64 marches (bit for bit the FP64 product), for checking it.  Synchronous; allocates its own device buffers. */
 int scg_product_check(const double * a, const double * b, double * p, int64_t n);
 /* Device FMA throughput in TFLOP/s for SCG_FP64 or SCG_FP32 (a register-only
  * FMA chain over all SMs, iters FMAs-per-accumulator). */

@@ -100,13 +100,13 @@ __global__ void k_inv_spacing(double const * coord, int64_t n, double hdt, doubl
     }
 }
 
-// The FP64 half step is bound by the FP64 pipe (one instruction per SM every 16
-// cycles), so its routines take the fewest FP64 instructions: the Jacobian
-// products are directional derivatives of the flux from the primitive
+// The FP64 half step is bound by the FP64 pipe (one instruction per SM every 19
+// cycles, see divide.cuh), so its routines take the fewest FP64 instructions: the
+// Jacobian products are directional derivatives of the flux from the primitive
 // variables, the divisions and the root are integer arithmetic (divide.cuh),
 // and what the grid fixes is read from tables: 98 FP64 instructions per output
-// point (196 with the Jacobian formed, FP64 Newton reciprocals and a library
-// root).  Every operation is written as the instruction it is, so the
+// point, 82 with half_warp's INT (196 with the Jacobian formed, FP64 Newton
+// reciprocals and a library root).  Every operation is written as the instruction it is, so the
 // fine-grained methods and the fused march round alike, as the reference
 // requires.
 __device__ __forceinline__ double fm(double a, double b, double c) { return __fma_rn(a, b, c); }

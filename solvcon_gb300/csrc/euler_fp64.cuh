@@ -297,7 +297,7 @@ __device__ __forceinline__ void soln64(MarchArgs<double, double> const & a, int6
     // index uf in local memory for it): a substep's instructions in one stretch
     // are more than the instruction caches hold, and FP64 tetrahedra and
     // hexahedra waited for them a fifth of the time.  384k tetrahedra 740 ->
-    // 688 us, 64k hexahedra 323 -> 298, 64k prisms 510 -> 440, 490k quadrilaterals
+    // 688 us, 64k hexahedra 323 -> 298, 128k prisms 510 -> 440, 490k quadrilaterals
     // 527 -> 490, 2M triangles 1348 -> 1331; most of it from the equations' loop.
 #pragma unroll 1
     for (int f = 0; f < NFC; ++f)

@@ -78,8 +78,8 @@ __device__ __forceinline__ void store_rec(float * base, float const * so0, float
 //   u_j + hdt ut_j + jdis . g_j - u_i  with  jdis = A_f + tau B_f,
 // so calc_soln, holding neighbour j's record, keeps
 //   p[f] = u_j + hdt ut_j + A_f . g_j  and  q[f] = B_f . g_j
-// per equation.  A_f = dB_f - mean(mid), B_f = mean(dB) - dB_f with FP32
-// geometry (R_f and Q_f with FP64 geometry); delta is zero for simplices.
+// per equation.  A_f = dB_f - mean(mid), B_f = mean(dB) - dB_f where the tables
+// hold mid (fp32-geom32), else the stored R_f and Q_f; delta is zero for simplices.
 // Whether the fused substep of cell type CT carries calc_soln's neighbour
 // terms to calc_dsoln (FP32 simplices) instead of gathering again.
 template <int CT>
@@ -100,10 +100,15 @@ __host__ __device__ constexpr bool carries()
 //  243 that the compiler takes; 490k quadrilaterals 62 at 96, 66 at its 126.
 //  FP64: enough warps to keep the FP64 pipes fed through their loads, spilling
 //  for it where a cell has many faces: 64k hexahedra 284 us at 128 (with its
-//  spills), 325 at 168, 314 at 255; 64k prisms (any mix) 430 at 168, 432 at 128,
+//  spills), 325 at 168, 314 at 255; 128k prisms (any mix) 430 at 168, 432 at 128,
 //  441 at 255; 384k tetrahedra 648 at 128, 657 at the 138 that the compiler takes,
 //  655 at 102; 490k quadrilaterals (any mix) 446 at 102, 451 at 124; triangles
 //  the same from 85 to 106.
+// A batch's tiles of 256 round the quotient down, so the budgets there are looser:
+// 128 registers for 96 to 128, none (one block, 255) for 168.  It does not
+// cost: 12 meshes of 1,024 to 16,000 prisms (any mix) 41.4 us per substep in
+// tiles of 256 against 44.9 in tiles of 128 (FP64 299 against 355), 12 of 512 to
+// 13,824 hexahedra 45.6 against 47.6 (FP64 349 against 391).
 template <int ND, typename R, int CT, int BLOCK, typename G = R>
 __host__ __device__ constexpr int min_blocks()
 {
@@ -162,7 +167,7 @@ struct CarrySh
     Tab q;
 };
 
-// Face means of mid and dB (FP32 geometry; zero with FP64 geometry).
+// Face means of mid and dB where the tables hold mid (fp32-geom32), else zeros.
 template <int CT, typename R, typename G, bool SH>
 __device__ __forceinline__ void face_means(GeoView<G, SH> const & gv, R * mm, R * mb)
 {
@@ -389,7 +394,7 @@ __device__ __forceinline__ void dsoln_cell(MarchArgs<R, G> const & a, GeoView<G,
     R const ofg1 = R(1) / R(NFGE);
 
     // Gradient-evaluation displacements: idis = dst - delta, dst = P + tau Q.
-    // With FP32 geometry P = mid - mean(mid) and Q = mean(dB) - dB are formed
+    // In fp32-geom32 P = mid - mean(mid) and Q = mean(dB) - dB are formed
     // here from the face means (the faces' values are read again rather than
     // held: they hit in L1, and registers bound this kernel's occupancy).
     R mm[ND], mb[ND];

@@ -49,8 +49,12 @@ struct STArgs
 // instead of recomputing them and its results stay bit-identical.  The four
 // divisors of a half step also get their reciprocals (rcp_fix, the bits kept in
 // a double), from which div_fix forms each quotient exactly as the division
-// would, on the integer pipe: the half step is bound by the FP64 pipe (53
-// instructions per element with its quotients there, 28 without).
+// would, on the integer pipe: with its quotients on the FP64 pipe (53
+// instructions per element there, 28 without) the half step was bound by it.
+// Now, above L2, it waits for DRAM first: the grid quantities, so0, so1 and cfl
+// lie point after point and a half step takes every second one, so it moves 252 B
+// per element for the 120 that it uses (8M elements 360 us, 5.6 TB/s, 83% of the
+// measured copy rate; the FP64 pipe 74% busy).
 enum
 {
     G_DXNEG = 0, // x - xneg
@@ -400,9 +404,9 @@ __global__ void k_st_bnd(STArgs a, int which)
 }
 
 // Grids above this many elements take 7 of an element's FP64 multiplications on
-// the integer pipe (k_st_half's INT, the same bits), where the FP64 pipes are
-// full (1M elements, linear 54.0 -> 49.3 us per half step, Burgers 67.9 -> 61.2;
-// 100,000 elements 7.6 -> 7.3).
+// the integer pipe (k_st_half's INT, the same bits), which takes the FP64 pipes
+// below what the loads allow (1M elements, linear 54.0 -> 49.3 us per half step,
+// Burgers 67.9 -> 61.2; 100,000 elements 7.6 -> 7.3).
 constexpr int64_t INT_ELEMENTS = 80000;
 
 class Spacetime

@@ -34,7 +34,8 @@ _OPS = {"prepare_ce": 0, "update": 1, "calc_solt": 2, "calc_soln": 3,
         "bc_soln": 4, "calc_cfl": 5, "calc_dsoln": 6, "bc_dsoln": 7,
         "march_substep": 8, "reset_state": 9}
 # "fp32" is the FP32 form (FP32 state and flux, geometry formed in FP64);
-# "fp32-geom64" names the same; "fp32-geom32" also stores the geometry FP32.
+# "fp32-geom64" names the same; "fp32-geom32" forms part of the geometry in
+# FP32 from fewer stored values.
 PRECISIONS = {"fp64": 0, "fp32": 1, "fp32-geom64": 1, "fp32-geom32": 2}
 _SWAP = (("so0c", "so0n"), ("so1c", "so1n"))
 
