@@ -62,10 +62,10 @@ ALG_BYTES.update({(w, "fp32-geom64"): ALG_BYTES[(w, "fp32")]
 # cells; absent until captured.  The FP64 records carry the state's flux terms
 # (288 B instead of 128 B), which trades DRAM bytes, idle in the FP64-bound
 # march, for FP64 operations.
-NCU_TRAFFIC_PER_CELL = {("tri2d", "fp64"): 1068.7,
+NCU_TRAFFIC_PER_CELL = {("tri2d", "fp64"): 1067.9,
                         ("tri2d", "fp32"): 351.7,
                         ("tri2d", "fp32-geom32"): 300.0,
-                        ("tet3d", "fp64"): 2135.7,
+                        ("tet3d", "fp64"): 2134.0,
                         ("tet3d", "fp32"): 754.5,
                         ("tet3d", "fp32-geom32"): 656.3}
 NCU_DP_FLOPS_PER_CELL = {("tri2d", "fp64"): 569.7, ("tet3d", "fp64"): 1479.7}
